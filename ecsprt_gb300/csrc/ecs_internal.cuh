@@ -58,7 +58,9 @@ struct MgLevel {
   T *t = nullptr;      // smoother scratch
   // z-line factorisation of the (lower, diag, upper) z-tridiagonal part,
   // cyclic closure by Sherman-Morrison (periodic z) or plain (reflecting z).
-  T *zl_a = nullptr, *zl_cp = nullptr, *zl_minv = nullptr, *zl_q = nullptr;
+  T *zl_minv = nullptr, *zl_q = nullptr;
+  // FP64 and long columns only (else recomputed from the density and 1/m):
+  T *zl_a = nullptr, *zl_cp = nullptr;
   T *zl_fb = nullptr, *zl_bb = nullptr;     // in-segment products of the recurrences
   T *zl_a0g = nullptr, *zl_qden = nullptr;  // per-column Sherman-Morrison scalars
 };

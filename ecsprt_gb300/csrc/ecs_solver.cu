@@ -85,9 +85,17 @@ __global__ void k_apply(OpK o, const T *__restrict__ n, const T *__restrict__ x,
 // y_k = d_k - cp_k y_{k+1} are affine in the value carried in, so each
 // segment solves from zero and the carried values are stitched afterwards
 // with the in-segment products fb_k = prod(-a_i/m_i) and bb_k = prod(-cp_i).
+// FP32 with segments of 8 stores 1/m and the Sherman-Morrison vector q only:
+// a, cp, fb and bb follow from the density and 1/m with the set-up's own
+// operations (the same bits), which is cheaper than reading four more words a
+// cell.  On this GPU FP64 arithmetic is the scarcer resource, so FP64 reads
+// them all; so do segments of 16 and more, whose recomputed factors would not
+// fit the registers.
+template <typename T>
+__host__ __device__ constexpr bool zl_stored(int S) { return sizeof(T) == 8 || S > 8; }
 template <typename T>
 struct ZlP {
-  T *a, *cp, *minv, *q, *fb, *bb;  // per cell
+  T *a, *cp, *minv, *q, *fb, *bb;  // per cell (a, cp, fb, bb: zl_stored only, else nullptr)
   T *a0g, *qden;                   // per column
 };
 // At most 16 segments a column (block of 32 x 16 threads); segments of 8,
@@ -100,28 +108,40 @@ static inline int seg_len(int N) {
   return 64;
 }
 
-// The z entries of every row (lower, upper, diagonal), one thread per cell:
-// the parallel half of the z-line set-up.
+// The z couplings of the rows: lower entry of plane k from the densities of
+// planes k and k - 1, upper entry from those of planes k and k + 1 (the same
+// operations as row11_vals); unit: density 1 everywhere.
 template <typename T>
-__global__ void k_zline_rows(OpK o, const T *__restrict__ n, T *__restrict__ lo, T *__restrict__ up,
-                             T *__restrict__ dg) {
+struct ZCoup {
+  T szz;
+  int unit;
+  __device__ __forceinline__ T operator()(T here, T other) const {
+    return unit ? szz * (T(1) + T(1)) : szz * (other + here);
+  }
+};
+template <typename T>
+static inline ZCoup<T> z_coupling(const OpK &o) {
+  return {sizeof(T) == 8 ? (T)o.szz : (T)o.fzz, o.unit};
+}
+
+// The diagonal of every row, one thread per cell: the parallel half of the
+// z-line set-up.
+template <typename T>
+__global__ void k_zline_rows(OpK o, const T *__restrict__ n, T *__restrict__ dg) {
   ECS_PDL_ENTRY();
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const Nbr q = nbr_of(o.g, i, j, k);
   T v[11];
   row11_n(n, o, q, v);
-  const unsigned c = q.c;
-  lo[c] = v[5];
-  up[c] = v[4];
-  dg[c] = v[10];
+  dg[q.c] = v[10];
 }
 
 // Factorisation of every column's z tridiagonal (one thread a column) from
-// the rows of k_zline_rows.
+// the density and the diagonal of k_zline_rows.
 template <typename T>
-__global__ void k_zline_setup(GridG g, const T *__restrict__ lo, const T *__restrict__ up,
-                              const T *__restrict__ dg, ZlP<T> z, int S) {
+__global__ void k_zline_setup(GridG g, ZCoup<T> zc, const T *__restrict__ n, const T *__restrict__ dg, ZlP<T> z,
+                              int S) {
   ECS_PDL_ENTRY();
   const int ncol = g.nx * g.ny;
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
@@ -130,28 +150,30 @@ __global__ void k_zline_setup(GridG g, const T *__restrict__ lo, const T *__rest
   // a one-cell column (2-D) has no z coupling: the plain solve, no periodic closure
   const bool cyc = g.bc[2] == 0 && g.nz > 1;
   const int N = g.nz;
-  const T lo0 = cyc ? __ldg(&lo[col]) : T(0), d0 = __ldg(&dg[col]);
+  const bool stored = z.a != nullptr;
+  const T n0 = __ldg(&n[col]), nN = __ldg(&n[(size_t)(N - 1) * plane + col]);
+  const T lo0 = cyc ? zc(n0, nN) : T(0), d0 = __ldg(&dg[col]);
   const T gamma = -d0;
   T cp_prev = T(0), dq_prev = T(0), fprod = T(1);
   // forward: factor T' and forward-substitute u = (gamma, 0, .., up_{N-1});
-  // the rows are read kBatch at a time, all loads first, so the recurrence
-  // waits on one memory latency a batch rather than one a cell
+  // the operands are read kBatch at a time, all loads first, so the
+  // recurrence waits on one memory latency a batch rather than one a cell
   constexpr int kBatch = 8;
+  T nprev = nN, nhere = n0;
   for (int k0 = 0; k0 < N; k0 += kBatch) {
-    T lv[kBatch], uv[kBatch], dv[kBatch];
+    T nv[kBatch], dv[kBatch];
 #pragma unroll
     for (int e = 0; e < kBatch; e++) {
-      const size_t c = (size_t)min(k0 + e, N - 1) * plane + col;
-      lv[e] = __ldg(&lo[c]);
-      uv[e] = __ldg(&up[c]);
-      dv[e] = __ldg(&dg[c]);
+      const int k = min(k0 + e, N - 1), kn = k + 1 < N ? k + 1 : 0;  // the plane above, wrapped
+      nv[e] = __ldg(&n[(size_t)kn * plane + col]);
+      dv[e] = __ldg(&dg[(size_t)k * plane + col]);
     }
 #pragma unroll
     for (int e = 0; e < kBatch; e++) {
       const int k = k0 + e;
       if (k >= N) break;
       const size_t c = (size_t)k * plane + col;
-      const T lk = lv[e], uk = uv[e], dk = dv[e];
+      const T lk = zc(nhere, nprev), uk = zc(nhere, nv[e]), dk = dv[e];
       T a = (k == 0) ? T(0) : lk;
       T upk = (k == N - 1) ? T(0) : uk;
       T bb = dk;
@@ -162,40 +184,54 @@ __global__ void k_zline_setup(GridG g, const T *__restrict__ lo, const T *__rest
       T cp = upk * minv;
       T u = cyc ? ((k == 0) ? gamma : ((k == N - 1) ? uk : T(0))) : T(0);
       T dq = (u - a * dq_prev) * minv;
-      z.a[c] = a;
-      z.cp[c] = cp;
       z.minv[c] = minv;
       z.q[c] = dq;
-      if (k % S == 0) fprod = T(1);
-      fprod *= -(a * minv);
-      z.fb[c] = fprod;
+      if (stored) {
+        z.a[c] = a;
+        z.cp[c] = cp;
+        if (k % S == 0) fprod = T(1);
+        fprod *= -(a * minv);
+        z.fb[c] = fprod;
+      }
       cp_prev = cp;
       dq_prev = dq;
+      nprev = nhere;
+      nhere = nv[e];
     }
   }
-  // backward substitution for q, in-segment products of -cp (this thread's
-  // own values from above, read back a batch at a time)
+  // backward substitution for q (this thread's own values from above, read
+  // back a batch at a time) and, where they are stored, the in-segment
+  // products of -cp
   T qn = z.q[(size_t)(N - 1) * plane + col];
-  T bprod = -z.cp[(size_t)(N - 1) * plane + col];
-  z.bb[(size_t)(N - 1) * plane + col] = bprod;
+  T bprod = T(1);
+  if (stored) {
+    bprod = -z.cp[(size_t)(N - 1) * plane + col];
+    z.bb[(size_t)(N - 1) * plane + col] = bprod;
+  }
+  T nup = nN;  // density of the plane above the current one
   for (int k0 = N - 2; k0 >= 0; k0 -= kBatch) {
-    T qv[kBatch], cv[kBatch];
+    T qv[kBatch], cv[kBatch], nv[kBatch];
 #pragma unroll
     for (int e = 0; e < kBatch; e++) {
       const size_t c = (size_t)max(k0 - e, 0) * plane + col;
       qv[e] = z.q[c];
-      cv[e] = z.cp[c];
+      cv[e] = z.minv[c];
+      nv[e] = __ldg(&n[c]);
     }
 #pragma unroll
     for (int e = 0; e < kBatch; e++) {
       const int k = k0 - e;
       if (k < 0) break;
       const size_t c = (size_t)k * plane + col;
-      qn = qv[e] - cv[e] * qn;
+      const T cp = zc(nv[e], nup) * cv[e];
+      nup = nv[e];
+      qn = qv[e] - cp * qn;
       z.q[c] = qn;
-      if ((k + 1) % S == 0) bprod = T(1);
-      bprod *= -cv[e];
-      z.bb[c] = bprod;
+      if (stored) {
+        if ((k + 1) % S == 0) bprod = T(1);
+        bprod *= -cp;
+        z.bb[c] = bprod;
+      }
     }
   }
   if (cyc) {
@@ -232,15 +268,22 @@ __global__ void k_zline_rhs(OpK o, const T *__restrict__ n, const T *__restrict_
 // Damped z-line Jacobi update: T' y = r by segments, Sherman-Morrison
 // closure of the periodic cycle, xn = xo + omega (y - s q - xo) (xo nullptr:
 // zero).  Block = 32 columns (consecutive x at one y) x P segments of S
-// cells; each phase loads its segment's operands at once so that one memory
-// latency covers the whole segment.
+// cells.  Bound by memory latency on the small levels and by L2 traffic on the
+// large ones.  FP32 with segments of 8 reads 5 words a cell instead of 9, and
+// its last operands are requested before the first barrier, so that two
+// memory latencies cover the solve.  Every thread runs the carried-value scan
+// over the segments itself (two barriers instead of four): 5.3 -> 3.9 us at
+// 32^3, 21.5 -> 15 us at 128^3.  Each phase keeps only the arrays that it
+// needs, so that two blocks of 512 threads fit an SM (with everything held
+// from the start, one block an SM: 7.5 against 6.4 us at 96^3).
 template <typename T, int S>
-__global__ void __launch_bounds__(32 * kMaxSeg) k_zline_seg(GridG g, ZlP<T> z, const T *__restrict__ r,
-                                                            const T *__restrict__ xo, T *__restrict__ xn,
-                                                            T omega) {
+__global__ void __launch_bounds__(32 * kMaxSeg, zl_stored<T>(S) ? 1 : 2)
+    k_zline_seg(GridG g, ZCoup<T> zc, const T *__restrict__ n, ZlP<T> z, const T *__restrict__ r,
+                const T *__restrict__ xo, T *__restrict__ xn, T omega) {
   ECS_PDL_ENTRY();
-  __shared__ T sA[kMaxSeg][33], sB[kMaxSeg][33], sIn[kMaxSeg][33];
-  __shared__ T sLast[32], sS[32];
+  constexpr bool kStored = zl_stored<T>(S);
+  __shared__ T sA[kMaxSeg][33], sB[kMaxSeg][33], sC[kMaxSeg][33], sD[kMaxSeg][33];
+  __shared__ T sLast[32];
   const int tx = threadIdx.x, p = threadIdx.y, P = blockDim.y;
   const int i = blockIdx.x * 32 + tx, j = blockIdx.y;
   const bool act = i < g.nx;
@@ -249,85 +292,123 @@ __global__ void __launch_bounds__(32 * kMaxSeg) k_zline_seg(GridG g, ZlP<T> z, c
   const int N = g.nz, k0 = p * S, k1 = min(N, k0 + S);
   const size_t c0 = (size_t)k0 * plane + col;
   auto in = [&](int q) { return act && k0 + q < k1; };
-  T loc[S];
+  T rv[S];          // r, then d, then y
+  T cv[S], fv[S];   // cp, fb
+  T qv[S], ov[kStored ? 1 : S];
+  T a0g = T(0), qden = T(0);
   // forward, from zero at the segment start
-  {
-    T rv[S], av[S], mv[S];
+  if constexpr (kStored) {
 #pragma unroll
     for (int q = 0; q < S; q++) {
       const size_t c = c0 + (size_t)q * plane;
       rv[q] = in(q) ? r[c] : T(0);
-      av[q] = in(q) ? z.a[c] : T(0);
-      mv[q] = in(q) ? z.minv[c] : T(0);
+      cv[q] = in(q) ? z.a[c] : T(0);
+      fv[q] = in(q) ? z.minv[c] : T(0);
     }
     T d = T(0);
 #pragma unroll
-    for (int q = 0; q < S; q++) {
-      if (in(q)) d = (rv[q] - av[q] * d) * mv[q];
-      loc[q] = d;
-    }
+    for (int q = 0; q < S; q++)
+      if (in(q)) {
+        d = (rv[q] - cv[q] * d) * fv[q];
+        rv[q] = d;
+      }
     sA[p][tx] = d;
-    sB[p][tx] = act ? z.fb[(size_t)(k1 - 1) * plane + col] : T(0);
-  }
-  __syncthreads();
-  if (p == 0) {
-    T din = T(0);
-    for (int pp = 0; pp < P; pp++) {
-      sIn[pp][tx] = din;
-      din = sA[pp][tx] + sB[pp][tx] * din;
-    }
-  }
-  __syncthreads();
-  // carried value in, then backward from zero at the segment end
-  {
-    const T din = sIn[p][tx];
-    T fv[S], cv[S];
+    sB[p][tx] = act && k0 < k1 ? z.fb[(size_t)(k1 - 1) * plane + col] : T(0);
+  } else {
+    T nv[S + 2];  // densities of planes k0 - 1 .. k0 + S
+    nv[0] = act && k0 > 0 && k0 < N ? n[c0 - plane] : T(0);
+    nv[S + 1] = act && k0 + S < N ? n[c0 + (size_t)S * plane] : T(0);
 #pragma unroll
     for (int q = 0; q < S; q++) {
       const size_t c = c0 + (size_t)q * plane;
-      fv[q] = in(q) ? z.fb[c] : T(0);
-      cv[q] = in(q) ? z.cp[c] : T(0);
+      rv[q] = in(q) ? r[c] : T(0);
+      nv[q + 1] = in(q) ? n[c] : T(0);
+      cv[q] = in(q) ? z.minv[c] : T(0);
     }
-    T y = T(0);
+    T d = T(0), fprod = T(1);
 #pragma unroll
-    for (int q = S - 1; q >= 0; q--) {
-      if (in(q)) y = (loc[q] + fv[q] * din) - cv[q] * y;
-      loc[q] = y;
-    }
-    // sA, sB are free again: the forward scan finished before the last barrier
-    sA[p][tx] = y;
-    sB[p][tx] = act ? z.bb[c0] : T(0);
-    if (p == P - 1) {  // y_{N-1}: nothing is carried into the last segment
-#pragma unroll
-      for (int q = 0; q < S; q++)
-        if (k0 + q == N - 1) sLast[tx] = loc[q];
-    }
-  }
-  __syncthreads();
-  if (p == 0) {
-    T yin = T(0);
-    for (int pp = P - 1; pp >= 0; pp--) {
-      sIn[pp][tx] = yin;
-      yin = sA[pp][tx] + sB[pp][tx] * yin;
-    }
-    sS[tx] = act ? (yin + z.a0g[col] * sLast[tx]) * z.qden[col] : T(0);  // yin = y_0
-  }
-  __syncthreads();
-  {
-    const T yin = sIn[p][tx], s = sS[tx];
-    T bv[S], qv[S], ov[S];
+    for (int q = 0; q < S; q++)
+      if (in(q)) {
+        const T a = k0 + q == 0 ? T(0) : zc(nv[q + 1], nv[q]);
+        const T up = k0 + q == N - 1 ? T(0) : zc(nv[q + 1], nv[q + 2]);
+        d = (rv[q] - a * d) * cv[q];
+        rv[q] = d;
+        fprod *= -(a * cv[q]);
+        fv[q] = fprod;
+        cv[q] = up * cv[q];
+      }
+    sA[p][tx] = d;
+    sB[p][tx] = k0 < k1 ? fprod : T(0);
 #pragma unroll
     for (int q = 0; q < S; q++) {
       const size_t c = c0 + (size_t)q * plane;
-      bv[q] = in(q) ? z.bb[c] : T(0);
       qv[q] = in(q) ? z.q[c] : T(0);
       ov[q] = (in(q) && xo) ? xo[c] : T(0);
     }
+  }
+  if (act) {
+    a0g = z.a0g[col];
+    qden = z.qden[col];
+  }
+  __syncthreads();
+  // the value carried in, then backward from zero at the segment end
+  {
+    T din = T(0);
+    for (int pp = 0; pp < p; pp++) din = sA[pp][tx] + sB[pp][tx] * din;
+    if constexpr (kStored) {
 #pragma unroll
-    for (int q = 0; q < S; q++) {
+      for (int q = 0; q < S; q++) {
+        const size_t c = c0 + (size_t)q * plane;
+        fv[q] = in(q) ? z.fb[c] : T(0);
+        cv[q] = in(q) ? z.cp[c] : T(0);
+      }
+    }
+    T y = T(0), bprod = T(1);
+#pragma unroll
+    for (int q = S - 1; q >= 0; q--) {
       if (in(q)) {
-        const T yk = loc[q] + bv[q] * yin;
-        xn[c0 + (size_t)q * plane] = ov[q] + omega * ((yk - s * qv[q]) - ov[q]);
+        y = (rv[q] + fv[q] * din) - cv[q] * y;
+        rv[q] = y;
+        if constexpr (!kStored) bprod *= -cv[q];
+        if (k0 + q == N - 1) sLast[tx] = y;  // y_{N-1}: nothing is carried into the last segment
+      }
+    }
+    if constexpr (kStored) bprod = in(0) ? z.bb[c0] : T(0);
+    sC[p][tx] = y;
+    sD[p][tx] = in(0) ? bprod : T(0);
+  }
+  __syncthreads();
+  {
+    T yin = T(0), run = T(0);
+    for (int pp = P - 1; pp >= 0; pp--) {
+      if (pp == p) yin = run;
+      run = sC[pp][tx] + sD[pp][tx] * run;
+    }
+    const T s = act ? (run + a0g * sLast[tx]) * qden : T(0);  // run = y_0
+    if constexpr (kStored) {
+#pragma unroll
+      for (int q = 0; q < S; q++) {
+        const size_t c = c0 + (size_t)q * plane;
+        fv[q] = in(q) ? z.bb[c] : T(0);
+        qv[q] = in(q) ? z.q[c] : T(0);
+      }
+    }
+    T bprod = T(1);
+#pragma unroll
+    for (int q = S - 1; q >= 0; q--) {
+      if (in(q)) {
+        const size_t c = c0 + (size_t)q * plane;
+        T o, bb;
+        if constexpr (kStored) {
+          o = xo ? xo[c] : T(0);
+          bb = fv[q];
+        } else {
+          o = ov[q];
+          bprod *= -cv[q];
+          bb = bprod;
+        }
+        const T yk = rv[q] + bb * yin;
+        xn[c] = o + omega * ((yk - s * qv[q]) - o);
       }
     }
   }
@@ -369,48 +450,9 @@ __global__ void k_restrict(GridG gf, GridG gc, const T *__restrict__ f, T *__res
   c[lin3(gc, I, J, K)] = s;
 }
 
-// The same full-weighting sum with the loops kept rolled (less code, for the
-// single-block cycle); the terms are added in the same order as k_restrict.
-template <typename T>
-__device__ __forceinline__ T restrict_at_rolled(const GridG &gf, const GridG &gc, const T *__restrict__ f, int I,
-                                                int J, int K) {
-  const bool semi = semi_z(gf, gc);
-  const int zl = semi ? 0 : -1, zc = semi ? K : 2 * K;
-  T s = T(0);
-#pragma unroll 1
-  for (int dk = zl; dk <= -zl; dk++) {
-    const T wk = semi ? T(1) : (dk == 0 ? T(0.5) : T(0.25));
-#pragma unroll 1
-    for (int dj = -1; dj <= 1; dj++) {
-      const T wj = dj == 0 ? T(0.5) : T(0.25);
-#pragma unroll 1
-      for (int di = -1; di <= 1; di++) {
-        const T wi = di == 0 ? T(0.5) : T(0.25);
-        s += wk * wj * wi * gval(f, gf, zc + dk, 2 * J + dj, 2 * I + di);
-      }
-    }
-  }
-  return s;
-}
-
-// Trilinear prolongation value at fine cell (i,j,k).
-template <typename T>
-__device__ __forceinline__ T prolong_at(const GridG &gf, const GridG &gc, const T *__restrict__ c, int i, int j,
-                                        int k) {
-  const bool semi = semi_z(gf, gc);
-  int i0 = i >> 1, j0 = j >> 1, k0 = semi ? k : k >> 1;
-  int ni = (i & 1) ? 2 : 1, nj = (j & 1) ? 2 : 1, nk = (!semi && (k & 1)) ? 2 : 1;
-  T wi = ni == 2 ? T(0.5) : T(1), wj = nj == 2 ? T(0.5) : T(1), wk = nk == 2 ? T(0.5) : T(1);
-  T s = T(0);
-  for (int a = 0; a < nk; a++)
-    for (int bq = 0; bq < nj; bq++)
-      for (int q = 0; q < ni; q++) s += gval(c, gc, k0 + a, j0 + bq, i0 + q);
-  return wi * wj * wk * s;
-}
-// f += P c.
-// The kernel's form: the coarse cells through the neighbour offsets of the
+// f += P c, trilinear: the coarse cells through the neighbour offsets of the
 // coarse cell (i/2, j/2, k/2); a term of the second cell along an axis is
-// added only for an odd index, in the order of prolong_at.
+// added only for an odd index, x innermost, then y, then z.
 template <typename T>
 __global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__restrict__ f) {
   ECS_PDL_ENTRY();
@@ -442,92 +484,188 @@ __global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__
 }
 
 // ---- whole V-cycle of the small levels in one thread block -------------------
-// The iterate, right-hand side, residual and scratch vectors of every small
-// level live in shared memory (s* are element offsets into it); the density
-// and the z-line factors are read-only and come through the L1 cache.
+// Levels of at most kSmallCells cells, all in one block of one thread a cell.
+// Every level's 11 row coefficients, its neighbour offsets (packed), its
+// z-line factors and its vectors live in shared memory (s* are offsets into
+// it, in elements; sn in 4-byte words of the integer part): the coefficients
+// and offsets are formed once per launch from the density, so that the
+// residual, right-hand side and transfer phases are a few shared-memory loads
+// and multiply-adds each.  The kernel runs each piece of its code once or a
+// few times per launch, so instruction fetch and the phases' latency bound it.
+// With the rows, wraps and index divisions redone in every phase and the
+// columns' recurrences through shared memory it took 24 us for 8^3 + 4^3 and
+// 70 us for a 6^3 coarsest level of 21 sweeps (FP32); 10 and 26 us in this
+// form.
 template <typename T>
 struct SmallLevel {
   OpK o;
-  const T *dens;   // in global memory, staged at sd
-  ZlP<T> z;        // in global memory, staged at sa, sc, sm, sq (cells) and s0, sqd (columns)
-  int sx, sb, sr, st;
-  int sd, sa, sc, sm, sq, s0, sqd;
+  const T *dens, *minv, *q, *a0g, *qden;  // in global memory
+  int sx, sb, sr, st;                     // vectors
+  int sco, sa, sc, sm, sq, s0, sqd;       // coefficients [11][n], factors (cells), column scalars
+  int sn;                                 // packed neighbour offsets [3][n]
 };
 constexpr int kMaxSmall = 8;
 template <typename T>
 struct SmallCycle {
-  int nl;
-  const T *cinv;  // transposed inverse of the coarsest operator, or nullptr; staged at scinv
-  int scinv;
+  int nl, ints;   // ints: element offset of the integer part
+  const T *cinv;  // transposed inverse of the coarsest operator, or nullptr
   SmallLevel<T> lv[kMaxSmall];
 };
-constexpr int kSmallThreads = 1024;
+constexpr size_t kSmallCells = 512;
+constexpr int kSmallThreads = (int)kSmallCells;
+// Planes that a column's thread keeps in registers; deeper columns (a
+// reflecting z is not coarsened) run their recurrences through shared memory.
+constexpr int kSmallPlanes = 8;
 
-// Thomas solve of one column with all vectors in shared memory: rin (right-
-// hand side) may be the same array as dp (the substitution scratch).
-// One column's z-line solve with the factors staged in shared memory.
+// Neighbour offsets of a small level's cell in three words: (xm, xp, ym),
+// (yp, zm, zp) as signed 10-bit fields, (i, j, k) as 10-bit fields.  Offsets
+// are below 512 in magnitude; kNoNbr marks a ghost, whose value is 0.
+constexpr int kNoNbr = -512;
+__device__ __forceinline__ unsigned pack3(int a, int b, int c) {
+  return ((unsigned)a & 1023u) | (((unsigned)b & 1023u) << 10) | (((unsigned)c & 1023u) << 20);
+}
+__device__ __forceinline__ int field_s(unsigned w, int f) { return (int)(w << (22 - 10 * f)) >> 22; }
+__device__ __forceinline__ int field_u(unsigned w, int f) { return (int)((w >> (10 * f)) & 1023u); }
+struct SmallNbr {
+  int xm, xp, ym, yp, zm, zp;
+};
+__device__ __forceinline__ SmallNbr small_nbr(const unsigned *nb, int n, int c) {
+  const unsigned w0 = nb[c], w1 = nb[n + c];
+  return {field_s(w0, 0), field_s(w0, 1), field_s(w0, 2), field_s(w1, 0), field_s(w1, 1), field_s(w1, 2)};
+}
 template <typename T>
-__device__ __forceinline__ void zline_col_s(const GridG &g, const ZlP<T> &z, const T *rin, T *dp,
-                                            const T *xo, T *xn, T omega, int col) {
-  const int plane = g.nx * g.ny, N = g.nz;
+__device__ __forceinline__ T sval(const T *f, int c, int off, bool valid) {
+  return valid ? f[c + off] : T(0);
+}
+// f at the row's entries, in the order of off_i/off_j/off_k; x and y are
+// periodic on every grid the solver takes, so only z has ghosts.
+template <typename T>
+__device__ __forceinline__ void small_row(const T *f, int c, const SmallNbr &q, T xe[11]) {
+  xe[0] = f[c + q.xp];
+  xe[1] = f[c + q.xm];
+  xe[2] = f[c + q.yp];
+  xe[3] = f[c + q.ym];
+  xe[4] = sval(f, c, q.zp, q.zp != kNoNbr);
+  xe[5] = sval(f, c, q.zm, q.zm != kNoNbr);
+  xe[6] = f[c + q.xp + q.yp];
+  xe[7] = f[c + q.xp + q.ym];
+  xe[8] = f[c + q.xm + q.yp];
+  xe[9] = f[c + q.xm + q.ym];
+  xe[10] = f[c];
+}
+
+// One column's z-line solve in shared memory: the right-hand side at rin (may
+// be the same array as the substitution scratch dp), xo and xn the iterate in
+// and out (all offsets into sm; xo < 0: zero).
+template <typename T>
+__device__ __forceinline__ void zline_col_s(const SmallLevel<T> &L, T *sm, int rin, int dp, int xo, int xn, T omega,
+                                            int col) {
+  const int plane = L.o.g.nx * L.o.g.ny, N = L.o.g.nz;
+  const T *a = sm + L.sa + col, *cp = sm + L.sc + col, *minv = sm + L.sm + col, *q = sm + L.sq + col;
+  const T *rp = sm + rin + col, *op = sm + (xo < 0 ? 0 : xo) + col;
+  T *d_ = sm + dp + col, *xp = sm + xn + col;
+  const T a0g = sm[L.s0 + col], qden = sm[L.sqd + col];
+  if (N <= kSmallPlanes) {  // operands first, then the recurrences in registers
+    T y[kSmallPlanes], av[kSmallPlanes], mv[kSmallPlanes], cv[kSmallPlanes];
+#pragma unroll
+    for (int k = 0; k < kSmallPlanes; k++)
+      if (k < N) {
+        y[k] = rp[k * plane];
+        av[k] = a[k * plane];
+        mv[k] = minv[k * plane];
+        cv[k] = cp[k * plane];
+      }
+    T d = T(0);
+#pragma unroll
+    for (int k = 0; k < kSmallPlanes; k++)
+      if (k < N) {
+        d = (y[k] - av[k] * d) * mv[k];
+        y[k] = d;
+      }
+    const T yN = d;
+    T yk = d;
+#pragma unroll
+    for (int k = kSmallPlanes - 2; k >= 0; k--)
+      if (k < N - 1) {
+        yk = y[k] - cv[k] * yk;
+        y[k] = yk;
+      }
+    const T s = (yk + a0g * yN) * qden;
+#pragma unroll
+    for (int k = 0; k < kSmallPlanes; k++)
+      if (k < N) {
+        const T ov = xo < 0 ? T(0) : op[k * plane];
+        xp[k * plane] = ov + omega * ((y[k] - s * q[k * plane]) - ov);
+      }
+    return;
+  }
   T d = T(0);
   for (int k = 0; k < N; k++) {
-    const int c = k * plane + col;
-    d = (rin[c] - z.a[c] * d) * z.minv[c];
-    dp[c] = d;
+    d = (rp[k * plane] - a[k * plane] * d) * minv[k * plane];
+    d_[k * plane] = d;
   }
   const T yN = d;
   T y = d;
   for (int k = N - 2; k >= 0; k--) {
-    const int c = k * plane + col;
-    y = dp[c] - z.cp[c] * y;
-    dp[c] = y;
+    y = d_[k * plane] - cp[k * plane] * y;
+    d_[k * plane] = y;
   }
-  const T s = (y + z.a0g[col] * yN) * z.qden[col];
+  const T s = (y + a0g * yN) * qden;
   for (int k = 0; k < N; k++) {
-    const int c = k * plane + col;
-    const T ov = xo ? xo[c] : T(0);
-    xn[c] = ov + omega * ((dp[c] - s * z.q[c]) - ov);
+    const T ov = xo < 0 ? T(0) : op[k * plane];
+    xp[k * plane] = ov + omega * ((d_[k * plane] - s * q[k * plane]) - ov);
   }
 }
 
-// A small level's density and z-line factors as staged in shared memory.
+// `sweeps` damped z-line Jacobi sweeps of level L: the first from xo (an
+// offset; < 0: zero) into xn, the next ones back and forth between xn and
+// alt.  Called up to three times a launch, so it is kept out of line (one copy
+// of its code to fetch); the arrays go by their offsets, so that every access
+// stays a shared-memory access.  A thread's coefficients and neighbour
+// offsets stay in registers over the sweeps (one cell a thread).
 template <typename T>
-struct SmallView {
-  const T *dens;
-  ZlP<T> z;
-};
-template <typename T>
-__device__ __forceinline__ SmallView<T> staged(const SmallLevel<T> &L, T *sm) {
-  SmallView<T> v;
-  v.dens = sm + L.sd;
-  v.z = L.z;
-  v.z.a = sm + L.sa; v.z.cp = sm + L.sc; v.z.minv = sm + L.sm; v.z.q = sm + L.sq;
-  v.z.a0g = sm + L.s0; v.z.qden = sm + L.sqd;
-  return v;
-}
-
-// One damped z-line Jacobi sweep of level L from xo (nullptr: zero) into xn.
-// The single-block cycle runs its code once per launch, so its time goes to
-// instruction fetch as much as to arithmetic: the sweep, called three times,
-// is kept out of line (one copy of its code).
-template <typename T>
-__device__ __noinline__ void blk_sweep(const SmallLevel<T> &L, T *sm, const T *b, const T *xo, T *xn, T omega) {
-  const GridG &g = L.o.g;
-  const SmallView<T> v = staged(L, sm);
-  T *r = sm + L.sr;
-  const T *rin = b;
-  if (xo) {
-    for (unsigned c = threadIdx.x; c < g.n; c += blockDim.x) {
-      int i, j, k;
-      cell_ijk(c, g, i, j, k);
-      r[c] = zline_rhs_at(v.dens, b, xo, L.o, i, j, k, c);
+__device__ __noinline__ void blk_sweep(const SmallLevel<T> &L, int ints_off, int b, int xo, int xn, int alt,
+                                       int sweeps, T omega) {
+  extern __shared__ unsigned char small_smem[];
+  T *sm = reinterpret_cast<T *>(small_smem);
+  const unsigned *ints = reinterpret_cast<const unsigned *>(sm + ints_off);
+  const int n = (int)L.o.g.n, ncol = L.o.g.nx * L.o.g.ny, c = threadIdx.x;
+  const bool live = c < n;
+  SmallNbr q = {0, 0, 0, 0, 0, 0};
+  T v[8], bc = T(0);
+  if (live) {
+    q = small_nbr(ints + L.sn, n, c);
+    const T *co = sm + L.sco + c;
+#pragma unroll
+    for (int e = 0; e < 8; e++) v[e] = co[(e < 4 ? e : e + 2) * n];
+    bc = sm[b + c];
+  }
+#pragma unroll 1
+  for (int sw = 0; sw < sweeps; sw++) {
+    int rin = b;
+    if (xo >= 0) {
+      if (live) {
+        const T *x = sm + xo + c;
+        T s = bc;
+        s -= v[0] * x[q.xp];
+        s -= v[1] * x[q.xm];
+        s -= v[2] * x[q.yp];
+        s -= v[3] * x[q.ym];
+        s -= v[4] * x[q.xp + q.yp];
+        s -= v[5] * x[q.xp + q.ym];
+        s -= v[6] * x[q.xm + q.yp];
+        s -= v[7] * x[q.xm + q.ym];
+        sm[L.sr + c] = s;
+      }
+      __syncthreads();
+      rin = L.sr;
     }
+    for (int col = threadIdx.x; col < ncol; col += blockDim.x) zline_col_s<T>(L, sm, rin, L.sr, xo, xn, omega, col);
     __syncthreads();
-    rin = r;
+    xo = xn;
+    xn = alt;
+    alt = xo;
   }
-  for (int col = threadIdx.x; col < g.nx * g.ny; col += blockDim.x) zline_col_s<T>(g, v.z, rin, r, xo, xn, omega, col);
-  __syncthreads();
 }
 
 // x_out = M(l0) b_in: V(1,1) over levels l0..l0+nl-1, all in this block.
@@ -537,52 +675,80 @@ __global__ void __launch_bounds__(kSmallThreads) k_vcycle_small(SmallCycle<T> sc
   ECS_PDL_ENTRY();
   extern __shared__ unsigned char small_smem[];
   T *sm = reinterpret_cast<T *>(small_smem);
+  unsigned *ints = reinterpret_cast<unsigned *>(sm + sc.ints);
   const int nl = sc.nl;
-  // stage the levels' densities and z-line factors, the coarse inverse and
-  // the right-hand side: every later load is a shared-memory load
+  // row coefficients, neighbour offsets and z-line factors of every level
+  // (the coarsest of a direct solve needs the offsets only), and the
+  // right-hand side
+#pragma unroll 1
   for (int l = 0; l < nl; l++) {
     const SmallLevel<T> &L = sc.lv[l];
-    const unsigned n = (unsigned)L.o.g.n, ncol = (unsigned)(L.o.g.nx * L.o.g.ny);
-    for (unsigned c = threadIdx.x; c < n; c += blockDim.x) {
-      sm[L.sd + c] = __ldg(&L.dens[c]);
-      sm[L.sa + c] = __ldg(&L.z.a[c]);
-      sm[L.sc + c] = __ldg(&L.z.cp[c]);
-      sm[L.sm + c] = __ldg(&L.z.minv[c]);
-      sm[L.sq + c] = __ldg(&L.z.q[c]);
-    }
-    for (unsigned c = threadIdx.x; c < ncol; c += blockDim.x) {
-      sm[L.s0 + c] = __ldg(&L.z.a0g[c]);
-      sm[L.sqd + c] = __ldg(&L.z.qden[c]);
-    }
-  }
-  if (sc.cinv) {
-    const unsigned nn = (unsigned)(sc.lv[nl - 1].o.g.n * sc.lv[nl - 1].o.g.n);
-    for (unsigned e = threadIdx.x; e < nn; e += blockDim.x) sm[sc.scinv + e] = __ldg(&sc.cinv[e]);
-  }
-  {
-    const SmallLevel<T> &L = sc.lv[0];
-    for (unsigned c = threadIdx.x; c < L.o.g.n; c += blockDim.x) sm[L.sb + c] = b_in[c];
-    __syncthreads();
-  }
-  // down
-  for (int l = 0; l < nl - 1; l++) {
-    const SmallLevel<T> &L = sc.lv[l];
-    const GridG &g = L.o.g;
-    T *b = sm + L.sb, *t = sm + L.st, *r = sm + L.sr;
-    blk_sweep(L, sm, b, (const T *)nullptr, t, omega);
-    const T *dl = sm + L.sd;
-    for (unsigned c = threadIdx.x; c < g.n; c += blockDim.x) {
+    const int n = (int)L.o.g.n, ncol = L.o.g.nx * L.o.g.ny;
+    const bool direct = l == nl - 1 && sc.cinv;
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
       int i, j, k;
-      cell_ijk(c, g, i, j, k);
-      r[c] = b[c] - apply_row(dl, (const T *)t, L.o, i, j, k);
+      cell_ijk((unsigned)c, L.o.g, i, j, k);
+      const Nbr q = nbr_of(L.o.g, i, j, k);
+      ints[L.sn + c] = pack3(q.xm, q.xp, q.ym);
+      ints[L.sn + n + c] = pack3(q.yp, q.vzm ? q.zm : kNoNbr, q.vzp ? q.zp : kNoNbr);
+      ints[L.sn + 2 * n + c] = pack3(i, j, k);
+      if (direct) continue;
+      const T mi = __ldg(&L.minv[c]);
+      sm[L.sm + c] = mi;
+      sm[L.sq + c] = __ldg(&L.q[c]);
+      T v[11];
+      row11_n(L.dens, L.o, q, v);
+#pragma unroll
+      for (int e = 0; e < 11; e++) sm[L.sco + e * n + c] = v[e];
+      sm[L.sa + c] = k == 0 ? T(0) : v[5];
+      sm[L.sc + c] = (k == L.o.g.nz - 1 ? T(0) : v[4]) * mi;
+    }
+    if (!direct)
+      for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
+        sm[L.s0 + c] = __ldg(&L.a0g[c]);
+        sm[L.sqd + c] = __ldg(&L.qden[c]);
+      }
+    if (l == 0)
+      for (int c = threadIdx.x; c < n; c += blockDim.x) sm[L.sb + c] = b_in[c];
+  }
+  __syncthreads();
+  // down
+#pragma unroll 1
+  for (int l = 0; l < nl - 1; l++) {
+    const SmallLevel<T> &L = sc.lv[l], &C = sc.lv[l + 1];
+    const GridG &g = L.o.g, &gc = C.o.g;
+    const int n = (int)g.n, nc = (int)gc.n;
+    T *b = sm + L.sb, *t = sm + L.st, *r = sm + L.sr;
+    blk_sweep(L, sc.ints, L.sb, -1, L.st, L.st, 1, omega);
+    const T *co = sm + L.sco;
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+      T xe[11];
+      small_row((const T *)t, c, small_nbr(ints + L.sn, n, c), xe);
+      T s = T(0);
+#pragma unroll
+      for (int e = 0; e < 11; e++) s += co[e * n + c] * xe[e];
+      r[c] = b[c] - s;
     }
     __syncthreads();
-    const SmallLevel<T> &C = sc.lv[l + 1];
-    T *cb = sm + C.sb;
-    for (unsigned c = threadIdx.x; c < C.o.g.n; c += blockDim.x) {
-      int I, J, K;
-      cell_ijk(c, C.o.g, I, J, K);
-      cb[c] = restrict_at_rolled(g, C.o.g, (const T *)r, I, J, K);
+    // full weighting, the terms in the order of k_restrict
+    const bool semi = semi_z(g, gc);
+    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+      const unsigned w = ints[C.sn + 2 * nc + c];
+      const int f = ((semi ? field_u(w, 2) : 2 * field_u(w, 2)) * g.ny + 2 * field_u(w, 1)) * g.nx + 2 * field_u(w, 0);
+      const SmallNbr q = small_nbr(ints + L.sn, n, f);
+      const int oz[3] = {q.zm, 0, q.zp}, oy[3] = {q.ym, 0, q.yp}, ox[3] = {q.xm, 0, q.xp};
+      T s = T(0);
+#pragma unroll
+      for (int dk = 0; dk < 3; dk++) {
+        if ((semi && dk != 1) || oz[dk] == kNoNbr) continue;
+        const T wk = semi ? T(1) : (dk == 1 ? T(0.5) : T(0.25));
+#pragma unroll
+        for (int dj = 0; dj < 3; dj++)
+#pragma unroll
+          for (int di = 0; di < 3; di++)
+            s += wk * (dj == 1 ? T(0.5) : T(0.25)) * (di == 1 ? T(0.5) : T(0.25)) * r[f + oz[dk] + oy[dj] + ox[di]];
+      }
+      sm[C.sb + c] = s;
     }
     __syncthreads();
   }
@@ -592,47 +758,50 @@ __global__ void __launch_bounds__(kSmallThreads) k_vcycle_small(SmallCycle<T> sc
     const SmallLevel<T> &L = sc.lv[nl - 1];
     const int n = (int)L.o.g.n;
     const T *b = sm + L.sb;
-    const T *ci = sm + sc.scinv;
     const int lane = threadIdx.x & 31;
     for (int r = threadIdx.x >> 5; r < n; r += blockDim.x >> 5) {
       T acc = T(0);
-      for (int k = lane; k < n; k += 32) acc += ci[k * n + r] * b[k];
+      for (int k = lane; k < n; k += 32) acc += __ldg(&sc.cinv[k * n + r]) * b[k];
       for (int s2 = 16; s2 >= 1; s2 >>= 1) acc += __shfl_xor_sync(ECS_FULL_MASK, acc, s2);
       if (lane == 0) sm[L.sx + r] = acc;
     }
     __syncthreads();
   } else {
+    // into x after an odd number of sweeps
     const SmallLevel<T> &L = sc.lv[nl - 1];
-    const T *b = sm + L.sb;
-    T *cur = sm + L.sx, *nxt = sm + L.st;
-    for (int sw = 0; sw < coarse_sweeps; sw++) {
-      blk_sweep(L, sm, b, sw == 0 ? (const T *)nullptr : cur, nxt, omega);
-      T *tmp = cur;
-      cur = nxt;
-      nxt = tmp;
-    }
-    if (cur != sm + L.sx) {
-      for (unsigned c = threadIdx.x; c < L.o.g.n; c += blockDim.x) sm[L.sx + c] = cur[c];
-      __syncthreads();
-    }
+    const int first = coarse_sweeps & 1 ? L.sx : L.st;
+    blk_sweep(L, sc.ints, L.sb, -1, first, L.sx + L.st - first, coarse_sweeps, omega);
   }
   // up
+#pragma unroll 1
   for (int l = nl - 2; l >= 0; l--) {
     const SmallLevel<T> &L = sc.lv[l], &C = sc.lv[l + 1];
-    const GridG &g = L.o.g;
+    const GridG &g = L.o.g, &gc = C.o.g;
+    const int n = (int)g.n, nc = (int)gc.n;
     T *t = sm + L.st;
     const T *cx = sm + C.sx;
-    for (unsigned c = threadIdx.x; c < g.n; c += blockDim.x) {
-      int i, j, k;
-      cell_ijk(c, g, i, j, k);
-      t[c] += prolong_at(g, C.o.g, cx, i, j, k);
+    // trilinear prolongation, the terms in the order of k_prolong_add
+    const bool semi = semi_z(g, gc);
+    for (int c = threadIdx.x; c < n; c += blockDim.x) {
+      const unsigned w = ints[L.sn + 2 * n + c];
+      const int i = field_u(w, 0), j = field_u(w, 1), k = field_u(w, 2);
+      const int q0 = ((semi ? k : k >> 1) * gc.ny + (j >> 1)) * gc.nx + (i >> 1);
+      const SmallNbr q = small_nbr(ints + C.sn, nc, q0);
+      const bool ti = i & 1, tj = j & 1, tk = !semi && (k & 1);
+      T s = T(0);
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        if (((e & 1) && !ti) || ((e & 2) && !tj) || ((e & 4) && (!tk || q.zp == kNoNbr))) continue;
+        s += cx[q0 + ((e & 4) ? q.zp : 0) + ((e & 2) ? q.yp : 0) + ((e & 1) ? q.xp : 0)];
+      }
+      t[c] += (ti ? T(0.5) : T(1)) * (tj ? T(0.5) : T(1)) * (tk ? T(0.5) : T(1)) * s;
     }
     __syncthreads();
-    blk_sweep(L, sm, sm + L.sb, t, sm + L.sx, omega);
+    blk_sweep(L, sc.ints, L.sb, L.st, L.sx, L.sx, 1, omega);
   }
   {
     const SmallLevel<T> &L = sc.lv[0];
-    for (unsigned c = threadIdx.x; c < L.o.g.n; c += blockDim.x) x_out[c] = sm[L.sx + c];
+    for (int c = threadIdx.x; c < (int)L.o.g.n; c += blockDim.x) x_out[c] = sm[L.sx + c];
   }
 }
 
@@ -1383,8 +1552,12 @@ int mg_alloc(EcsCtx *ctx) {
     L.nx = nx; L.ny = ny; L.nz = nz;
     L.n = (size_t)nx * ny * nz;
     L.hx = hx; L.hy = hy; L.hz = hz;
-    T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_a, &L.zl_cp, &L.zl_minv, &L.zl_q, &L.zl_fb, &L.zl_bb};
+    T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_minv, &L.zl_q};
     for (auto a : arr) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
+    if (zl_stored<T>(seg_len<T>(nz))) {
+      T **more[] = {&L.zl_a, &L.zl_cp, &L.zl_fb, &L.zl_bb};
+      for (auto a : more) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
+    }
     ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_a0g, (size_t)nx * ny * sizeof(T)));
     ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_qden, (size_t)nx * ny * sizeof(T)));
     mg.lv.push_back(L);
@@ -1457,9 +1630,9 @@ template <typename T>
 int zline_factor(EcsCtx *ctx, MgLevel<T> &L, cudaStream_t s) {
   const int ncol = L.nx * L.ny;
   const OpK o = op_level(ctx, L);
-  ecs_launch_pdl(k_zline_rows<T>, blocks3(o.g), threads3(), 0, s, o, L.dens, L.x, L.b, L.r);  // x, b, r are free here
+  ecs_launch_pdl(k_zline_rows<T>, blocks3(o.g), threads3(), 0, s, o, L.dens, L.r);  // r is free here
   ECS_LAUNCHED(ctx);
-  ecs_launch_pdl(k_zline_setup<T>, ecs_div_up(ncol, kColBlock), kColBlock, 0, s, o.g, L.x, L.b, L.r, zl_of(L), seg_len<T>(L.nz));
+  ecs_launch_pdl(k_zline_setup<T>, ecs_div_up(ncol, kColBlock), kColBlock, 0, s, o.g, z_coupling<T>(o), L.dens, L.r, zl_of(L), seg_len<T>(L.nz));
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
@@ -1556,32 +1729,46 @@ int sweep(EcsCtx *ctx, MgLevel<T> &L, const T *b, const T *xo, T *xn) {
     r = L.r;
   }
   const int S = seg_len<T>(L.nz);
+  const ZCoup<T> zc = z_coupling<T>(o);
   const dim3 grid((unsigned)((L.nx + 31) / 32), (unsigned)L.ny);
   const dim3 block(32, (unsigned)((L.nz + S - 1) / S));
   if (S == 8)
-    ecs_launch_pdl(k_zline_seg<T, 8>, grid, block, 0, ctx->stream, o.g, zl_of(L), r, xo, xn, kOmega<T>());
+    ecs_launch_pdl(k_zline_seg<T, 8>, grid, block, 0, ctx->stream, o.g, zc, L.dens, zl_of(L), r, xo, xn, kOmega<T>());
   else if (S == 16)
-    ecs_launch_pdl(k_zline_seg<T, 16>, grid, block, 0, ctx->stream, o.g, zl_of(L), r, xo, xn, kOmega<T>());
+    ecs_launch_pdl(k_zline_seg<T, 16>, grid, block, 0, ctx->stream, o.g, zc, L.dens, zl_of(L), r, xo, xn, kOmega<T>());
   else if (S == 32)
-    ecs_launch_pdl(k_zline_seg<T, 32>, grid, block, 0, ctx->stream, o.g, zl_of(L), r, xo, xn, kOmega<T>());
+    ecs_launch_pdl(k_zline_seg<T, 32>, grid, block, 0, ctx->stream, o.g, zc, L.dens, zl_of(L), r, xo, xn, kOmega<T>());
   else
-    ecs_launch_pdl(k_zline_seg<T, 64>, grid, block, 0, ctx->stream, o.g, zl_of(L), r, xo, xn, kOmega<T>());
+    ecs_launch_pdl(k_zline_seg<T, 64>, grid, block, 0, ctx->stream, o.g, zc, L.dens, zl_of(L), r, xo, xn, kOmega<T>());
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
 
-constexpr size_t kSmallCells = 512;
 constexpr size_t kSmallSmem = 200 * 1024;  // shared memory of the single-block cycle
 
-// Shared memory of a single-block cycle over levels l..: per level 4
-// vectors, the staged density and 4 z-line factor arrays, 2 column arrays;
-// the coarse inverse.
+// Layout of a single-block cycle over levels l.. in shared memory (offsets in
+// sc, if given): per level 4 vectors, 11 row coefficients and 4 z-line factor
+// arrays, 2 column arrays, and 3 words a cell of neighbour offsets at the end.
+// Returns its bytes: at most 164 B a cell and 16 B a column in FP64, for the
+// at most 683 cells that such levels have together.
 template <typename T>
-size_t small_bytes(const Multigrid<T> &mg, size_t l) {
-  size_t words = 0;
-  for (size_t q = l; q < mg.lv.size(); q++) words += mg.lv[q].n * 9 + (size_t)mg.lv[q].nx * mg.lv[q].ny * 2;
-  if (mg.cinv) words += mg.lv.back().n * mg.lv.back().n;
-  return words * sizeof(T);
+size_t small_layout(const Multigrid<T> &mg, size_t l, SmallCycle<T> *sc) {
+  int off = 0, ni = 0;
+  for (size_t q = l; q < mg.lv.size(); q++) {
+    const int n = (int)mg.lv[q].n, nc = mg.lv[q].nx * mg.lv[q].ny;
+    if (sc) {
+      SmallLevel<T> &S = sc->lv[q - l];
+      S.sx = off; S.sb = off + n; S.sr = off + 2 * n; S.st = off + 3 * n;
+      S.sco = off + 4 * n;
+      S.sa = off + 15 * n; S.sc = off + 16 * n; S.sm = off + 17 * n; S.sq = off + 18 * n;
+      S.s0 = off + 19 * n; S.sqd = off + 19 * n + nc;
+      S.sn = ni;
+    }
+    off += 19 * n + 2 * nc;
+    ni += 3 * n;
+  }
+  if (sc) sc->ints = off;
+  return (size_t)off * sizeof(T) + (size_t)ni * sizeof(unsigned);
 }
 
 // One V(1,1) cycle on level l: xout = M(l) b, zero initial guess.  Levels of
@@ -1591,26 +1778,18 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
   Multigrid<T> &mg = mg_of<T>(ctx);
   MgLevel<T> &L = mg.lv[l];
   int rc;
-  if (L.n <= kSmallCells && mg.lv.size() - l <= (size_t)kMaxSmall && small_bytes(mg, l) <= kSmallSmem) {
+  if (L.n <= kSmallCells && mg.lv.size() - l <= (size_t)kMaxSmall && small_layout<T>(mg, l, nullptr) <= kSmallSmem) {
     SmallCycle<T> sc;
     sc.nl = (int)(mg.lv.size() - l);
     sc.cinv = mg.cinv;
-    int off = 0;
+    const size_t bytes = small_layout<T>(mg, l, &sc);
     for (int q = 0; q < sc.nl; q++) {
       MgLevel<T> &M = mg.lv[l + q];
       SmallLevel<T> &S = sc.lv[q];
       S.o = op_level(ctx, M);
       S.dens = M.dens;
-      S.z = zl_of(M);
-      const int nq = (int)M.n, nc = M.nx * M.ny;
-      S.sx = off; S.sb = off + nq; S.sr = off + 2 * nq; S.st = off + 3 * nq;
-      S.sd = off + 4 * nq; S.sa = off + 5 * nq; S.sc = off + 6 * nq; S.sm = off + 7 * nq; S.sq = off + 8 * nq;
-      S.s0 = off + 9 * nq; S.sqd = off + 9 * nq + nc;
-      off += 9 * nq + 2 * nc;
+      S.minv = M.zl_minv; S.q = M.zl_q; S.a0g = M.zl_a0g; S.qden = M.zl_qden;
     }
-    sc.scinv = off;
-    if (sc.cinv) off += (int)(mg.lv.back().n * mg.lv.back().n);
-    const size_t bytes = (size_t)off * sizeof(T);
     static std::atomic<bool> attr_set[2];  // zero-initialised: false
     if (!attr_set[sizeof(T) == 8]) {
       ECS_CUDA(ctx, cudaFuncSetAttribute(k_vcycle_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));

@@ -166,34 +166,6 @@ __device__ __forceinline__ void row_x(const T *__restrict__ x, const Nbr &q, T x
   xe[10] = x[q.c];
 }
 
-// (A x)(k,j,i)
-template <typename T>
-__device__ __forceinline__ T apply_row(const T *__restrict__ n, const T *__restrict__ x, const OpK &o, int i,
-                                       int j, int k) {
-  T v[11];
-  row11(n, o, i, j, k, v);
-  T s = T(0);
-#pragma unroll
-  for (int e = 0; e < 11; e++) s += v[e] * gval(x, o.g, k + off_k(e), j + off_j(e), i + off_i(e));
-  return s;
-}
-
-// b - A_xy x at (k,j,i), A_xy = the 8 in-plane entries of the row.
-template <typename T>
-__device__ __forceinline__ T zline_rhs_at(const T *__restrict__ n, const T *__restrict__ b,
-                                          const T *__restrict__ x, const OpK &o, int i, int j, int k,
-                                          unsigned c) {
-  T v[11];
-  row11(n, o, i, j, k, v);
-  T s = b[c];
-#pragma unroll
-  for (int e = 0; e < 10; e++) {
-    if (e == 4 || e == 5) continue;
-    s -= v[e] * gval(x, o.g, k, j + off_j(e), i + off_i(e));
-  }
-  return s;
-}
-
 // Operator scale factors for spacing (hx, hy, hz), src/lhs.c:366-375.  The
 // constant-coefficient Laplacian of -lhs laplacian (ComputeLaplacianLHS3D,
 // src/lhs.c:101-191: 1/h^2 off the diagonal, minus their sum on it, the same
