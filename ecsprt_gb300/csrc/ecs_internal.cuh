@@ -65,6 +65,14 @@ struct MgLevel {
   T *zl_a0g = nullptr, *zl_qden = nullptr;  // per-column Sherman-Morrison scalars
 };
 
+// Thread-block cluster that runs the sweeps of the coarsest level (ctas = 0:
+// none).
+struct CoarseShape {
+  int ctas = 0, rows = 0, threads = 0;  // CTAs, rows of the largest CTA, threads a CTA
+  int ew = 0;                           // plane stride of the iterate
+  size_t smem = 0;
+};
+
 template <typename T>
 struct Multigrid {
   std::vector<MgLevel<T>> lv;
@@ -72,6 +80,7 @@ struct Multigrid {
   // explicit inverse of the coarsest operator (transposed), when it is small
   T *cinv = nullptr;
   T *cwork = nullptr;  // Gauss-Jordan work matrix [n][2n]
+  CoarseShape cluster;
 };
 
 // Instantiated graph of a whole potential solve (refinement sweeps, each an

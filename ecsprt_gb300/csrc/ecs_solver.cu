@@ -26,10 +26,14 @@
 #include <math.h>
 #include <string.h>
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <vector>
 
 #include "ecs_stencil.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -805,6 +809,218 @@ __global__ void __launch_bounds__(kSmallThreads) k_vcycle_small(SmallCycle<T> sc
   }
 }
 
+// ---- sweeps of a coarsest level too large for the direct solve ---------------
+// A grid whose axes turn odd early ends in a coarsest level of thousands of
+// cells, solved by kCoarseSweeps damped z-line sweeps.  As two launches a sweep
+// (right-hand side, z-line solve) the sweeps are launch latency, some 5 us
+// each and half of a solve and more.  Here one
+// thread-block cluster runs them all: the rows of the level are split over
+// its CTAs, the density, the iterate and its halo rows live in shared memory,
+// the right-hand side and the factors in registers, and each CTA writes its
+// edge rows into its neighbours' halos through distributed shared memory
+// before the cluster barrier that ends a sweep.  Thread (p, column) owns
+// segment p of the column, as in k_zline_seg, with the same operations in the
+// same order.  FP32 only: sixteen SMs hold too few FP64 units (the launches
+// over all SMs are faster there).  Bound by the latency of a sweep's three
+// barriers and, from some 20,000 cells on, by instruction issue on sixteen
+// SMs: solves of 30^3 (coarsest 15^3) 1.19 -> 0.90 ms, 66 x 54 x 42 (33 x 27 x
+// 21) 2.20 -> 1.68 ms, 100 x 72 x 50 (50 x 36 x 25) 3.50 -> 3.42 ms.
+constexpr int kClusterMax = 16;
+constexpr int kClusterSeg = 8;
+constexpr size_t kClusterSmem = 220 * 1024;
+__host__ __device__ __forceinline__ int row_begin(int ny, int ctas, int r) { return (int)((long long)ny * r / ctas); }
+
+// Planes of the iterate are EW elements apart (its columns and halo rows,
+// rounded up to a constant, so that a column's loads differ by immediates).
+template <typename T, int EW, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_coarse_sweeps(OpK o, ZCoup<T> zc, const T *__restrict__ dens, ZlP<T> z, const T *__restrict__ b,
+                    T *__restrict__ xout, int rows, int sweeps, T omega) {
+  ECS_PDL_ENTRY();
+  constexpr int S = kClusterSeg;
+  extern __shared__ __align__(16) unsigned char coarse_smem[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int nx = o.g.nx, ny = o.g.ny, N = o.g.nz;
+  const int W = rows * nx;  // columns of a CTA
+  const int P = (N + S - 1) / S, NP = P * S;
+  float4 *C = reinterpret_cast<float4 *>(coarse_smem);  // [2][N][W]: in-plane row entries 0-3 and 6-9
+  T *X = reinterpret_cast<T *>(C + 2 * N * W);          // [2][NP][EW]: rows -1 .. R, planes past N stay 0
+  T *sA = X + 2 * NP * EW, *sB = sA + P * W, *sC = sB + P * W, *sD = sC + P * W, *sLast = sD + P * W;
+  const int r0 = row_begin(ny, ctas, rank), R = row_begin(ny, ctas, rank + 1) - r0;
+  const int prev = rank ? rank - 1 : ctas - 1, next = rank + 1 < ctas ? rank + 1 : 0;
+  T *Xprev = cl.map_shared_rank(X, prev), *Xnext = cl.map_shared_rank(X, next);
+  const int prev_rows = row_begin(ny, ctas, prev + 1) - row_begin(ny, ctas, prev);
+  const unsigned plane = (unsigned)(nx * ny);
+  const int p = (int)threadIdx.x / W, lc = (int)threadIdx.x - p * W, lr = lc / nx, i = lc - lr * nx;
+  const bool act = p < P && lr < R;
+  const int k0 = p * S;
+  const int j = r0 + lr, col = j * nx + i;
+  auto in = [&](int q) { return act && k0 + q < N; };
+  // the segment's operands; a cell past the last plane changes nothing:
+  // mv = 0, fv = 0 and cv = -1 keep its d and y at 0 and the products as they are
+  T bv[S], av[S], mv[S], cv[S], fv[S], qv[S], xv[S];
+  {
+    T nv[S + 2];
+    nv[0] = in(0) && k0 > 0 ? dens[(unsigned)(k0 - 1) * plane + col] : T(0);
+#pragma unroll
+    for (int q = 0; q <= S; q++) nv[q + 1] = in(q) ? dens[(unsigned)(k0 + q) * plane + col] : T(0);
+    T fprod = T(1);
+#pragma unroll
+    for (int q = 0; q < S; q++) {
+      bv[q] = av[q] = mv[q] = fv[q] = qv[q] = xv[q] = T(0);
+      cv[q] = T(-1);
+      if (in(q)) {
+        const int k = k0 + q;
+        const Nbr nb = nbr_of(o.g, i, j, k);
+        T v[11];
+        row11_n(dens, o, nb, v);
+        C[k * W + lc] = make_float4(v[0], v[1], v[2], v[3]);
+        C[(N + k) * W + lc] = make_float4(v[6], v[7], v[8], v[9]);
+        const unsigned c = (unsigned)k * plane + col;
+        bv[q] = b[c];
+        mv[q] = z.minv[c];
+        qv[q] = z.q[c];
+        av[q] = k == 0 ? T(0) : zc(nv[q + 1], nv[q]);
+        cv[q] = (k == N - 1 ? T(0) : zc(nv[q + 1], nv[q + 2])) * mv[q];
+        fprod *= -(av[q] * mv[q]);
+        fv[q] = fprod;
+      }
+    }
+    if (p < P) sB[p * W + lc] = fprod;
+    T bprod = T(1);
+#pragma unroll
+    for (int q = S - 1; q >= 0; q--) bprod *= -cv[q];
+    if (p < P) sD[p * W + lc] = bprod;
+  }
+  const T a0g = act ? z.a0g[col] : T(0), qden = act ? z.qden[col] : T(0);
+  // element offsets of this segment's first cell and its in-plane neighbours
+  const int at = k0 * EW + nx + lc, xm = i > 0 ? -1 : nx - 1, xp = i < nx - 1 ? 1 : 1 - nx;
+  cl.sync();  // every CTA runs before it is written to
+#pragma unroll 1
+  for (int sw = 0; sw < sweeps; sw++) {
+    const int buf = (sw & 1) * NP * EW, nbuf = NP * EW - buf;
+    T rv[S];
+#pragma unroll
+    for (int q = 0; q < S; q++) rv[q] = bv[q];
+    if (sw > 0 && act) {  // b - A_xy x, the entries in the order of k_zline_rhs
+      const T *x0 = X + buf + at;
+      const T *e0 = x0 + xp, *e1 = x0 + xm, *e2 = x0 + nx, *e3 = x0 - nx;
+      const T *e6 = e0 + nx, *e7 = e0 - nx, *e8 = e1 + nx, *e9 = e1 - nx;
+      const float4 *cu = C + k0 * W + lc, *cw = cu + N * W;
+#pragma unroll
+      for (int q = 0; q < S; q++) {
+        const float4 u = *cu, w = *cw;
+        const int step = k0 + q + 1 < N ? W : 0;  // past the last plane: its entries times 0
+        cu += step;
+        cw += step;
+        T s = rv[q];
+        s -= u.x * e0[q * EW];
+        s -= u.y * e1[q * EW];
+        s -= u.z * e2[q * EW];
+        s -= u.w * e3[q * EW];
+        s -= w.x * e6[q * EW];
+        s -= w.y * e7[q * EW];
+        s -= w.z * e8[q * EW];
+        s -= w.w * e9[q * EW];
+        rv[q] = s;
+      }
+    }
+    {
+      T d = T(0);
+#pragma unroll
+      for (int q = 0; q < S; q++) {
+        d = (rv[q] - av[q] * d) * mv[q];
+        rv[q] = d;
+      }
+      if (p < P) sA[p * W + lc] = d;
+    }
+    __syncthreads();
+    {
+      T din = T(0);
+      for (int pp = 0; pp < p; pp++) din = sA[pp * W + lc] + sB[pp * W + lc] * din;
+      T y = T(0), yl = T(0);
+#pragma unroll
+      for (int q = S - 1; q >= 0; q--) {
+        y = (rv[q] + fv[q] * din) - cv[q] * y;
+        rv[q] = y;
+        if (k0 + q == N - 1) yl = y;
+      }
+      if (p < P) sC[p * W + lc] = y;
+      if (p == P - 1) sLast[lc] = yl;
+    }
+    __syncthreads();
+    if (act) {
+      T yin = T(0), run = T(0);
+      for (int pp = P - 1; pp >= 0; pp--) {
+        if (pp == p) yin = run;
+        run = sC[pp * W + lc] + sD[pp * W + lc] * run;
+      }
+      const T s = (run + a0g * sLast[lc]) * qden;  // run = y_0
+      T bprod = T(1);
+#pragma unroll
+      for (int q = S - 1; q >= 0; q--) {
+        bprod *= -cv[q];
+        const T yk = rv[q] + bprod * yin;
+        xv[q] = xv[q] + omega * ((yk - s * qv[q]) - xv[q]);
+      }
+      if (sw == sweeps - 1) {
+#pragma unroll
+        for (int q = 0; q < S; q++)
+          if (in(q)) xout[(unsigned)(k0 + q) * plane + col] = xv[q];
+      } else {
+        T *xn = X + nbuf + at;
+#pragma unroll
+        for (int q = 0; q < S; q++) xn[q * EW] = xv[q];
+        if (lr == 0) {
+          T *h = Xprev + nbuf + k0 * EW + (prev_rows + 1) * nx + i;
+#pragma unroll
+          for (int q = 0; q < S; q++) h[q * EW] = xv[q];
+        }
+        if (lr == R - 1) {
+          T *h = Xnext + nbuf + k0 * EW + i;
+#pragma unroll
+          for (int q = 0; q < S; q++) h[q * EW] = xv[q];
+        }
+      }
+    }
+    cl.sync();  // the halos are in place (and nothing is written after a CTA's end)
+  }
+}
+
+// Cluster of the sweeps of an nx x ny x nz level: one CTA up to 2048 cells,
+// then a CTA for each 2048 (a sweep of that many cells takes about as long as
+// the cluster barrier), at most sixteen and one a row; 0 CTAs when the level
+// does not fit (or its columns are cut into longer segments).
+static CoarseShape coarse_shape(int nx, int ny, int nz) {
+  CoarseShape s;
+  if (nz > kClusterSeg * kMaxSeg) return s;
+  const int P = (nz + kClusterSeg - 1) / kClusterSeg, NP = P * kClusterSeg;
+  for (int c = 1; c <= kClusterMax && c <= ny; c *= 2) {
+    const int rows = (ny + c - 1) / c, ew = (rows + 2) * nx;
+    const long long threads = (long long)rows * nx * P;
+    const int EW = ew <= 128 ? 128 : (ew <= 256 ? 256 : 512);
+    const size_t words = (size_t)8 * nz * rows * nx + (size_t)2 * NP * EW + (size_t)(4 * P + 1) * rows * nx;
+    const bool fits = threads <= 640 && ew <= EW && words * sizeof(float) <= kClusterSmem;
+    if (fits) {
+      s.ctas = c;
+      s.rows = rows;
+      s.threads = (int)((threads + 31) / 32 * 32);
+      s.ew = EW;
+      s.smem = words * sizeof(float);
+      if ((size_t)nx * ny * nz <= (size_t)2048 * c) break;
+    }
+  }
+  return s;
+}
+// The instantiation for a shape's plane stride.
+template <typename T>
+using CoarseKernel = void (*)(OpK, ZCoup<T>, const T *, ZlP<T>, const T *, T *, int, int, T);
+template <typename T>
+static CoarseKernel<T> coarse_kernel(const CoarseShape &s) {
+  return s.ew == 128 ? k_coarse_sweeps<T, 128, 640> : (s.ew == 256 ? k_coarse_sweeps<T, 256, 640> : k_coarse_sweeps<T, 512, 640>);
+}
+
 // ---- direct solve of the coarsest level -----------------------------------------
 constexpr int kDirectMax = 128;           // largest coarsest level solved directly
 constexpr size_t kInverseSmem = 160 * 1024;  // shared memory of its Gauss-Jordan work matrix
@@ -1542,6 +1758,9 @@ template <>
 Multigrid<float> &mg_of<float>(EcsCtx *ctx) { return ctx->mg32; }
 
 template <typename T>
+int coarse_attrs(EcsCtx *ctx, CoarseShape &cs);
+
+template <typename T>
 int mg_alloc(EcsCtx *ctx) {
   Multigrid<T> &mg = mg_of<T>(ctx);
   if (mg.built) return ECS_OK;
@@ -1585,6 +1804,14 @@ int mg_alloc(EcsCtx *ctx) {
   if (nc <= (size_t)kDirectMax) {
     ECS_CUDA(ctx, cudaMalloc((void **)&mg.cinv, nc * nc * sizeof(T)));
     ECS_CUDA(ctx, cudaMalloc((void **)&mg.cwork, nc * 2 * nc * sizeof(T)));
+  } else if constexpr (sizeof(T) == 4) {
+    const MgLevel<T> &C = mg.lv.back();
+    CoarseShape cs = coarse_shape(C.nx, C.ny, C.nz);
+    if (cs.ctas > 0) {
+      const int rc = coarse_attrs<T>(ctx, cs);
+      if (rc) return rc;
+    }
+    mg.cluster = cs;
   }
   mg.built = true;
   return ECS_OK;
@@ -1771,6 +1998,53 @@ size_t small_layout(const Multigrid<T> &mg, size_t l, SmallCycle<T> *sc) {
   return (size_t)off * sizeof(T) + (size_t)ni * sizeof(unsigned);
 }
 
+// Sizes the cluster of the coarsest level's sweeps (no CTAs: two launches a
+// sweep), checking that the device can place it.
+template <typename T>
+int coarse_attrs(EcsCtx *ctx, CoarseShape &cs) {
+  auto kernel = coarse_kernel<T>(cs);
+  ECS_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem));
+  ECS_CUDA(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cs.ctas);
+  cfg.blockDim = dim3((unsigned)cs.threads);
+  cfg.dynamicSmemBytes = cs.smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cs.ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    cs.ctas = 0;
+  }
+  return ECS_OK;
+}
+template <typename T>
+int launch_coarse_sweeps(EcsCtx *ctx, MgLevel<T> &L, const CoarseShape &cs, const T *b, T *xout) {
+  const OpK o = op_level(ctx, L);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cs.ctas);
+  cfg.blockDim = dim3((unsigned)cs.threads);
+  cfg.dynamicSmemBytes = cs.smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cs.ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  const ZCoup<T> zc = z_coupling<T>(o);
+  const ZlP<T> z = zl_of(L);
+  cudaLaunchKernelEx(&cfg, coarse_kernel<T>(cs), o, zc, (const T *)L.dens, z, b, xout, cs.rows, kCoarseSweeps, kOmega<T>());
+  ECS_LAUNCHED(ctx);
+  return ECS_OK;
+}
+
 // One V(1,1) cycle on level l: xout = M(l) b, zero initial guess.  Levels of
 // at most kSmallCells cells run as one single-block kernel.
 template <typename T>
@@ -1800,6 +2074,9 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
     return ECS_OK;
   }
   if (l + 1 == mg.lv.size()) {
+    if constexpr (sizeof(T) == 4) {
+      if (mg.cluster.ctas > 0) return launch_coarse_sweeps<T>(ctx, L, mg.cluster, b, xout);
+    }
     if ((rc = sweep<T>(ctx, L, b, nullptr, xout))) return rc;
     for (int s = 0; s < (kCoarseSweeps - 1) / 2; s++) {
       if ((rc = sweep<T>(ctx, L, b, xout, L.t))) return rc;
