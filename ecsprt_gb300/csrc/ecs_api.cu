@@ -117,7 +117,7 @@ int64_t ecs_ctx_device_bytes(const EcsParams *p, int precision, int64_t cap) {
   const int64_t t = precision == ECS_PREC_FP64 ? 8 : 4;  // solver arithmetic
   int64_t b = 0;
   b += n * 8 * (1 + 4 + 1) + n * 8 * 4;  // phi, moments, rhs; fixed-point accumulators
-  b += n * 8 * 2 + (m + 2) * 1024 * 8;   // FP64 residual and correction, reductions
+  b += n * 8 + (m + 2) * 4096 * 8;       // FP64 residual, reductions
   if (p->lhs_type != ECS_LHS_IDENTITY) b += n * 8 * 11;  // FP64 row coefficients of the residuals
   // multigrid: 7 cell arrays (11 in FP64 and for columns of more than 128
   // cells) and 2 plane arrays a level, levels summing to at most 8/7 of the
@@ -127,7 +127,7 @@ int64_t ecs_ctx_device_bytes(const EcsParams *p, int precision, int64_t cap) {
     b += (2 * m + 1) * n * 8;  // Krylov bases V, Z
     b += cap * 48 + ne * 32;   // ions (6 FP64), E numerators
   } else {
-    b += (2 * m + 3) * n * 4;  // Krylov bases V, Z, two FP32 work vectors
+    b += (2 * m + 2) * n * 4;  // Krylov bases V, Z, the normalised residual
     b += cap * 72 + ne * 16;   // ions (two 32-byte record buffers, sort keys, permutation), E numerators
     const int64_t keys = (int64_t)((p->Nx + ECS_TILE_X - 1) / ECS_TILE_X) * ((p->Ny + ECS_TILE_Y - 1) / ECS_TILE_Y) *
                          ((p->Nz + ECS_TILE_Z - 1) / ECS_TILE_Z) * ECS_TILE_CELLS;

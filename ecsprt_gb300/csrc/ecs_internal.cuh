@@ -168,8 +168,7 @@ struct EcsCtx {
   double *kz64 = nullptr;           // FP64 preconditioned basis Z [m*ncell]
   float *kv32 = nullptr;            // FP32 Krylov basis for the inner solve
   float *kz32 = nullptr;
-  double *w64 = nullptr;            // FP64 work vectors
-  double *r64 = nullptr;
+  double *r64 = nullptr;            // FP64 residual
   double *coef64 = nullptr;         // the FP64 operator's 11 row coefficients a cell (SoA), for the refinement residuals
   double *dots = nullptr;           // device scalars (norms, means) [m+2]
   double *h_dots = nullptr;         // pinned host copy

@@ -53,7 +53,7 @@ struct KrylovDev {
   int jprev;       // index of the step that just finished
   int done;        // 1: converged, broke down or out of steps
   int nits;        // Arnoldi steps taken
-  double beta, res, inv_scale, mean;
+  double beta, res, inv_scale, mean, hn;
   double h1[kSlots], h2[kSlots];
   double H[(kKrylovMax + 1) * kKrylovMax];
   double cs[kKrylovMax], sn[kKrylovMax], g[kKrylovMax + 1], y[kKrylovMax];
@@ -1402,21 +1402,6 @@ __device__ __forceinline__ void slot_totals(const double *partial, int ns, int n
   }
 }
 
-// x64 += a * e (e in T)
-template <typename T>
-__global__ void k_axpy64(size_t n, double a, const T *__restrict__ e, double *__restrict__ x) {
-  ECS_PDL_ENTRY();
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    x[q] += a * (double)e[q];
-}
-// d = s * scale[0] in the precision of d (the FP64 residual, normalised, to T)
-template <typename T>
-__global__ void k_scale_to(size_t n, const double *__restrict__ s, const double *__restrict__ scale, T *__restrict__ d) {
-  ECS_PDL_ENTRY();
-  const T a = (T)scale[0];
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    d[q] = (T)s[q] * a;
-}
 // v -= value[0]
 template <typename T>
 __global__ void k_sub_value(size_t n, T *__restrict__ v, const double *__restrict__ value) {
@@ -1478,64 +1463,98 @@ __global__ void __launch_bounds__(kB, 4) k_dots1(size_t n, const T *__restrict__
   slot_totals(partial, nv, (int)gridDim.x, kd->h1);
 }
 
-// Arnoldi bookkeeping of step j, in the last block of the pass-2 launch:
-// reduce the pass-2 partials into h2 and w.w, form column j of the
-// Hessenberg matrix, apply the previous Givens rotations and a new one,
-// update the residual estimate and decide whether the cycle stops.
-__device__ __forceinline__ void arnoldi_update(KrylovDev *kd, int nb, const double *partial,
-                                               cudaGraphConditionalHandle cond, int use_graph) {
+// Arnoldi bookkeeping of step j.  Its first part, in the last block of the
+// pass-2 launch, is what the next kernel waits for: the pass-2 partials
+// reduced into h2 and w.w, and the norm of the new basis vector.
+__device__ __noinline__ void arnoldi_norm(KrylovDev *kd, int nb, const double *partial) {
   __shared__ double red[kSlots];
-  if (kd->done) {  // stopped before this step (b = 0): keep the state
-    if (threadIdx.x == 0 && use_graph) cudaGraphSetConditional(cond, 0u);
-    return;
-  }
+  if (kd->done) return;  // stopped before this step (b = 0): keep the state
   const int j = kd->j, nv = j + 1;
   slot_totals(partial, nv + 1, nb, red);
   __syncthreads();
+  if (threadIdx.x <= j) kd->h2[threadIdx.x] = red[threadIdx.x];
   if (threadIdx.x != 0) return;
-  const int m = kKrylovMax;
   double ss = 0.0;
-  for (int q = 0; q <= j; q++) {
-    kd->h2[q] = red[q];
-    ss += red[q] * red[q];
-  }
-  const double ww = red[nv];
-  const double hn = sqrt(fmax(ww - ss, 0.0));
-  double *H = kd->H;
-  for (int q = 0; q <= j; q++) H[q * m + j] = kd->h1[q] + kd->h2[q];
-  H[(j + 1) * m + j] = hn;
-  for (int q = 0; q < j; q++) {
-    const double a = H[q * m + j], c = H[(q + 1) * m + j];
-    H[q * m + j] = kd->cs[q] * a + kd->sn[q] * c;
-    H[(q + 1) * m + j] = -kd->sn[q] * a + kd->cs[q] * c;
-  }
-  const double a = H[j * m + j], c = H[(j + 1) * m + j];
-  const double r = sqrt(a * a + c * c);
-  kd->cs[j] = r > 0 ? a / r : 1.0;
-  kd->sn[j] = r > 0 ? c / r : 0.0;
-  H[j * m + j] = r;
-  H[(j + 1) * m + j] = 0.0;
-  kd->g[j + 1] = -kd->sn[j] * kd->g[j];
-  kd->g[j] = kd->cs[j] * kd->g[j];
-  const double res = fabs(kd->g[j + 1]);
-  kd->res = res;
-  kd->nits = j + 1;
+  for (int q = 0; q <= j; q++) ss += red[q] * red[q];
+  const double hn = sqrt(fmax(red[nv] - ss, 0.0));
+  kd->hn = hn;
   kd->inv_scale = hn > 0 ? 1.0 / hn : 0.0;
   kd->jprev = j;
-  const int done = (res <= kd->tol_rel * kd->beta) || hn == 0.0 || (j + 1 >= kd->maxit) ||
-                   (j + 1 >= kKrylovMax) || !isfinite(res);
-  kd->done = done;
-  if (!done) kd->j = j + 1;
-  if (use_graph) cudaGraphSetConditional(cond, done ? 0u : 1u);
+}
+
+// The rest, in a block of its own beside the blocks that scale the new basis
+// vector (it takes about as long as they do): column j of the Hessenberg
+// matrix, the previous Givens rotations and a new one, the residual estimate
+// and the decision whether the cycle stops; when it does, the solve of H y = g
+// (upper triangular).  One thread works through the column, a chain of FP64
+// operations, on shared memory that the block filled.
+__device__ __noinline__ void arnoldi_rotate(KrylovDev *kd, cudaGraphConditionalHandle cond, int use_graph) {
+  constexpr int m = kKrylovMax;
+  __shared__ double col[kSlots], scs[m], ssn[m], g[m + 1], y[m];
+  __shared__ double Hs[m * m];  // Hs[r * m + c]: the upper triangle's earlier columns
+  __shared__ int stop;
+  const int done0 = kd->done, j = kd->j, tid = threadIdx.x;
+  if (done0) {  // stopped before this step (b = 0): keep the state
+    if (tid == 0 && use_graph) cudaGraphSetConditional(cond, 0u);
+    return;
+  }
+  for (int e = tid; e < j; e += blockDim.x) {
+    scs[e] = kd->cs[e];
+    ssn[e] = kd->sn[e];
+  }
+  for (int e = tid; e <= j; e += blockDim.x) {
+    g[e] = kd->g[e];
+    col[e] = kd->h1[e] + kd->h2[e];
+  }
+  for (int e = tid; e < j * j; e += blockDim.x) Hs[(e / j) * m + e % j] = kd->H[(e / j) * m + e % j];
+  __syncthreads();
+  if (tid == 0) {
+    const double hn = kd->hn;
+    col[j + 1] = hn;
+    for (int q = 0; q < j; q++) {
+      const double a = col[q], c = col[q + 1];
+      col[q] = fma(scs[q], a, ssn[q] * c);
+      col[q + 1] = fma(scs[q], c, -ssn[q] * a);
+    }
+    const double a = col[j], c = hn;
+    const double r = sqrt(fma(a, a, c * c));
+    const double cs = r > 0 ? a / r : 1.0, sn = r > 0 ? c / r : 0.0;
+    kd->cs[j] = cs;
+    kd->sn[j] = sn;
+    col[j] = r;
+    const double g1 = -sn * g[j], g0 = cs * g[j];
+    kd->g[j + 1] = g1;
+    kd->g[j] = g0;
+    g[j] = g0;
+    const double res = fabs(g1);
+    kd->res = res;
+    kd->nits = j + 1;
+    const int done = (res <= kd->tol_rel * kd->beta) || hn == 0.0 || (j + 1 >= kd->maxit) ||
+                     (j + 1 >= kKrylovMax) || !isfinite(res);
+    kd->done = done;
+    if (!done) kd->j = j + 1;
+    if (use_graph) cudaGraphSetConditional(cond, done ? 0u : 1u);
+    stop = done;
+    if (done)
+      for (int q = j; q >= 0; q--) {
+        double t = g[q];
+        for (int r2 = q + 1; r2 <= j; r2++) t -= (r2 == j ? col[q] : Hs[q * m + r2]) * y[r2];
+        y[q] = t / (q == j ? col[j] : Hs[q * m + q]);
+      }
+  }
+  __syncthreads();
+  if (tid <= j) {
+    kd->H[tid * m + j] = col[tid];
+    if (stop) kd->y[tid] = y[tid];
+  }
 }
 
 // w = V_{j+1} - sum_q h1[q] V_q (stored, in the first slot chunk), then
 // pass 2: partial dots of V_0..V_j with the new w (slots 0..j) and of w with
-// itself (slot j+1); the last block runs the Arnoldi bookkeeping.
+// itself (slot j+1); the last block forms the new vector's norm.
 template <typename T, int W>
 __global__ void __launch_bounds__(kB, 4) k_orth1_dots2(size_t n, T *__restrict__ V, KrylovDev *__restrict__ kd,
-                                                       double *__restrict__ partial, cudaGraphConditionalHandle cond,
-                                                       int use_graph) {
+                                                       double *__restrict__ partial) {
   ECS_PDL_ENTRY();
   __shared__ T h[kSlots];
   const int nv = kd->j + 1, nslot = nv + 1;
@@ -1572,14 +1591,21 @@ __global__ void __launch_bounds__(kB, 4) k_orth1_dots2(size_t n, T *__restrict__
     block_chunk(acc, v0, nslot, partial);
   }
   if (!last_block(&kd->ticket[1])) return;
-  arnoldi_update(kd, (int)gridDim.x, partial, cond, use_graph);
+  arnoldi_norm(kd, (int)gridDim.x, partial);
 }
 
 // V_{j+1} = (w - sum_q h2[q] V_q) / h_{j+1,j}, also copied to the
-// preconditioner input vin (j = the step that just finished).
+// preconditioner input vin (j = the step that just finished: the fields read
+// here are those of arnoldi_norm).  Block 0 does the rest of the bookkeeping
+// meanwhile.
 template <typename T, int W>
-__global__ void k_orth2_scale(size_t n, T *__restrict__ V, const KrylovDev *__restrict__ kd, T *__restrict__ vin) {
+__global__ void k_orth2_scale(size_t n, T *__restrict__ V, KrylovDev *kd, T *__restrict__ vin,
+                              cudaGraphConditionalHandle cond, int use_graph) {
   ECS_PDL_ENTRY();
+  if (blockIdx.x == 0) {
+    arnoldi_rotate(kd, cond, use_graph);
+    return;
+  }
   __shared__ T h[kSlots + 1];
   const int j = kd->jprev, nv = j + 1;
   if (threadIdx.x < kSlots) h[threadIdx.x] = (int)threadIdx.x < nv ? (T)kd->h2[threadIdx.x] : T(0);
@@ -1587,8 +1613,8 @@ __global__ void k_orth2_scale(size_t n, T *__restrict__ V, const KrylovDev *__re
   __syncthreads();
   T *w = V + (size_t)(j + 1) * n;
   const T sc = h[kSlots];
-  const size_t nw = n / W;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += (size_t)gridDim.x * blockDim.x) {
+  const size_t nw = n / W, stride = (size_t)(gridDim.x - 1) * blockDim.x;
+  for (size_t e = (size_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; e < nw; e += stride) {
     Pack<T, W> s = ld_pack<T, W>(w + e * W);
     for (int q = 0; q < nv; q++) {
       const Pack<T, W> vq = ld_pack<T, W>(V + (size_t)q * n + e * W);
@@ -1626,17 +1652,84 @@ __global__ void k_apply_dyn(OpK o, const T *__restrict__ n, const T *__restrict_
   V[(size_t)(jj + 1) * o.g.n + c] = s;
 }
 
+// Device state of the iterative-refinement loop.
+struct RefineDev {
+  double bnorm, rel;
+  int its, sweeps;
+  int done;  // converged, out of iterations, stalled or non-finite
+  int nonfinite;
+};
+
+// Refinement sweeps in one solve: each sweep runs at least one FGMRES step
+// (or ends the solve), so max_it bounds them; this caps the loop regardless.
+constexpr int kMaxSweeps = 64;
+
+// What the norm that ends a refinement sweep (or starts the solve) decides.
+struct RefineArgs {
+  RefineDev *rd;
+  double rtol, tol_floor;
+  int max_it;
+  int decide;  // 0: set the state up only
+  int after;   // 1: the residual is that of a finished sweep
+};
+// Relative residual of the current sweep from its norm; decides whether
+// another correction follows (condition `cond` of the sweep loop) and sets
+// the FGMRES tolerance and step limit of that correction.
+__device__ __forceinline__ void refine_decide(const RefineArgs &ra, KrylovDev *kd, double norm,
+                                              cudaGraphConditionalHandle cond) {
+  RefineDev *rd = ra.rd;
+  if (ra.after) {
+    rd->its += kd->nits;
+    rd->sweeps += 1;
+    if (kd->nits == 0) rd->done = 1;
+  }
+  if (rd->bnorm > 0.0) {
+    const double rel = norm / rd->bnorm;
+    rd->rel = rel;
+    if (!isfinite(rel)) rd->nonfinite = 1;
+  }
+  const bool stop = rd->done || rd->nonfinite || rd->rel <= ra.rtol || rd->its >= ra.max_it || rd->sweeps >= kMaxSweeps;
+  if (stop) {
+    rd->done = 1;
+  } else {
+    const double tol = fmax(fmax(0.5 * ra.rtol / rd->rel, 1e-14), ra.tol_floor);
+    kd->tol_rel = tol;
+    kd->maxit = min(kKrylovMax, max(ra.max_it - rd->its, 1));
+  }
+  cudaGraphSetConditional(cond, stop ? 0u : 1u);
+}
+
+// Start of an FGMRES cycle on a vector of norm sqrt(u2).  In a graph it also
+// (re)arms the Arnoldi loop's condition, which keeps its last value between
+// cycles of one launch.
+__device__ __forceinline__ void cycle_begin(KrylovDev *kd, double u2, cudaGraphConditionalHandle cond, int use_graph) {
+  const double beta = sqrt(u2);
+  kd->beta = beta;
+  kd->res = beta;
+  kd->j = 0;
+  kd->jprev = 0;
+  kd->nits = 0;
+  kd->done = !(beta > 0.0) || kd->maxit < 1;
+  kd->inv_scale = beta > 0.0 ? 1.0 / beta : 0.0;
+  for (int q = 0; q <= kKrylovMax; q++) kd->g[q] = 0.0;
+  kd->g[0] = beta;
+  if (use_graph) cudaGraphSetConditional(cond, kd->done ? 0u : 1u);
+}
+
 // Grid-wide sums of a vector in packs of W, finished by the last block:
-//   kRedMean  out[0] = sum(v) / div
-//   kRedNorm  out[0] = ||v||, out[1] = 1 / ||v|| (0 for v = 0)
-//   kRedBeta  start of an FGMRES cycle: beta = ||v|| into the control block;
-//             in a graph it also (re)arms the Arnoldi loop's condition,
-//             which keeps its last value between cycles of one launch.
-enum { kRedMean = 0, kRedNorm = 1, kRedBeta = 2 };
+//   kRedMean   out[0] = sum(v) / div
+//   kRedNorm   out[0] = ||v||, out[1] = 1 / ||v|| (0 for v = 0)
+//   kRedBeta   start of an FGMRES cycle: beta = ||v|| into the control block
+//   kRedInit   kRedNorm of the right-hand side, which sets the refinement
+//              state up (and decides on the first correction: ra.decide)
+//   kRedCheck  kRedNorm of a residual, and the refinement loop's decision
+// The decisions ride on the reductions because a one-thread kernel of their
+// own costs a launch (2 to 3 us) each.
+enum { kRedMean = 0, kRedNorm = 1, kRedBeta = 2, kRedInit = 3, kRedCheck = 4 };
 template <typename T, int W, int M>
 __global__ void __launch_bounds__(kB) k_reduce(size_t nw, const T *__restrict__ v, double *__restrict__ partial,
                                                double div, double *out, KrylovDev *kd,
-                                               cudaGraphConditionalHandle cond, int use_graph) {
+                                               cudaGraphConditionalHandle cond, int use_graph, RefineArgs ra) {
   ECS_PDL_ENTRY();
   KSum<T> acc;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += (size_t)gridDim.x * blockDim.x) {
@@ -1650,62 +1743,119 @@ __global__ void __launch_bounds__(kB) k_reduce(size_t nw, const T *__restrict__ 
   if (threadIdx.x != 0) return;
   if (M == kRedMean) {
     out[0] = u / div;
-  } else if (M == kRedNorm) {
-    out[0] = sqrt(u);
-    out[1] = u > 0.0 ? 1.0 / sqrt(u) : 0.0;
+  } else if (M == kRedBeta) {
+    cycle_begin(kd, u, cond, use_graph);
   } else {
-    const double beta = sqrt(u);
-    kd->beta = beta;
-    kd->res = beta;
-    kd->j = 0;
-    kd->jprev = 0;
-    kd->nits = 0;
-    kd->done = !(beta > 0.0) || kd->maxit < 1;
-    kd->inv_scale = beta > 0.0 ? 1.0 / beta : 0.0;
-    for (int q = 0; q <= kKrylovMax; q++) kd->g[q] = 0.0;
-    kd->g[0] = beta;
-    if (use_graph) cudaGraphSetConditional(cond, kd->done ? 0u : 1u);
+    const double norm = sqrt(u);
+    out[0] = norm;
+    out[1] = u > 0.0 ? 1.0 / sqrt(u) : 0.0;
+    if (M == kRedInit) {
+      RefineDev *rd = ra.rd;
+      rd->bnorm = norm;
+      rd->rel = 0.0;
+      rd->its = 0;
+      rd->sweeps = 0;
+      rd->done = !(norm > 0.0);
+      rd->nonfinite = 0;
+    }
+    if ((M == kRedInit && ra.decide) || M == kRedCheck) refine_decide(ra, kd, norm, cond);
   }
 }
 
-// V_0 = b / beta, vin = V_0, x = 0
+// The normalised FP64 residual to FP32, d = s scale[0], and the cycle's
+// beta = ||d||, with the sums of k_reduce.  The first sweep from phi = 0
+// (rd, its s0) takes the right-hand side for the residual.
+template <int W>
+__global__ void __launch_bounds__(kB) k_scale_beta(size_t nw, const double *__restrict__ s0,
+                                                   const double *__restrict__ s1, const RefineDev *rd,
+                                                   const double *__restrict__ scale, float *__restrict__ d,
+                                                   double *__restrict__ partial, KrylovDev *kd,
+                                                   cudaGraphConditionalHandle cond, int use_graph) {
+  ECS_PDL_ENTRY();
+  const double *s = rd && rd->sweeps == 0 ? s0 : s1;
+  const float a = (float)scale[0];
+  KSum<float> acc;
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += (size_t)gridDim.x * blockDim.x) {
+    Pack<float, W> p;
+    if constexpr (W == 4) {
+      const Pack<double, 2> lo = ld_pack<double, 2>(s + e * 4), hi = ld_pack<double, 2>(s + e * 4 + 2);
+      p.v[0] = (float)lo.v[0] * a;
+      p.v[1] = (float)lo.v[1] * a;
+      p.v[2] = (float)hi.v[0] * a;
+      p.v[3] = (float)hi.v[1] * a;
+    } else {
+      p.v[0] = (float)s[e] * a;
+    }
+    st_pack<float, W>(d + e * W, p);
+#pragma unroll
+    for (int i = 0; i < W; i++) acc.add(p.v[i] * p.v[i]);
+  }
+  block_partial(acc, partial);
+  if (!last_block(&kd->ticket[7])) return;
+  const double u = partials_total(partial, (int)gridDim.x);
+  if (threadIdx.x == 0) cycle_begin(kd, u, cond, use_graph);
+}
+
+// V_0 = b / beta, vin = V_0
 template <typename T>
 __global__ void k_cycle_start(size_t n, const T *__restrict__ b, T *__restrict__ V, T *__restrict__ vin,
-                              T *__restrict__ x, const KrylovDev *__restrict__ kd) {
+                              const KrylovDev *__restrict__ kd) {
   ECS_PDL_ENTRY();
   const T sc = (T)kd->inv_scale;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const T v = b[e] * sc;
     V[e] = v;
     vin[e] = v;
-    x[e] = T(0);
   }
 }
 
-// y = H^-1 g (upper triangular, nits x nits)
-__global__ void k_cycle_solve(KrylovDev *kd) {
-  ECS_PDL_ENTRY();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const int m = kKrylovMax, nj = kd->nits;
-  for (int q = nj - 1; q >= 0; q--) {
-    double s = kd->g[q];
-    for (int r2 = q + 1; r2 < nj; r2++) s -= kd->H[q * m + r2] * kd->y[r2];
-    kd->y[q] = s / kd->H[q * m + q];
-  }
-}
-
-// x += sum_q y[q] Z_q
-template <typename T>
-__global__ void k_cycle_combine(size_t n, const T *__restrict__ Z, const KrylovDev *__restrict__ kd, T *__restrict__ x) {
+// End of a cycle, one pass over Z and phi: phi += scale[0] sum_q y[q] Z_q
+// (scale nullptr: 1), and with MEAN also mean[0] = the mean of the new phi,
+// with the sums of k_reduce (packs of W cells).
+template <typename T, int W, bool MEAN>
+__global__ void __launch_bounds__(kB) k_cycle_finish(size_t nw, size_t n, const T *__restrict__ Z, KrylovDev *kd,
+                                                     const double *__restrict__ scale, double *__restrict__ phi,
+                                                     double *__restrict__ partial, double *mean) {
   ECS_PDL_ENTRY();
   __shared__ T y[kKrylovMax];
   const int nj = kd->nits;
+  const double a = scale ? scale[0] : 1.0;
   if (threadIdx.x < kKrylovMax) y[threadIdx.x] = (int)threadIdx.x < nj ? (T)kd->y[threadIdx.x] : T(0);
   __syncthreads();
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    T s = x[e];
-    for (int q = 0; q < nj; q++) s += y[q] * Z[(size_t)q * n + e];
-    x[e] = s;
+  KSum<double> acc;
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += (size_t)gridDim.x * blockDim.x) {
+    Pack<double, W> p = ld_pack<double, W>(phi + e * W);
+    T s[W];
+#pragma unroll
+    for (int i = 0; i < W; i++) s[i] = T(0);
+#pragma unroll 4
+    for (int q = 0; q < nj; q++) {
+      const T yq = y[q], *zq = Z + (size_t)q * n + e * W;
+      T zv[W];
+      if constexpr (W == 2 && sizeof(T) == 4) {
+        const float2 f = *reinterpret_cast<const float2 *>(zq);
+        zv[0] = f.x;
+        zv[1] = f.y;
+      } else {
+        const Pack<T, W> f = ld_pack<T, W>(zq);
+#pragma unroll
+        for (int i = 0; i < W; i++) zv[i] = f.v[i];
+      }
+#pragma unroll
+      for (int i = 0; i < W; i++) s[i] += yq * zv[i];
+    }
+#pragma unroll
+    for (int i = 0; i < W; i++) {
+      p.v[i] += a * (double)s[i];
+      if (MEAN) acc.add(p.v[i]);
+    }
+    st_pack<double, W>(phi + e * W, p);
+  }
+  if constexpr (MEAN) {
+    block_partial(acc, partial);
+    if (!last_block(&kd->ticket[2 + kRedMean])) return;
+    const double u = partials_total(partial, (int)gridDim.x);
+    if (threadIdx.x == 0) mean[0] = u / (double)n;
   }
 }
 
@@ -1730,13 +1880,13 @@ inline bool packed4(size_t n) { return (n & 3) == 0; }
 // A grid-wide sum of v (kRed* mode M) on the context's stream.
 template <typename T, int M>
 int launch_reduce(EcsCtx *ctx, size_t n, const T *v, double div, double *out, cudaGraphConditionalHandle cond,
-                  int use_graph) {
+                  int use_graph, const RefineArgs &ra = RefineArgs()) {
   KrylovDev *kd = (KrylovDev *)ctx->kdev;
   constexpr int W = kPack<T>;
   if (packed4(n))
-    ecs_launch_pdl(k_reduce<T, W, M>, dot_blocks(ctx, n / W), kB, 0, ctx->stream, n / W, v, ctx->red, div, out, kd, cond, use_graph);
+    ecs_launch_pdl(k_reduce<T, W, M>, dot_blocks(ctx, n / W), kB, 0, ctx->stream, n / W, v, ctx->red, div, out, kd, cond, use_graph, ra);
   else
-    ecs_launch_pdl(k_reduce<T, 1, M>, dot_blocks(ctx, n), kB, 0, ctx->stream, n, v, ctx->red, div, out, kd, cond, use_graph);
+    ecs_launch_pdl(k_reduce<T, 1, M>, dot_blocks(ctx, n), kB, 0, ctx->stream, n, v, ctx->red, div, out, kd, cond, use_graph, ra);
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
@@ -2110,30 +2260,34 @@ template <>
 double *basis_z<double>(EcsCtx *ctx) { return ctx->kz64; }
 template <>
 float *basis_z<float>(EcsCtx *ctx) { return ctx->kz32; }
-// right-hand side and correction of the FGMRES cycle in precision T
+// right-hand side of the FGMRES cycle in precision T
 template <typename T>
 T *cycle_b(EcsCtx *ctx);
 template <>
 double *cycle_b<double>(EcsCtx *ctx) { return ctx->r64; }
 template <>
 float *cycle_b<float>(EcsCtx *ctx) { return ctx->kz32 + (size_t)ctx->krylov_m * ctx->ncell; }
+// Kernels before the Arnoldi loop: the cycle's right-hand side (mixed: the
+// normalised FP64 residual, r64 or, with first = rhs in a graph's first sweep,
+// the right-hand side), its norm, V_0.
 template <typename T>
-T *cycle_x(EcsCtx *ctx);
-template <>
-double *cycle_x<double>(EcsCtx *ctx) { return ctx->w64; }
-template <>
-float *cycle_x<float>(EcsCtx *ctx) { return ctx->kz32 + (size_t)(ctx->krylov_m + 1) * ctx->ncell; }
-
-// Kernels before the Arnoldi loop: ||b||, V_0, x = 0.
-template <typename T>
-int cycle_pre(EcsCtx *ctx, cudaGraphConditionalHandle cond, int use_graph) {
+int cycle_pre(EcsCtx *ctx, const double *first, cudaGraphConditionalHandle cond, int use_graph) {
   const size_t n = ctx->ncell;
   KrylovDev *kd = (KrylovDev *)ctx->kdev;
   Multigrid<T> &mg = mg_of<T>(ctx);
-  const T *b = cycle_b<T>(ctx);
-  int rc = launch_reduce<T, kRedBeta>(ctx, n, b, 1.0, nullptr, cond, use_graph);
-  if (rc) return rc;
-  ecs_launch_pdl(k_cycle_start<T>, blocks_for(ctx, n), kB, 0, ctx->stream, n, b, basis_v<T>(ctx), mg.lv[0].b, cycle_x<T>(ctx), kd);
+  T *b = cycle_b<T>(ctx);
+  if constexpr (sizeof(T) == 4) {
+    const RefineDev *rd = first ? (const RefineDev *)ctx->rdev : nullptr;
+    if (packed4(n))
+      ecs_launch_pdl(k_scale_beta<4>, dot_blocks(ctx, n / 4), kB, 0, ctx->stream, n / 4, first, ctx->r64, rd, ctx->dots + 1, b, ctx->red, kd, cond, use_graph);
+    else
+      ecs_launch_pdl(k_scale_beta<1>, dot_blocks(ctx, n), kB, 0, ctx->stream, n, first, ctx->r64, rd, ctx->dots + 1, b, ctx->red, kd, cond, use_graph);
+    ECS_LAUNCHED(ctx);
+  } else {
+    int rc = launch_reduce<T, kRedBeta>(ctx, n, b, 1.0, nullptr, cond, use_graph);
+    if (rc) return rc;
+  }
+  ecs_launch_pdl(k_cycle_start<T>, blocks_for(ctx, n), kB, 0, ctx->stream, n, b, basis_v<T>(ctx), mg.lv[0].b, kd);
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
@@ -2157,46 +2311,60 @@ int cycle_step(EcsCtx *ctx, cudaGraphConditionalHandle cond, int use_graph) {
   }
   ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.x, mean, Z, V, kd);
   ECS_LAUNCHED(ctx);
-  // classical Gram-Schmidt, two passes (the second ends with the Arnoldi
-  // bookkeeping)
+  // classical Gram-Schmidt, two passes
   constexpr int W = kPack<T>;
   if (packed4(n)) {
     const unsigned nb = dot_blocks(ctx, n / W);
     ecs_launch_pdl(k_dots1<T, W>, nb, kB, 0, ctx->stream, n, V, kd, ctx->red);
     ECS_LAUNCHED(ctx);
-    ecs_launch_pdl(k_orth1_dots2<T, W>, nb, kB, 0, ctx->stream, n, V, kd, ctx->red, cond, use_graph);
+    ecs_launch_pdl(k_orth1_dots2<T, W>, nb, kB, 0, ctx->stream, n, V, kd, ctx->red);
     ECS_LAUNCHED(ctx);
   } else {
     const unsigned nb = dot_blocks(ctx, n);
     ecs_launch_pdl(k_dots1<T, 1>, nb, kB, 0, ctx->stream, n, V, kd, ctx->red);
     ECS_LAUNCHED(ctx);
-    ecs_launch_pdl(k_orth1_dots2<T, 1>, nb, kB, 0, ctx->stream, n, V, kd, ctx->red, cond, use_graph);
+    ecs_launch_pdl(k_orth1_dots2<T, 1>, nb, kB, 0, ctx->stream, n, V, kd, ctx->red);
     ECS_LAUNCHED(ctx);
   }
   if (packed4(n))
-    ecs_launch_pdl(k_orth2_scale<T, W>, blocks_for(ctx, n / W), kB, 0, ctx->stream, n, V, kd, L0.b);
+    ecs_launch_pdl(k_orth2_scale<T, W>, blocks_for(ctx, n / W) + 1, kB, 0, ctx->stream, n, V, kd, L0.b, cond, use_graph);
   else
-    ecs_launch_pdl(k_orth2_scale<T, 1>, blocks_for(ctx, n), kB, 0, ctx->stream, n, V, kd, L0.b);
+    ecs_launch_pdl(k_orth2_scale<T, 1>, blocks_for(ctx, n) + 1, kB, 0, ctx->stream, n, V, kd, L0.b, cond, use_graph);
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
 
-// Kernels after the loop: x = sum_q y_q Z_q.
+// Kernels after the loop: phi += (||r||) sum_q y_q Z_q, mean projection.
+template <typename T, int W, bool MEAN>
+void launch_finish(EcsCtx *ctx) {
+  const size_t n = ctx->ncell;
+  ecs_launch_pdl(k_cycle_finish<T, W, MEAN>, dot_blocks(ctx, n / W), kB, 0, ctx->stream, n / W, n, basis_z<T>(ctx),
+                 (KrylovDev *)ctx->kdev, sizeof(T) == 4 ? ctx->dots : nullptr, ctx->phi, ctx->red, ctx->dots + 2);
+}
 template <typename T>
 int cycle_post(EcsCtx *ctx) {
   const size_t n = ctx->ncell;
-  KrylovDev *kd = (KrylovDev *)ctx->kdev;
-  ecs_launch_pdl(k_cycle_solve, 1, 32, 0, ctx->stream, kd);
+  constexpr int W = kPack<double>;
+  const bool mean = fully_periodic(ctx);
+  if (packed4(n)) {
+    if (mean) launch_finish<T, W, true>(ctx);
+    else launch_finish<T, W, false>(ctx);
+  } else {
+    if (mean) launch_finish<T, 1, true>(ctx);
+    else launch_finish<T, 1, false>(ctx);
+  }
   ECS_LAUNCHED(ctx);
-  ecs_launch_pdl(k_cycle_combine<T>, blocks_for(ctx, n), kB, 0, ctx->stream, n, basis_z<T>(ctx), kd, cycle_x<T>(ctx));
-  ECS_LAUNCHED(ctx);
+  if (mean) {
+    ecs_launch_pdl(k_sub_value<double>, blocks_for(ctx, n), kB, 0, ctx->stream, n, ctx->phi, ctx->dots + 2);
+    ECS_LAUNCHED(ctx);
+  }
   return ECS_OK;
 }
 
-// One FGMRES cycle on (cycle_b, cycle_x) with tolerance tol (relative to
-// ||b||) and at most maxit steps, launched from the host step by step (the
-// host reads the stop flag after each step); the control block ends up in
-// ctx->kdev_host.
+// One FGMRES cycle on r64 with tolerance tol (relative to its norm) and at
+// most maxit steps, launched from the host step by step (the host reads the
+// stop flag after each step), its correction added to phi; the control block
+// ends up in ctx->kdev_host.
 template <typename T>
 int fgmres_cycle(EcsCtx *ctx, double tol, int maxit) {
   KrylovDev *kd = (KrylovDev *)ctx->kdev;
@@ -2206,7 +2374,7 @@ int fgmres_cycle(EcsCtx *ctx, double tol, int maxit) {
   ECS_CUDA(ctx, cudaMemcpyAsync(kd, ctl, offsetof(KrylovDev, j), cudaMemcpyHostToDevice, ctx->stream));
   int rc;
   cudaGraphConditionalHandle none = 0;
-  if ((rc = cycle_pre<T>(ctx, none, 0))) return rc;
+  if ((rc = cycle_pre<T>(ctx, nullptr, none, 0))) return rc;
   KrylovDev *hk = (KrylovDev *)ctx->kdev_host;
   for (int s = 0; s < kKrylovMax; s++) {
     ECS_CUDA(ctx, cudaMemcpyAsync(&hk->done, &kd->done, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2222,81 +2390,7 @@ int norm64_dev(EcsCtx *ctx, const double *v, double *out2) {
   return launch_reduce<double, kRedNorm>(ctx, ctx->ncell, v, 1.0, out2, 0, 0);
 }
 
-template <typename T>
-int project_mean(EcsCtx *ctx, T *v) {
-  if (!fully_periodic(ctx)) return ECS_OK;
-  size_t n = ctx->ncell;
-  int rc = launch_reduce<T, kRedMean>(ctx, n, v, (double)n, ctx->dots + 2, 0, 0);
-  if (rc) return rc;
-  ecs_launch_pdl(k_sub_value<T>, blocks_for(ctx, n), kB, 0, ctx->stream, n, v, ctx->dots + 2);
-  ECS_LAUNCHED(ctx);
-  return ECS_OK;
-}
-
 // ---- the whole solve on the device ------------------------------------------
-// Device state of the iterative-refinement loop.
-struct RefineDev {
-  double bnorm, rel;
-  int its, sweeps;
-  int done;  // converged, out of iterations, stalled or non-finite
-  int nonfinite;
-};
-
-__global__ void k_solve_init(RefineDev *rd, const double *__restrict__ dots) {
-  ECS_PDL_ENTRY();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  rd->bnorm = dots[0];
-  rd->rel = 0.0;
-  rd->its = 0;
-  rd->sweeps = 0;
-  rd->done = !(dots[0] > 0.0);
-  rd->nonfinite = 0;
-}
-
-// Refinement sweeps in one solve: each sweep runs at least one FGMRES step
-// (or ends the solve), so max_it bounds them; this caps the loop regardless.
-constexpr int kMaxSweeps = 64;
-
-// Relative residual of the current sweep (norm in dots[0]); decides whether
-// another correction follows (condition `cond` of the sweep loop) and sets
-// the FGMRES tolerance and step limit of that correction.
-__global__ void k_refine_check(RefineDev *rd, KrylovDev *kd, const double *__restrict__ dots, double rtol,
-                               int max_it, double tol_floor, cudaGraphConditionalHandle cond) {
-  ECS_PDL_ENTRY();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (rd->bnorm > 0.0) {
-    const double rel = dots[0] / rd->bnorm;
-    rd->rel = rel;
-    if (!isfinite(rel)) rd->nonfinite = 1;
-  }
-  const bool stop = rd->done || rd->nonfinite || rd->rel <= rtol || rd->its >= max_it || rd->sweeps >= kMaxSweeps;
-  if (stop) {
-    rd->done = 1;
-  } else {
-    const double tol = fmax(fmax(0.5 * rtol / rd->rel, 1e-14), tol_floor);
-    kd->tol_rel = tol;
-    kd->maxit = min(kKrylovMax, max(max_it - rd->its, 1));
-  }
-  cudaGraphSetConditional(cond, stop ? 0u : 1u);
-}
-
-__global__ void k_refine_update(RefineDev *rd, const KrylovDev *__restrict__ kd) {
-  ECS_PDL_ENTRY();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  rd->its += kd->nits;
-  rd->sweeps += 1;
-  if (kd->nits == 0) rd->done = 1;
-}
-
-// x64 += scale[0] * e (scale nullptr: 1)
-template <typename T>
-__global__ void k_axpy64_dev(size_t n, const double *__restrict__ scale, const T *__restrict__ e, double *__restrict__ x) {
-  ECS_PDL_ENTRY();
-  const double a = scale ? scale[0] : 1.0;
-  for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x)
-    x[q] += a * (double)e[q];
-}
-
 // Mixed-precision residual: r64 = b64 - A64(n64) x64.
 // r = b - A x in FP64 from the stored coefficients (the same products and
 // sum as computing them in place).
@@ -2368,42 +2462,32 @@ int capture_graph(EcsCtx *ctx, cudaStream_t s, cudaGraph_t *g) {
 }
 
 template <typename T>
-int refine_decide(EcsCtx *ctx, double rtol, int max_it, cudaGraphConditionalHandle h) {
-  const double tol_floor = sizeof(T) == 4 ? 2e-6 : 0.0;
-  ecs_launch_pdl(k_refine_check, 1, 32, 0, ctx->stream, (RefineDev *)ctx->rdev, (KrylovDev *)ctx->kdev, ctx->dots, rtol, max_it,
-                                            tol_floor, h);
-  ECS_LAUNCHED(ctx);
-  return ECS_OK;
+RefineArgs refine_args(EcsCtx *ctx, double rtol, int max_it, int decide, int after) {
+  return {(RefineDev *)ctx->rdev, rtol, sizeof(T) == 4 ? 2e-6 : 0.0, max_it, decide, after};
 }
 
 // Residual of the current phi, its norm and the check that sets the sweep
 // loop's condition h (on ctx->stream).
 template <typename T>
-int refine_check(EcsCtx *ctx, double rtol, int max_it, cudaGraphConditionalHandle h) {
+int refine_check(EcsCtx *ctx, double rtol, int max_it, int after, cudaGraphConditionalHandle h) {
   const EcsParams &p = ctx->p;
   const OpK o64 = make_op(p, p.Nx, p.Ny, p.Nz, p.dx, p.dy, p.dz);
   ecs_launch_pdl(k_residual64, blocks3(o64.g), threads3(), 0, ctx->stream, o64, (const double *)ctx->coef64, ctx->phi, ctx->rhs, ctx->r64);
   ECS_LAUNCHED(ctx);
-  int rc = norm64_dev(ctx, ctx->r64, ctx->dots);
-  if (rc) return rc;
-  return refine_decide<T>(ctx, rtol, max_it, h);
+  return launch_reduce<double, kRedCheck>(ctx, ctx->ncell, ctx->r64, 1.0, ctx->dots, h, 1,
+                                          refine_args<T>(ctx, rtol, max_it, 1, after));
 }
 
 // The correction of one sweep: the FGMRES cycle (the Arnoldi loop as a WHILE
 // node captured on capture stream `lvl`), phi update, mean projection.
 template <typename T>
-int refine_correct(EcsCtx *ctx, int lvl) {
-  const size_t n = ctx->ncell;
+int refine_correct(EcsCtx *ctx, int lvl, int warm) {
   int rc;
-  if (sizeof(T) == 4) {  // the normalised FP64 residual to FP32
-    ecs_launch_pdl(k_scale_to<float>, blocks_for(ctx, n), kB, 0, ctx->stream, n, ctx->r64, ctx->dots + 1, (float *)cycle_b<T>(ctx));
-    ECS_LAUNCHED(ctx);
-  }
   cudaGraph_t g = nullptr, body = nullptr;
   if ((rc = capture_graph(ctx, ctx->stream, &g))) return rc;
   cudaGraphConditionalHandle hw;
   ECS_CUDA(ctx, cudaGraphConditionalHandleCreate(&hw, g, 0, 0));
-  if ((rc = cycle_pre<T>(ctx, hw, 1))) return rc;
+  if ((rc = cycle_pre<T>(ctx, warm ? nullptr : ctx->rhs, hw, 1))) return rc;
   if ((rc = capture_conditional(ctx, ctx->stream, hw, cudaGraphCondTypeWhile, &body))) return rc;
   cudaStream_t outer = ctx->stream;
   ctx->stream = ctx->capst[lvl];
@@ -2415,20 +2499,13 @@ int refine_correct(EcsCtx *ctx, int lvl) {
   ctx->stream = outer;
   if (rc) return rc;
   ECS_CUDA(ctx, ce);
-  if ((rc = cycle_post<T>(ctx))) return rc;
-  ecs_launch_pdl(k_axpy64_dev<T>, blocks_for(ctx, n), kB, 0, ctx->stream, n, sizeof(T) == 4 ? ctx->dots : nullptr,
-                                                             cycle_x<T>(ctx), ctx->phi);
-  ECS_LAUNCHED(ctx);
-  if ((rc = project_mean<double>(ctx, ctx->phi))) return rc;
-  ecs_launch_pdl(k_refine_update, 1, 32, 0, ctx->stream, (RefineDev *)ctx->rdev, (const KrylovDev *)ctx->kdev);
-  ECS_LAUNCHED(ctx);
-  return ECS_OK;
+  return cycle_post<T>(ctx);
 }
 
 // The nodes of one solve, appended to the graph being captured on
 // ctx->stream:
-//   [phi = 0, r = b | r = b - A phi]  ||r||  init  check
-//   WHILE( scale  cycle(WHILE Arnoldi)  phi += e  update  residual  norm  check )
+//   [phi = 0, r = b | r = b - A phi]  ||r||, init, check
+//   WHILE( scale, beta  cycle(WHILE Arnoldi)  phi += e  residual  norm, check )
 // The checks set the sweep loop's condition; everything stays on the device.
 // The kernel counts of the head, a sweep and an Arnoldi step go to sgraph.
 template <typename T>
@@ -2440,23 +2517,25 @@ int capture_solve(EcsCtx *ctx, double rtol, int max_it, int warm) {
   cudaError_t ce;
   cudaGraph_t top = nullptr;
   if ((rc = capture_graph(ctx, ctx->stream, &top))) return rc;
-  if ((rc = norm64_dev(ctx, ctx->rhs, ctx->dots))) return rc;  // ||b||
-  ecs_launch_pdl(k_solve_init, 1, 32, 0, ctx->stream, (RefineDev *)ctx->rdev, ctx->dots);
-  ECS_LAUNCHED(ctx);
-  if (identity_lhs(ctx)) {  // -lhs identity (ComputeIdentityLHS, src/lhs.c:11-23): phi = b exactly
+  const bool identity = identity_lhs(ctx);
+  cudaGraphConditionalHandle hs = 0;
+  if (!identity) ECS_CUDA(ctx, cudaGraphConditionalHandleCreate(&hs, top, 0, cudaGraphCondAssignDefault));
+  // ||b||; from phi = 0 the residual is b, and the same norm decides
+  rc = launch_reduce<double, kRedInit>(ctx, n, ctx->rhs, 1.0, ctx->dots, hs, 1,
+                                       refine_args<T>(ctx, rtol, max_it, !warm && !identity, 0));
+  if (rc) return rc;
+  if (identity) {  // -lhs identity (ComputeIdentityLHS, src/lhs.c:11-23): phi = b exactly
     ECS_CUDA(ctx, cudaMemcpyAsync(ctx->phi, ctx->rhs, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     sg.k_head = ctx->launches - launches0;
     sg.k_sweep = sg.k_step = 0;
     return ECS_OK;
   }
-  cudaGraphConditionalHandle hs;
-  ECS_CUDA(ctx, cudaGraphConditionalHandleCreate(&hs, top, 0, cudaGraphCondAssignDefault));
-  if (!warm) {  // phi = 0: the residual is b and its norm is known
+  if (!warm) {
     ECS_CUDA(ctx, cudaMemsetAsync(ctx->phi, 0, n * sizeof(double), ctx->stream));
-    ECS_CUDA(ctx, cudaMemcpyAsync(ctx->r64, ctx->rhs, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-    rc = refine_decide<T>(ctx, rtol, max_it, hs);
+    if (sizeof(T) == 8)  // the mixed cycle reads b itself in its first sweep
+      ECS_CUDA(ctx, cudaMemcpyAsync(ctx->r64, ctx->rhs, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   } else {
-    rc = refine_check<T>(ctx, rtol, max_it, hs);
+    rc = refine_check<T>(ctx, rtol, max_it, 0, hs);
   }
   if (rc) return rc;
   sg.k_head = ctx->launches - launches0;
@@ -2470,8 +2549,8 @@ int capture_solve(EcsCtx *ctx, double rtol, int max_it, int warm) {
     return ecs_cuda_check(ctx, ce, "sweep capture");
   }
   const int64_t l1 = ctx->launches;
-  rc = refine_correct<T>(ctx, 2);
-  if (!rc) rc = refine_check<T>(ctx, rtol, max_it, hs);
+  rc = refine_correct<T>(ctx, 2, warm);
+  if (!rc) rc = refine_check<T>(ctx, rtol, max_it, 1, hs);
   sg.k_sweep = ctx->launches - l1 - sg.k_step;
   ce = cudaStreamEndCapture(ctx->stream, &body);
   ctx->stream = outer;
@@ -2690,7 +2769,6 @@ int ecs_solver_alloc(EcsCtx *ctx) {
     ECS_CUDA(ctx, cudaMalloc((void **)&ctx->dots, (size_t)(m + 2) * sizeof(double)));
     ECS_CUDA(ctx, cudaMallocHost((void **)&ctx->h_dots, (size_t)(m + 2) * sizeof(double)));
     ECS_CUDA(ctx, cudaMalloc((void **)&ctx->r64, n * sizeof(double)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->w64, n * sizeof(double)));
     ECS_CUDA(ctx, cudaMalloc(&ctx->kdev, sizeof(KrylovDev)));
     ECS_CUDA(ctx, cudaMemset(ctx->kdev, 0, sizeof(KrylovDev)));
     ECS_CUDA(ctx, cudaMallocHost(&ctx->kdev_host, sizeof(KrylovDev)));
@@ -2708,9 +2786,9 @@ int ecs_solver_alloc(EcsCtx *ctx) {
     ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kz64, (size_t)m * n * sizeof(double)));
   }
   if (ctx->prec == ECS_PREC_MIXED && !ctx->kv32) {
-    // V, Z and two extra FP32 vectors (normalised residual, correction)
+    // V, Z and the normalised residual
     ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kv32, (size_t)(m + 1) * n * sizeof(float)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kz32, (size_t)(m + 2) * n * sizeof(float)));
+    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kz32, (size_t)(m + 1) * n * sizeof(float)));
   }
   return ECS_OK;
 }
@@ -2816,17 +2894,11 @@ int ecs_solver_run(EcsCtx *ctx, double rtol, int max_it, int warm, EcsSolveStats
       const double tol_cycle = std::max(0.5 * rtol / rel, 1e-14);
       if (ctx->prec == ECS_PREC_FP64) {
         // the cycle solves A e = r64 directly (beta = ||r64||)
-        if ((rc = fgmres_cycle<double>(ctx, tol_cycle, max_it - its))) return rc;
-        ecs_launch_pdl(k_axpy64<double>, blocks_for(ctx, n), kB, 0, ctx->stream, n, 1.0, ctx->w64, ctx->phi);
+        rc = fgmres_cycle<double>(ctx, tol_cycle, max_it - its);
       } else {
-        float *r32 = cycle_b<float>(ctx), *e32 = cycle_x<float>(ctx);
-        ecs_launch_pdl(k_scale_to<float>, blocks_for(ctx, n), kB, 0, ctx->stream, n, ctx->r64, ctx->dots + 1, r32);
-        ECS_LAUNCHED(ctx);
-        if ((rc = fgmres_cycle<float>(ctx, std::max(tol_cycle, 2e-6), max_it - its))) return rc;
-        ecs_launch_pdl(k_axpy64<float>, blocks_for(ctx, n), kB, 0, ctx->stream, n, rn, e32, ctx->phi);
+        rc = fgmres_cycle<float>(ctx, std::max(tol_cycle, 2e-6), max_it - its);
       }
-      ECS_LAUNCHED(ctx);
-      if ((rc = project_mean<double>(ctx, ctx->phi))) return rc;
+      if (rc) return rc;
       cycle_pending = true;
     }
   }
@@ -2870,7 +2942,7 @@ int ecs_solver_free(EcsCtx *ctx) {
     if (e) cudaEventDestroy(e);
   free_mg(ctx->mg64);
   free_mg(ctx->mg32);
-  void *ptrs[] = {ctx->kv64, ctx->kz64, ctx->kv32, ctx->kz32, ctx->w64, ctx->r64, ctx->coef64, ctx->dots, ctx->red,
+  void *ptrs[] = {ctx->kv64, ctx->kz64, ctx->kv32, ctx->kz32, ctx->r64, ctx->coef64, ctx->dots, ctx->red,
                   ctx->kdev, ctx->rdev};
   for (void *q : ptrs)
     if (q) cudaFree(q);
