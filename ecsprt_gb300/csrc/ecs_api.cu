@@ -122,7 +122,7 @@ int64_t ecs_ctx_device_bytes(const EcsParams *p, int precision, int64_t cap) {
   // multigrid: 7 cell arrays (11 in FP64 and for columns of more than 128
   // cells) and 2 plane arrays a level, levels summing to at most 8/7 of the
   // finest; the coarsest level's inverse (<= 128 cells)
-  b += (n * (precision == ECS_PREC_FP64 || p->Nz > 128 ? 11 : 7) + n / 4) * t * 8 / 7 + 128 * 128 * 3 * t;
+  b += (n * (precision == ECS_PREC_FP64 || p->Nz > 128 ? 11 : 7) + n / 4) * t * 8 / 7 + 128 * 128 * t;
   if (precision == ECS_PREC_FP64) {
     b += (2 * m + 1) * n * 8;  // Krylov bases V, Z
     b += cap * 48 + ne * 32;   // ions (6 FP64), E numerators

@@ -79,7 +79,6 @@ struct Multigrid {
   bool built = false;
   // explicit inverse of the coarsest operator (transposed), when it is small
   T *cinv = nullptr;
-  T *cwork = nullptr;  // Gauss-Jordan work matrix [n][2n]
   CoarseShape cluster;
 };
 

@@ -1022,141 +1022,63 @@ static CoarseKernel<T> coarse_kernel(const CoarseShape &s) {
 }
 
 // ---- direct solve of the coarsest level -----------------------------------------
-constexpr int kDirectMax = 128;           // largest coarsest level solved directly
-constexpr size_t kInverseSmem = 160 * 1024;  // shared memory of its Gauss-Jordan work matrix
-// One block of 32 warps (fewer warps make a pivot step slower: the row
-// updates dominate, not the barriers).
-constexpr int kInvThreads = 1024;
+constexpr int kDirectMax = 128;  // largest coarsest level solved directly
+constexpr int kInvTpr = 8;       // threads a row up to 64 cells
 
-// invT = (A + sigma 1 1^T)^-1, transposed (invT[k n + r] = inv[r][k]), by
-// Gauss-Jordan elimination with partial pivoting on M = [A | I] (n x 2n, in
-// global memory), one block.  sigma = mean |A_rr| / n removes the constant
-// null space of a fully periodic operator (regularize = 1); without it the
-// operator is regular.  Pivot ties go to the lowest row, so the result is
-// reproducible.
-template <typename T>
-__global__ void __launch_bounds__(kInvThreads) k_coarse_inverse(OpK o, const T *__restrict__ dens, int regularize,
-                                                         T *__restrict__ Mg, T *__restrict__ invT) {
-  ECS_PDL_ENTRY();
-  extern __shared__ unsigned char inv_smem[];
-  T *M = Mg ? Mg : reinterpret_cast<T *>(inv_smem);  // work matrix in shared memory when it fits
-  __shared__ T fac[kDirectMax];
-  __shared__ T wv[32];
-  __shared__ int piv;
-  __shared__ T sigma;
-  const GridG &g = o.g;
-  const int n = (int)g.n, w = 2 * n, tid = threadIdx.x, bs = blockDim.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < n * w; e += bs) M[e] = T(0);
-  __syncthreads();
-  for (int r = tid; r < n; r += bs) {
-    int i, j, k;
-    cell_ijk((unsigned)r, g, i, j, k);
-    T v[11];
-    row11(dens, o, i, j, k, v);
-    for (int e = 0; e < 11; e++) {
-      int ii = i + off_i(e), jj = j + off_j(e), kk = k + off_k(e);
-      bool out = false;
-      if (ii < 0 || ii >= g.nx) { if (g.bc[0]) out = true; else ii = ii < 0 ? ii + g.nx : ii - g.nx; }
-      if (jj < 0 || jj >= g.ny) { if (g.bc[1]) out = true; else jj = jj < 0 ? jj + g.ny : jj - g.ny; }
-      if (kk < 0 || kk >= g.nz) { if (g.bc[2]) out = true; else kk = kk < 0 ? kk + g.nz : kk - g.nz; }
-      if (!out) M[(size_t)r * w + ((kk * g.ny + jj) * g.nx + ii)] += v[e];
-    }
-    M[(size_t)r * w + n + r] = T(1);
-  }
-  __syncthreads();
-  if (regularize) {
-    T t = T(0);
-    for (int r = tid; r < n; r += bs) t += fabs(M[(size_t)r * w + r]);
-    for (int s = 16; s >= 1; s >>= 1) t += __shfl_xor_sync(ECS_FULL_MASK, t, s);
-    if (lane == 0) wv[warp] = t;
-    __syncthreads();
-    if (tid == 0) {
-      T u = T(0);
-      for (int q = 0; q < (bs >> 5); q++) u += wv[q];
-      sigma = u / (T(n) * T(n));
-    }
-    __syncthreads();
-    for (int e = tid; e < n * n; e += bs) M[(size_t)(e / n) * w + (e % n)] += sigma;
-    __syncthreads();
-  }
-  // elimination: rows by warp, columns by lane
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int c = 0; c < n; c++) {
-    // pivot: largest |M[r][c]|, r >= c, lowest row on ties (warp 0)
-    if (ty == 0) {
-      T best = T(-1);
-      int bi = n;
-      for (int r = c + tx; r < n; r += 32) {
-        const T a = fabs(M[(size_t)r * w + c]);
-        if (a > best) { best = a; bi = r; }
-      }
-      for (int s = 16; s >= 1; s >>= 1) {
-        const T ob = __shfl_xor_sync(ECS_FULL_MASK, best, s);
-        const int oi = __shfl_xor_sync(ECS_FULL_MASK, bi, s);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      if (tx == 0) {
-        piv = bi < n ? bi : c;
-        const T pv = M[(size_t)piv * w + c];
-        sigma = pv != T(0) ? T(1) / pv : T(0);  // reused as 1 / pivot
-      }
-    }
-    __syncthreads();
-    const int pr = piv;
-    if (pr != c)
-      for (int e = threadIdx.x; e < w; e += blockDim.x) {
-        const T t = M[(size_t)c * w + e];
-        M[(size_t)c * w + e] = M[(size_t)pr * w + e];
-        M[(size_t)pr * w + e] = t;
-      }
-    __syncthreads();
-    const T ip = sigma;
-    for (int e = threadIdx.x; e < w; e += blockDim.x) M[(size_t)c * w + e] *= ip;
-    for (int r = threadIdx.x; r < n; r += blockDim.x) fac[r] = r == c ? T(0) : M[(size_t)r * w + c];
-    __syncthreads();
-    for (int r = ty; r < n; r += bs >> 5) {
-      const T f = fac[r];
-      if (f != T(0))
-        for (int q = tx; q < w; q += 32) M[(size_t)r * w + q] -= f * M[(size_t)c * w + q];
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < n * n; e += bs) {
-    const int r = e / n, k = e - r * n;
-    invT[(size_t)k * n + r] = M[(size_t)r * w + n + k];
-  }
+// Order-preserving integer of |a|: 0 for a NaN, which is never a pivot.
+__device__ __forceinline__ unsigned pivot_key(float a) {
+  return isnan(a) ? 0u : (__float_as_uint(a) & 0x7fffffffu) + 1u;
+}
+__device__ __forceinline__ unsigned long long pivot_key(double a) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+  return b > 0x7ff0000000000000ull ? 0ull : b + 1ull;
+}
+__device__ __forceinline__ unsigned warp_max_key(unsigned k) { return __reduce_max_sync(ECS_FULL_MASK, k); }
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) {
+  const unsigned hi = __reduce_max_sync(ECS_FULL_MASK, (unsigned)(k >> 32));
+  const unsigned lo = __reduce_max_sync(ECS_FULL_MASK, (unsigned)(k >> 32) == hi ? (unsigned)k : 0u);
+  return ((unsigned long long)hi << 32) | lo;
 }
 
-// The same inverse for n <= kRegInvMax with the work matrix in registers:
-// row r of M = [A | I] belongs to the tpr threads tid / tpr == r, thread jr
-// holding columns jr + tpr u.  Pivoting is implicit: the pivot of column c
-// is the largest |M[r][c]| among rows not yet used (lowest row on ties),
-// and the row used at step c ends up holding row c of the inverse.  Each
-// step needs two barriers: column c and the scaled pivot row pass through
-// shared memory (double-buffered by the parity of c).
-constexpr int kRegInvMax = 64;
-constexpr int kRegCols = 2 * kRegInvMax * kRegInvMax / kInvThreads;  // 8 columns a thread
-template <typename T>
-__global__ void __launch_bounds__(kInvThreads) k_coarse_inverse_reg(OpK o, const T *__restrict__ dens,
-                                                                    int regularize, T *__restrict__ invT) {
+// invT = (A + sigma 1 1^T)^-1, transposed (invT[k n + r] = inv[r][k]), by
+// Gauss-Jordan elimination with partial pivoting, one block, the matrix in
+// registers: row r belongs to the TPR threads tid / TPR == r, thread jr
+// holding columns jr + TPR u (u < COLS).  sigma = mean |A_rr| / n removes the
+// constant null space of a fully periodic operator (regularize = 1); without
+// it the operator is regular.
+// The elimination is in place: when row pr is the pivot of column c, the
+// column has served its purpose, and its slot takes the column of the inverse
+// that starts there (identity column pr).  Pivoting is implicit: the pivot of
+// column c is the largest |M[r][c]| among rows not yet used; the row used at
+// step c ends up holding row c of the inverse.  Ties go to the lowest row
+// (SWAP: to the lowest position, as if rows c and pr were exchanged at each
+// step), so the result is reproducible.
+// A step needs two barriers: column c and the scaled pivot row pass through
+// shared memory (double-buffered by the parity of c), and every warp finds the
+// pivot for itself, with integer compares of |a|'s bits and warp maxima.  In
+// FP64 that matters most: compares and a reciprocal in all 32 warps, and the
+// half of [A | I] that is known to be zero or done, kept the one FP64 pipe
+// busy for 644 us at 64 cells (157 us now; FP32 74 -> 35 us).
+template <typename T, int ROWS, int TPR, bool SWAP>
+__global__ void __launch_bounds__(ROWS *TPR) k_coarse_inverse(OpK o, const T *__restrict__ dens, int regularize,
+                                                              T *__restrict__ invT) {
   ECS_PDL_ENTRY();
-  __shared__ T colbuf[2][kRegInvMax];
-  __shared__ T prow[2][2 * kRegInvMax];
-  __shared__ int rowpos[kRegInvMax];
+  constexpr int COLS = ROWS / TPR, RPL = ROWS / 32;  // columns a thread, rows a lane (pivot search)
+  __shared__ T colbuf[2][ROWS];
+  __shared__ T prow[2][ROWS];
+  __shared__ int rowpos[ROWS], colrow[ROWS];  // step at which a row was the pivot, and the other way round
   __shared__ T wsum[32];
   __shared__ T sigma;
   const GridG &g = o.g;
-  const int n = (int)g.n, w = 2 * n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int tpr = n <= 32 ? 32 : 16;  // threads a row
-  const int r = tid / tpr, jr = tid % tpr;
+  const int n = (int)g.n, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r = tid / TPR, jr = tid % TPR;
   const bool live = r < n;
   // Every access to M below has a compile-time index (u), so M stays in
   // registers.
-  T M[kRegCols];
+  T M[COLS];
 #pragma unroll
-  for (int u = 0; u < kRegCols; u++) M[u] = T(0);
-  if (live) {  // row r: the operator's entries in the reference's order, then the identity
+  for (int u = 0; u < COLS; u++) M[u] = T(0);
+  if (live) {  // row r: the operator's entries in the reference's order
     int i, j, k;
     cell_ijk((unsigned)r, g, i, j, k);
     T v[11];
@@ -1172,18 +1094,17 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_inverse_reg(OpK o, const
       tc[e] = out ? -1 : (kk * g.ny + jj) * g.nx + ii;
     }
 #pragma unroll
-    for (int u = 0; u < kRegCols; u++) {
-      const int q = jr + tpr * u;
+    for (int u = 0; u < COLS; u++) {
+      const int q = jr + TPR * u;
 #pragma unroll
       for (int e = 0; e < 11; e++)
         if (tc[e] == q) M[u] += v[e];
-      if (q == n + r) M[u] = T(1);
     }
   }
   if (regularize) {  // sigma = sum |A_rr| / n^2 over the diagonal, added to every entry of A
 #pragma unroll
-    for (int u = 0; u < kRegCols; u++)
-      if (live && jr + tpr * u == r) colbuf[0][r] = fabs(M[u]);
+    for (int u = 0; u < COLS; u++)
+      if (live && jr + TPR * u == r) colbuf[0][r] = fabs(M[u]);
     __syncthreads();
     T t = tid < n ? colbuf[0][tid] : T(0);
     for (int s2 = 16; s2 >= 1; s2 >>= 1) t += __shfl_xor_sync(ECS_FULL_MASK, t, s2);
@@ -1191,71 +1112,79 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_inverse_reg(OpK o, const
     __syncthreads();
     if (tid == 0) {
       T u2 = T(0);
-      for (int q = 0; q < (kInvThreads >> 5); q++) u2 += wsum[q];
+      for (int q = 0; q < ROWS * TPR / 32; q++) u2 += wsum[q];
       sigma = u2 / (T(n) * T(n));
     }
     __syncthreads();
     const T sg = sigma;
 #pragma unroll
-    for (int u = 0; u < kRegCols; u++)
-      if (live && jr + tpr * u < n) M[u] += sg;
+    for (int u = 0; u < COLS; u++)
+      if (live && jr + TPR * u < n) M[u] += sg;
   }
   __syncthreads();  // colbuf[0] is free again
   if (live && jr == 0) colbuf[0][r] = M[0];  // column 0
-  unsigned long long used = 0ull;
-  // step c = j0 + tpr u0: column c is column u0 of the threads jr == j0
+  // the lane's rows lane + 32 g2 in the pivot search: their positions, -1 once used
+  int pos[RPL];
 #pragma unroll
-  for (int u0 = 0; u0 < kRegCols; u0++) {
-    for (int j0 = 0; j0 < tpr; j0++) {
-      const int c = j0 + tpr * u0;
+  for (int g2 = 0; g2 < RPL; g2++) pos[g2] = lane + 32 * g2 < n ? lane + 32 * g2 : -1;
+  // step c = j0 + TPR u0: column c is column u0 of the threads jr == j0
+#pragma unroll
+  for (int u0 = 0; u0 < COLS; u0++) {
+#pragma unroll 1
+    for (int j0 = 0; j0 < TPR; j0++) {
+      const int c = j0 + TPR * u0;
       if (c >= n) break;
       const int b = c & 1;
       __syncthreads();  // column c complete
-      T best = T(-1);
-      int bi = n;
-      for (int rr = lane; rr < n; rr += 32) {
-        if ((used >> rr) & 1ull) continue;
-        const T a = fabs(colbuf[b][rr]);
-        if (a > best) { best = a; bi = rr; }
-      }
-      for (int s2 = 16; s2 >= 1; s2 >>= 1) {
-        const T ob = __shfl_xor_sync(ECS_FULL_MASK, best, s2);
-        const int oi = __shfl_xor_sync(ECS_FULL_MASK, bi, s2);
-        if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-      }
-      const int pr = bi < n ? bi : __ffsll((long long)~used) - 1;
-      used |= 1ull << pr;
-      const T pv = colbuf[b][pr];
-      const T ip = pv != T(0) ? T(1) / pv : T(0);
-      if (tid == 0) rowpos[pr] = c;
-      if (r == pr) {
+      decltype(pivot_key(T(0))) key[RPL], best = 0;
 #pragma unroll
-        for (int u = 0; u < kRegCols; u++) {
-          const int q = jr + tpr * u;
-          if (q < w) {
-            M[u] *= ip;
-            prow[b][q] = M[u];
-          }
+      for (int g2 = 0; g2 < RPL; g2++) {
+        key[g2] = pos[g2] >= 0 ? pivot_key(colbuf[b][lane + 32 * g2]) : 0;
+        best = key[g2] > best ? key[g2] : best;
+      }
+      best = warp_max_key(best);
+      // the lowest position among the candidates (all unused rows if every one is NaN)
+      unsigned cand = 0xffffffffu;  // position << 8 | row
+#pragma unroll
+      for (int g2 = 0; g2 < RPL; g2++)
+        if (pos[g2] >= 0 && key[g2] == best) cand = min(cand, ((unsigned)pos[g2] << 8) | (unsigned)(lane + 32 * g2));
+      cand = __reduce_min_sync(ECS_FULL_MASK, cand);
+      const int pr = (int)(cand & 255u), ppos = (int)(cand >> 8);
+#pragma unroll
+      for (int g2 = 0; g2 < RPL; g2++) {
+        if (SWAP && pos[g2] == c) pos[g2] = ppos;  // the row at position c moves to the pivot's
+        if (lane + 32 * g2 == pr) pos[g2] = -1;
+      }
+      if (tid == 0) {
+        rowpos[pr] = c;
+        colrow[c] = pr;
+      }
+      if (r == pr) {
+        const T pv = colbuf[b][pr];
+        const T ip = pv != T(0) ? T(1) / pv : T(0);
+        if (jr == j0) M[u0] = T(1);
+#pragma unroll
+        for (int u = 0; u < COLS; u++) {
+          M[u] *= ip;
+          prow[b][jr + TPR * u] = M[u];
         }
       }
       __syncthreads();  // scaled pivot row complete
       if (live && r != pr) {
         const T f = colbuf[b][r];
+        if (jr == j0) M[u0] = T(0);
         if (f != T(0)) {
 #pragma unroll
-          for (int u = 0; u < kRegCols; u++) {
-            const int q = jr + tpr * u;
-            if (q < w) M[u] -= f * prow[b][q];
-          }
+          for (int u = 0; u < COLS; u++) M[u] -= f * prow[b][jr + TPR * u];
         }
       }
       // column c + 1 for the next step: column u0 of j0 + 1, or column
       // u0 + 1 of thread 0 of the row
       if (live && c + 1 < n) {
-        if (j0 + 1 < tpr) {
+        if (j0 + 1 < TPR) {
           if (jr == j0 + 1) colbuf[b ^ 1][r] = M[u0];
-        } else if (u0 + 1 < kRegCols) {
-          if (jr == 0) colbuf[b ^ 1][r] = M[u0 + 1 < kRegCols ? u0 + 1 : u0];
+        } else if (u0 + 1 < COLS) {
+          if (jr == 0) colbuf[b ^ 1][r] = M[u0 + 1 < COLS ? u0 + 1 : u0];
         }
       }
     }
@@ -1264,9 +1193,9 @@ __global__ void __launch_bounds__(kInvThreads) k_coarse_inverse_reg(OpK o, const
   if (live) {
     const int row = rowpos[r];
 #pragma unroll
-    for (int u = 0; u < kRegCols; u++) {
-      const int q = jr + tpr * u;
-      if (q >= n && q < w) invT[(size_t)(q - n) * n + row] = M[u];
+    for (int u = 0; u < COLS; u++) {
+      const int q = jr + TPR * u;
+      if (q < n) invT[(size_t)colrow[q] * n + row] = M[u];
     }
   }
 }
@@ -1953,7 +1882,6 @@ int mg_alloc(EcsCtx *ctx) {
   const size_t nc = mg.lv.back().n;
   if (nc <= (size_t)kDirectMax) {
     ECS_CUDA(ctx, cudaMalloc((void **)&mg.cinv, nc * nc * sizeof(T)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&mg.cwork, nc * 2 * nc * sizeof(T)));
   } else if constexpr (sizeof(T) == 4) {
     const MgLevel<T> &C = mg.lv.back();
     CoarseShape cs = coarse_shape(C.nx, C.ny, C.nz);
@@ -2073,19 +2001,11 @@ int mg_setup(EcsCtx *ctx) {
   ECS_CUDA(ctx, cudaEventRecord(ctx->sev[2], sb));
   if (mg.cinv) {
     MgLevel<T> &C = mg.lv.back();
-    const size_t bytes = C.n * 2 * C.n * sizeof(T);
-    const bool in_smem = bytes <= kInverseSmem;
-    static std::atomic<bool> attr_set[2];  // zero-initialised: false
-    if (!attr_set[sizeof(T) == 8]) {
-      ECS_CUDA(ctx, cudaFuncSetAttribute(k_coarse_inverse<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInverseSmem));
-      attr_set[sizeof(T) == 8] = true;
-    }
-    if (C.n <= (size_t)kRegInvMax)
-      ecs_launch_pdl(k_coarse_inverse_reg<T>, 1, kInvThreads, 0, sa, op_level(ctx, C), C.dens, fully_periodic(ctx) ? 1 : 0,
-                                                          mg.cinv);
+    const int reg = fully_periodic(ctx) ? 1 : 0;
+    if (C.n <= 64)
+      ecs_launch_pdl(k_coarse_inverse<T, 64, kInvTpr, false>, 1, 64 * kInvTpr, 0, sa, op_level(ctx, C), C.dens, reg, mg.cinv);
     else
-      ecs_launch_pdl(k_coarse_inverse<T>, 1, kInvThreads, in_smem ? bytes : 0, sa, 
-          op_level(ctx, C), C.dens, fully_periodic(ctx) ? 1 : 0, in_smem ? nullptr : mg.cwork, mg.cinv);
+      ecs_launch_pdl(k_coarse_inverse<T, 128, 8, true>, 1, 1024, 0, sa, op_level(ctx, C), C.dens, reg, mg.cinv);
     ECS_LAUNCHED(ctx);
   }
   ECS_CUDA(ctx, cudaEventRecord(ctx->sev[3], sa));
@@ -2417,8 +2337,7 @@ void free_mg(Multigrid<T> &mg) {
   }
   mg.lv.clear();
   if (mg.cinv) cudaFree(mg.cinv);
-  if (mg.cwork) cudaFree(mg.cwork);
-  mg.cinv = mg.cwork = nullptr;
+  mg.cinv = nullptr;
   mg.built = false;
 }
 

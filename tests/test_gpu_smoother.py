@@ -44,3 +44,19 @@ def test_iterations_at_segment_and_cluster_edges(built, grid):
     assert st.relres <= 1e-8
     assert st.iterations <= ITERATIONS[grid]
     assert np.array_equal(phi, again)  # fixed orders throughout: bit-identical on repetition
+
+
+@pytest.mark.parametrize("prec", [E.ECS_PREC_FP64, E.ECS_PREC_MIXED])
+@pytest.mark.parametrize("grid", [(4, 4, 4), (4, 4, 8), (5, 5, 5), (4, 8, 4), (5, 5, 4, "reflect"), (5, 5, 5, "reflect")],
+                         ids=lambda g: "x".join(map(str, g)))
+def test_coarsest_inverse_is_the_inverse(built, grid, prec):
+    """Grids of one level (64 to 128 cells: each kernel, and its last row) are solved
+    by the coarsest inverse alone: one or two preconditioned steps, for each
+    of the two refinement sweeps in mixed precision."""
+    nx, ny, nz = grid[:3]
+    rng = np.random.default_rng(7)
+    d = 1.0 + 0.3 * rng.standard_normal((nz, ny, nx)).clip(-2, 2)
+    with E.Context(params(grid), prec) as ctx:
+        _, st = ctx.solve_density(d)
+    assert st.relres <= 1e-8
+    assert st.iterations <= (2 if prec == E.ECS_PREC_FP64 else 4)
