@@ -48,7 +48,6 @@ struct rd {
 __device__ __forceinline__ rd operator+(rd a, rd b) { return {__dadd_rn(a.v, b.v)}; }
 __device__ __forceinline__ rd operator-(rd a, rd b) { return {__dsub_rn(a.v, b.v)}; }
 __device__ __forceinline__ rd operator*(rd a, rd b) { return {__dmul_rn(a.v, b.v)}; }
-__device__ __forceinline__ rd operator/(rd a, rd b) { return {__ddiv_rn(a.v, b.v)}; }
 
 constexpr int kBlock = 256;
 
@@ -56,11 +55,34 @@ struct TileG {
   int ntx, nty, ntz;  // tiles per axis
 };
 
+// FP64 values compare as these integers do (both zeros alike; NaNs beyond the
+// infinities, on the side of their sign).  FP64 compares issue on the FP64
+// pipe, which is the scarce one here.
+__host__ __device__ __forceinline__ long long order_key(long long bits) {
+  return bits < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)bits) : bits;
+}
+__device__ __forceinline__ long long order_key(double v) { return order_key((long long)__double_as_longlong(v)); }
+__device__ __forceinline__ bool finite64(double v) { return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000; }
+constexpr int kNoShift = 1 << 20;
+
 // ---- deposit fixed point ---------------------------------------------------
-// FP64: rint(v 2^S) by the FP64 conversion.
+// FP64: rint(v 2^S), ties to even, by shifting the significand.  GB300 issues
+// FP64 at 1/64 of the FP32 rate, and a conversion counts as FP64: the scaling
+// and the conversion of one value held the pipe as long as a hundred integer
+// instructions do the issue slots.
 struct FixScale64 {
-  double s;
-  __device__ __forceinline__ long long put(double v) const { return __double2ll_rn(v * s); }
+  double s;  // 2^S
+  int top;   // 1075 - S: a significand's right shift is top - (exponent field)
+  __device__ __forceinline__ long long put(double v) const {
+    const int hi = __double2hiint(v), sh0 = top - ((hi >> 20) & 0x7ff);
+    if (sh0 < 1) return __double2ll_rn(v * s);  // beyond every value that a deposit accepts
+    const int sh = min(sh0, 63);                // 63: rounds to 0 (zero and subnormal values too)
+    const unsigned long long m =
+        ((unsigned long long)(((unsigned)hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(v);
+    const unsigned long long q = m >> sh;
+    const unsigned long long r = (m + ((1ull << (sh - 1)) - 1ull + (q & 1ull))) >> sh;
+    return hi < 0 ? -(long long)r : (long long)r;
+  }
   // flux contribution v w
   __device__ __forceinline__ long long putvw(double v, double w) const { return put(v * w); }
 };
@@ -188,6 +210,9 @@ struct PartK {
   size_t ncell;
   double dx, dy, dz;
   double lo[3], hi[3], L[3];  // grid bounds (x0, x1, Lx per axis)
+  double dinv[3];             // 1 / cell width, rounded
+  int dsh[3];                 // cell width = 2^-dsh exactly, or kNoShift
+  long long klo[3], khi[3], kvmax;  // order_key of lo, hi and the velocity bound
   // Boris constants, src/velocities.c:307-320
   double t, s, esc[3];
   float tf, sf, escf[3];
@@ -204,7 +229,7 @@ struct PartK {
   uint32_t key0, key1, step;
   // fixed-point scales of the deposit: density 2^Sn, flux 2^Sf (Sf = Sn - e_v
   // for the velocity bound 2^e_v), and the bound itself
-  double fixn64, fixf64;
+  FixScale64 fixn64, fixf64;
   FixScale32 fixn32;  // density: two words
   FixWord32 fixf32;   // flux: one word
   double vmax;
@@ -216,12 +241,12 @@ struct PartK {
 // ---- deposit ---------------------------------------------------------------
 // Linear node index of corner b (xb = b&1, yb = b>>1&1, zb = b>>2) of cell
 // (i,j,k), or -1 when it falls outside a non-periodic dimension.
-__device__ __forceinline__ long long corner_node(const PartK &k, int i, int j, int kk, int b) {
+__device__ __forceinline__ int corner_node(const PartK &k, int i, int j, int kk, int b) {
   int ii = i + (b & 1), jj = j + ((b >> 1) & 1), zz = kk + (b >> 2);
   if (ii >= k.Nx) { if (k.bc[0]) return -1; ii -= k.Nx; }
   if (jj >= k.Ny) { if (k.bc[1]) return -1; jj -= k.Ny; }
   if (zz >= k.Nz) { if (k.bc[2]) return -1; zz -= k.Nz; }
-  return ((long long)zz * k.Ny + jj) * k.Nx + ii;
+  return (zz * k.Ny + jj) * k.Nx + ii;  // at most 2^30 nodes
 }
 
 // Deposit one particle's CIC contributions (src/moments.c:162-205): weights
@@ -236,14 +261,19 @@ __device__ __forceinline__ long long corner_node(const PartK &k, int i, int j, i
 // one atomic for that node and field.  Any mix of cells in a warp is handled;
 // cell-sorted ions give few groups and so few atomics.  `tile` is this warp's
 // 32 x 33 int64 scratch (padded against bank conflicts).  All lanes of the
-// warp must call this together.
+// warp must call this together.  The nodes of every lane's corners go through
+// the tile too (8 x 33 int32 after the values), so that a group costs a few
+// loads and one atomic.
 constexpr int kTileStride = 33;
+constexpr size_t kTileBytes = 32 * kTileStride * sizeof(long long) + 8 * kTileStride * sizeof(int);
 
 template <typename T, typename FixN, typename FixF>
-__device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, long long *tile, const PartK &k,
+__device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsigned char *tile_mem, const PartK &k,
                                              bool active, int i, int j, int kk, T wxh, T wyh,
                                              T wzh, T v0, T v1, T v2, const FixN &fn, const FixF &ff) {
   const int lane = threadIdx.x & 31;
+  long long *tile = reinterpret_cast<long long *>(tile_mem);
+  int *nodes = reinterpret_cast<int *>(tile + 32 * kTileStride);
   const T wxl = T(1) - wxh, wyl = T(1) - wyh, wzl = T(1) - wzh;
   // inactive lanes contribute the zero entry (bias included for FP32)
   const long long zero_n = fn.put(T(0)), zero_f = ff.putvw(T(0), T(0));
@@ -251,6 +281,7 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, long l
   for (int b = 0; b < 8; b++) {
     const T wz = (b & 4) ? wzh : wzl, wy = (b & 2) ? wyh : wyl, wx = (b & 1) ? wxh : wxl;
     const T w = wz * wy * wx;
+    nodes[b * kTileStride + lane] = corner_node(k, i, j, kk, b);
     tile[(b + 0) * kTileStride + lane] = active ? fn.put(w) : zero_n;
     tile[(b + 8) * kTileStride + lane] = active ? ff.putvw(v0, w) : zero_f;
     tile[(b + 16) * kTileStride + lane] = active ? ff.putvw(v1, w) : zero_f;
@@ -264,7 +295,7 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, long l
   if (rem == ECS_FULL_MASK && peers == ECS_FULL_MASK) {
     // the whole warp deposits into one cell: plain 32-term sums
     const long long sum = lane < 8 ? full_sum(row, fn) : full_sum(row, ff);
-    const long long node = corner_node(k, i, j, kk, lane & 7);
+    const int node = nodes[(lane & 7) * kTileStride];
     if (node >= 0 && sum != 0)
       atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
     rem = 0;
@@ -272,12 +303,9 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, long l
   while (rem) {
     const int lead = __ffs(rem) - 1;
     const unsigned grp = __shfl_sync(ECS_FULL_MASK, peers, lead);
-    const int gi = __shfl_sync(ECS_FULL_MASK, i, lead);
-    const int gj = __shfl_sync(ECS_FULL_MASK, j, lead);
-    const int gk = __shfl_sync(ECS_FULL_MASK, kk, lead);
     rem &= ~grp;
     const long long sum = lane < 8 ? group_sum(row, grp, fn) : group_sum(row, grp, ff);
-    const long long node = corner_node(k, gi, gj, gk, lane & 7);
+    const int node = nodes[(lane & 7) * kTileStride + lead];
     if (node >= 0 && sum != 0)
       atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
   }
@@ -528,29 +556,61 @@ __device__ __forceinline__ void gather64(const double4_32a *__restrict__ E, cons
   }
 }
 
-// Fractional grid coordinate and cell index along one axis; positions at
-// exactly the upper bound (possible only when r + L rounds to L in the
-// reference's single wrap) are folded onto the lower bound.
-__device__ __forceinline__ bool cell_coord(double pos, double d, int N, rd &x, int &ix) {
-  x = rd{pos} / rd{d};
-  ix = (int)x.v;
-  if (ix >= N) {
-    x = x - rd{(double)N};
-    ix -= N;
+// pos / d along axis a, correctly rounded.  A power-of-two width (1 in grid
+// units) is an exponent shift; otherwise the quotient from the rounded
+// reciprocal y, corrected by q + (pos - q d) y twice: the first correction
+// makes it faithful, and Markstein's theorem (IBM J. Res. Dev. 34, 1990) makes
+// the second correctly rounded.  Values outside the exponent range in which
+// neither step can lose a bit take the division itself.
+__device__ __forceinline__ double div_axis(const PartK &k, int a, double d, double pos) {
+  const int hi = __double2hiint(pos), e = (hi >> 20) & 0x7ff;
+  if (e < 128 || e > 1920) return order_key(pos) == 0 ? pos : __ddiv_rn(pos, d);
+  if (k.dsh[a] != kNoShift) return __hiloint2double(hi + k.dsh[a] * (1 << 20), __double2loint(pos));
+  const double y = k.dinv[a];
+  const double q0 = __dmul_rn(pos, y);
+  const double q1 = __fma_rn(__fma_rn(-q0, d, pos), y, q0);
+  return __fma_rn(__fma_rn(-q1, d, pos), y, q1);
+}
+
+// Cell index ix and fraction w along one axis; positions at exactly the
+// upper bound (possible only when r + L rounds to L in the reference's single
+// wrap) are folded onto the lower bound.  The whole part is split off the
+// significand; only the (exact) subtraction is FP64 work.
+__device__ __forceinline__ bool cell_coord(const PartK &k, int a, double d, int N, double pos, int &ix, rd &w) {
+  double x = div_axis(k, a, d, pos);
+  const int hi = __double2hiint(x), t = ((hi >> 20) & 0x7ff) - 1023;
+  if (t > 20 || (hi < 0 && order_key(x) != 0)) return false;  // beyond any grid, not a number, or negative
+  double whole = 0.0;
+  ix = 0;
+  if (t >= 0) {
+    const int cut = 20 - t;
+    ix = (int)((((unsigned)hi & 0xfffffu) | 0x100000u) >> cut);
+    whole = __hiloint2double((int)((unsigned)hi & (0xffffffffu << cut)), 0);
   }
-  return ix >= 0 && ix < N && x.v >= 0.0;
+  if (ix >= N) {
+    x = __dsub_rn(x, (double)N);
+    ix -= N;
+    whole = (double)ix;
+    if (ix >= N) return false;
+  }
+  w = rd{x} - rd{whole};
+  return true;
+}
+__device__ __forceinline__ bool cell_coords(const PartK &k, double px, double py, double pz, int &i, int &j, int &kk,
+                                            rd &wx, rd &wy, rd &wz) {
+  return cell_coord(k, 0, k.dx, k.Nx, px, i, wx) & cell_coord(k, 1, k.dy, k.Ny, py, j, wy) &
+         cell_coord(k, 2, k.dz, k.Nz, pz, kk, wz);
 }
 
 __device__ __forceinline__ void push64(const PartK &k, const double4_32a *__restrict__ E, double px,
                                        double py, double pz, double &vx, double &vy, double &vz,
                                        bool &ok) {
-  rd x, y, z;
-  int i, j, kk;
-  ok = cell_coord(px, k.dx, k.Nx, x, i) & cell_coord(py, k.dy, k.Ny, y, j) &
-       cell_coord(pz, k.dz, k.Nz, z, kk);
+  rd wx{0}, wy{0}, wz{0};
+  int i = 0, j = 0, kk = 0;
+  ok = cell_coords(k, px, py, pz, i, j, kk, wx, wy, wz);
   if (!ok) return;
   rd f[3];
-  gather64(E, k, i, j, kk, x - rd{(double)i}, y - rd{(double)j}, z - rd{(double)kk}, f);
+  gather64(E, k, i, j, kk, wx, wy, wz, f);
   rd vxm = rd{vx} + rd{k.esc[0]} * f[0];
   rd vym = rd{vy} + rd{k.esc[1]} * f[1];
   rd vzm = rd{vz} + rd{k.esc[2]} * f[2];
@@ -566,29 +626,27 @@ __device__ __forceinline__ void push64(const PartK &k, const double4_32a *__rest
 // reflecting axes reflect specularly.
 __device__ __forceinline__ void move64(const PartK &k, double &p, double &v, int d) {
   rd r = rd{p} + rd{v} * rd{k.dt};
-  if (k.bc[d] == ECS_BC_PERIODIC) {
-    if (r.v < k.lo[d]) r = r + rd{k.L[d]};
-    if (r.v >= k.hi[d]) r = r - rd{k.L[d]};
-  } else {
-    if (r.v < k.lo[d]) { r = rd{2.0 * k.lo[d]} - r; v = -v; }
-    if (r.v >= k.hi[d]) { r = rd{2.0 * k.hi[d]} - r; v = -v; }
+  if (order_key(r.v) < k.klo[d]) {
+    if (k.bc[d] == ECS_BC_PERIODIC) r = r + rd{k.L[d]};
+    else { r = rd{2.0 * k.lo[d]} - r; v = -v; }
+  }
+  if (order_key(r.v) >= k.khi[d]) {
+    if (k.bc[d] == ECS_BC_PERIODIC) r = r - rd{k.L[d]};
+    else { r = rd{2.0 * k.hi[d]} - r; v = -v; }
   }
   p = r.v;
 }
 
-__device__ __forceinline__ void deposit64(long long *acc, long long *tile, const PartK &k, bool active, double px,
+__device__ __forceinline__ void deposit64(long long *acc, unsigned char *tile, const PartK &k, bool active, double px,
                                           double py, double pz, double vx, double vy, double vz) {
-  rd x{0}, y{0}, z{0};
+  rd wx{0}, wy{0}, wz{0};
   int i = 0, j = 0, kk = 0;
-  bool ok = active;
-  if (active)
-    ok = cell_coord(px, k.dx, k.Nx, x, i) & cell_coord(py, k.dy, k.Ny, y, j) &
-         cell_coord(pz, k.dz, k.Nz, z, kk);
-  double wx = ok ? (x - rd{(double)i}).v : 0.0;
-  double wy = ok ? (y - rd{(double)j}).v : 0.0;
-  double wz = ok ? (z - rd{(double)kk}).v : 0.0;
-  deposit_warp<double>(acc, tile, k, ok, i, j, kk, wx, wy, wz, vx, vy, vz, FixScale64{k.fixn64},
-                       FixScale64{k.fixf64});
+  const bool ok = active && cell_coords(k, px, py, pz, i, j, kk, wx, wy, wz);
+  if (!ok) {
+    i = j = kk = 0;
+    wx = wy = wz = rd{0.0};
+  }
+  deposit_warp<double>(acc, tile, k, ok, i, j, kk, wx.v, wy.v, wz.v, vx, vy, vz, k.fixn64, k.fixf64);
 }
 
 __device__ __forceinline__ void hash64(double px, double py, double pz, double vx, double vy,
@@ -605,59 +663,103 @@ __device__ __forceinline__ void hash64(double px, double py, double pz, double v
 }
 
 // mode bits: 1 push, 2 collide, 4 move, 8 deposit
-__global__ void __launch_bounds__(kBlock) k_particles64(PartK k, int mode, int64_t np,
-                                                        double *__restrict__ px,
-                                                        double *__restrict__ py,
-                                                        double *__restrict__ pz,
-                                                        double *__restrict__ vxa,
-                                                        double *__restrict__ vya,
-                                                        double *__restrict__ vza,
-                                                        const double4_32a *__restrict__ E,
-                                                        long long *__restrict__ acc,
-                                                        EcsDevStatus *st) {
-  extern __shared__ long long shm_tiles[];
-  long long *tile = shm_tiles + (threadIdx.x >> 5) * 32 * kTileStride;
-  const int64_t lane = threadIdx.x & 31;
+//
+// Bound by the FP64 pipe (1/64 of the FP32 rate): what the reference's
+// arithmetic does not need in FP64 (divisions by the cell width, comparisons,
+// conversions, fixed-point rounding) runs on the integer units, and ions that
+// collide are put aside in a queue of their warp (their number, velocity after
+// the push) until 32 of them fill it, instead of holding the other lanes: the
+// FP64 logarithms, square roots and sines of one attempt otherwise cost every
+// second warp as much as its pushes.  64^3, 64 ions a cell, step with
+// collisions: 17.2 -> 6.8 ms.
+constexpr int kQueue = 64;  // entries a warp: fewer than 32 left over, and 32 more
+constexpr size_t kQueueBytes = kQueue * (3 * sizeof(double) + sizeof(int));
+__global__ void __launch_bounds__(kBlock, 2) k_particles64(PartK k, int mode, int64_t np,
+                                                           double *__restrict__ px,
+                                                           double *__restrict__ py,
+                                                           double *__restrict__ pz,
+                                                           double *__restrict__ vxa,
+                                                           double *__restrict__ vya,
+                                                           double *__restrict__ vza,
+                                                           const double4_32a *__restrict__ E,
+                                                           long long *__restrict__ acc,
+                                                           EcsDevStatus *st) {
+  extern __shared__ __align__(16) unsigned char shm_tiles[];
+  unsigned char *mine = shm_tiles + (threadIdx.x >> 5) * (kTileBytes + kQueueBytes);
+  double *qv = reinterpret_cast<double *>(mine + kTileBytes);  // [3][kQueue]
+  int *qip = reinterpret_cast<int *>(qv + 3 * kQueue);
+  const int lane = threadIdx.x & 31;
+  const bool collide = (mode & 2) && k.collide;
+  unsigned int nacc = 0, nref = 0;
+  int queued = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < np;
-       base += stride) {
-    const int64_t ip = base + lane;
-    const bool active = ip < np;
+  int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+  for (;;) {
+    int64_t ip;
+    bool active;
     double x = 0, y = 0, z = 0, vx = 0, vy = 0, vz = 0;
-    if (active) {
-      x = px[ip]; y = py[ip]; z = pz[ip];
-      vx = vxa[ip]; vy = vya[ip]; vz = vza[ip];
-    }
-    bool ok = true;
-    if ((mode & 1) && active) {
-      push64(k, E, x, y, z, vx, vy, vz, ok);
-      if (!ok) atomicOr(&st->flags, ECS_FLAG_RANGE);
-    }
-    unsigned int nacc = 0, nref = 0;
-    if ((mode & 2) && k.collide) {
+    if (queued >= 32 || (base >= np && queued > 0)) {  // a warp of colliding ions
+      const int n = min(queued, 32), at = queued - n + lane;
+      queued -= n;
+      active = lane < n;
+      ip = active ? qip[at] : 0;
       if (active) {
+        x = px[ip]; y = py[ip]; z = pz[ip];
+        vx = qv[at]; vy = qv[kQueue + at]; vz = qv[2 * kQueue + at];
         uint32_t h0, h1;
         hash64(x, y, z, vx, vy, vz, h0, h1);
-        collide_ion<double>(k, h0, h1, h1, vx, vy, vz, nacc, nref);
+        collide_attempts<double>(k, h0, h1, gate_uniform(k, h1), vx, vy, vz, nacc, nref);
       }
-      flush_counts(st, nacc, nref);
+      __syncwarp();
+    } else if (base < np) {
+      ip = base + lane;
+      base += stride;
+      active = ip < np;
+      if (active) {
+        x = px[ip]; y = py[ip]; z = pz[ip];
+        vx = vxa[ip]; vy = vya[ip]; vz = vza[ip];
+      }
+      bool ok = true;
+      if ((mode & 1) && active) {
+        push64(k, E, x, y, z, vx, vy, vz, ok);
+        if (!ok) atomicOr(&st->flags, ECS_FLAG_RANGE);
+      }
+      if (collide) {
+        uint32_t h0, h1;
+        hash64(x, y, z, vx, vy, vz, h0, h1);
+        const bool open = active && gate_open(k, gate_uniform(k, h1));
+        const unsigned m = __ballot_sync(ECS_FULL_MASK, open);
+        if (open) {
+          const int at = queued + __popc(m & ((1u << lane) - 1u));
+          qip[at] = (int)ip;
+          qv[at] = vx;
+          qv[kQueue + at] = vy;
+          qv[2 * kQueue + at] = vz;
+          active = false;
+        }
+        queued += __popc(m);
+        __syncwarp();
+      }
+    } else {
+      break;
     }
     if ((mode & 4) && active) {
       move64(k, x, vx, 0);
       move64(k, y, vy, 1);
       move64(k, z, vz, 2);
     }
-    if (active && !(isfinite(vx) && isfinite(vy) && isfinite(vz))) atomicOr(&st->flags, ECS_FLAG_NONFINITE);
+    if (active && !(finite64(vx) && finite64(vy) && finite64(vz))) atomicOr(&st->flags, ECS_FLAG_NONFINITE);
     if (mode & 8) {
-      if (active && !(fabs(vx) <= k.vmax && fabs(vy) <= k.vmax && fabs(vz) <= k.vmax))
+      if (active && (order_key(fabs(vx)) > k.kvmax || order_key(fabs(vy)) > k.kvmax || order_key(fabs(vz)) > k.kvmax))
         atomicOr(&st->flags, ECS_FLAG_RANGE);
-      deposit64(acc, tile, k, active, x, y, z, vx, vy, vz);
+      deposit64(acc, mine, k, active, x, y, z, vx, vy, vz);
     }
     if (active) {
       if (mode & 4) { px[ip] = x; py[ip] = y; pz[ip] = z; }
       if (mode & 7) { vxa[ip] = vx; vya[ip] = vy; vza[ip] = vz; }
     }
   }
+  if (collide) flush_counts(st, nacc, nref);
 }
 
 // ==========================================================================
@@ -917,8 +1019,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_particles32(PartK k, int mode, in
                                                          long long *__restrict__ acc,
                                                          int32_t *__restrict__ count, int32_t *__restrict__ keys,
                                                          EcsDevStatus *st) {
-  extern __shared__ long long shm_tiles[];
-  long long *tile = shm_tiles + (threadIdx.x >> 5) * 32 * kTileStride;
+  extern __shared__ __align__(16) unsigned char shm_tiles[];
+  unsigned char *tile = shm_tiles + (threadIdx.x >> 5) * kTileBytes;
   const int64_t lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < np;
@@ -1015,7 +1117,7 @@ __device__ __forceinline__ void tile_finish(const PartK &k, int mode, EcsDevStat
     } else {  // outside the window, or fast: straight into the global accumulators
 #pragma unroll 1
       for (int bc = 0; bc < 8; bc++) {
-        const long long gnode = corner_node(k, q.i, q.j, q.kk, bc);
+        const int gnode = corner_node(k, q.i, q.j, q.kk, bc);
         if (gnode < 0) continue;
         const float w = (((bc & 4) ? wzh : wzl) * ((bc & 2) ? wyh : wyl)) * ((bc & 1) ? wxh : wxl);
         int hi, lo;
@@ -1415,6 +1517,11 @@ __global__ void k_estimate32(PartK k, int64_t np, const float4 *__restrict__ ion
 }
 
 // ---- host helpers -----------------------------------------------------------------
+long long host_key(double v) {
+  long long b;
+  memcpy(&b, &v, sizeof b);
+  return order_key(b);
+}
 PartK make_k(const EcsCtx *ctx, double dt) {
   const EcsParams &p = ctx->p;
   PartK k;
@@ -1427,6 +1534,14 @@ PartK make_k(const EcsCtx *ctx, double dt) {
   k.lo[0] = p.x0; k.lo[1] = p.y0; k.lo[2] = p.z0;
   k.hi[0] = p.x1; k.hi[1] = p.y1; k.hi[2] = p.z1;
   k.L[0] = p.Lx; k.L[1] = p.Ly; k.L[2] = p.Lz;
+  const double width[3] = {p.dx, p.dy, p.dz};
+  for (int d = 0; d < 3; d++) {
+    k.dinv[d] = 1.0 / width[d];
+    int e = 0;
+    k.dsh[d] = frexp(width[d], &e) == 0.5 && e >= -62 && e <= 64 ? 1 - e : kNoShift;
+    k.klo[d] = host_key(k.lo[d]);
+    k.khi[d] = host_key(k.hi[d]);
+  }
   // src/velocities.c:307-320, same operation order
   double tscale = 0.5 * (p.qi / p.mi) * dt;
   k.t = tscale * p.B0;
@@ -1466,13 +1581,14 @@ PartK make_k(const EcsCtx *ctx, double dt) {
     m ^= m >> 16; m *= 0x7feb352du; m ^= m >> 15; m *= 0x846ca68bu; m ^= m >> 16;
     k.stepmix = m ^ k.key1;
   }
-  k.fixn64 = ldexp(1.0, ctx->shift_n);
-  k.fixf64 = ldexp(1.0, ctx->shift_f);
+  k.fixn64 = {ldexp(1.0, ctx->shift_n), 1075 - ctx->shift_n};
+  k.fixf64 = {ldexp(1.0, ctx->shift_f), 1075 - ctx->shift_f};
   k.fixn32 = {ldexpf(1.0f, ctx->shift_n), ldexpf(1.0f, ctx->shift_n - kFixSplit), -ldexpf(1.0f, kFixSplit - ctx->shift_n)};
   k.fixf32 = {ldexpf(1.0f, ctx->shift_f)};
   // the velocity bound 2^e_v behind the flux scale (ecs_fix_shifts)
   k.vmax = ldexp(1.0, (ctx->prec == ECS_PREC_FP64 ? ECS_FIX_SHIFT_FP64 : ECS_FIX_SHIFT_MIXED_FLUX) - ctx->shift_f);
   k.vmaxf = (float)k.vmax;
+  k.kvmax = host_key(k.vmax);
   k.vwinf = (float)(k.vmax / 8.0);
   k.tg = {ctx->ntile[0], ctx->ntile[1], ctx->ntile[2]};
   return k;
@@ -1939,10 +2055,11 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
   int rc = pass_params(ctx, dt, mode, k);
   if (rc) return rc;
   ctx->pgen++;
-  const size_t shm = (size_t)(kBlock / 32) * 32 * kTileStride * sizeof(long long);
+  const size_t shm = (size_t)(kBlock / 32) * kTileBytes;
+  const size_t shm64 = (size_t)(kBlock / 32) * (kTileBytes + kQueueBytes);
   static std::atomic<bool> attr_set{false};
   if (!attr_set) {
-    cudaFuncSetAttribute(k_particles64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
+    cudaFuncSetAttribute(k_particles64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm64);
     cudaFuncSetAttribute(k_particles32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
     attr_set = true;
   }
@@ -1954,7 +2071,8 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
   unsigned int g = grid_blocks(ctx, ctx->np, 3);
   if (ctx->ev[0]) cudaEventRecord(ctx->ev[0], ctx->stream);
   if (ctx->prec == ECS_PREC_FP64) {
-    k_particles64<<<g, kBlock, shm, ctx->stream>>>(k, mode, ctx->np, ctx->px, ctx->py, ctx->pz, ctx->vx,
+    g = grid_blocks(ctx, ctx->np, 2);  // the blocks that fit the SMs at once
+    k_particles64<<<g, kBlock, shm64, ctx->stream>>>(k, mode, ctx->np, ctx->px, ctx->py, ctx->pz, ctx->vx,
                                                 ctx->vy, ctx->vz, ctx->eext64, ctx->acc, ctx->dstat);
   } else if (ctx->tiles_valid) {
     // after an index sort the pass reads the records through the permutation
