@@ -71,21 +71,57 @@ constexpr int kNoShift = 1 << 20;
 // and the conversion of one value held the pipe as long as a hundred integer
 // instructions do the issue slots.
 struct FixScale64 {
-  double s;  // 2^S
-  int top;   // 1075 - S: a significand's right shift is top - (exponent field)
-  __device__ __forceinline__ long long put(double v) const {
-    const int hi = __double2hiint(v), sh0 = top - ((hi >> 20) & 0x7ff);
-    if (sh0 < 1) return __double2ll_rn(v * s);  // beyond every value that a deposit accepts
-    const int sh = min(sh0, 63);                // 63: rounds to 0 (zero and subnormal values too)
-    const unsigned long long m =
-        ((unsigned long long)(((unsigned)hi & 0xfffffu) | 0x100000u) << 32) | (unsigned)__double2loint(v);
+  int top;  // 1075 - S: a significand's right shift is top - (exponent field)
+  // m 2^(e - 1075 + S) rounded, for a 53-bit significand m and e <= top - 1
+  __device__ __forceinline__ long long round(unsigned mh, unsigned ml, int e) const {
+    const int sh = min(top - e, 63);  // 63: rounds to 0 (zero and subnormal values too)
+    const unsigned long long m = ((unsigned long long)mh << 32) | ml;
     const unsigned long long q = m >> sh;
-    const unsigned long long r = (m + ((1ull << (sh - 1)) - 1ull + (q & 1ull))) >> sh;
-    return hi < 0 ? -(long long)r : (long long)r;
+    return (long long)((m + ((1ull << (sh - 1)) - 1ull + (q & 1ull))) >> sh);
   }
-  // flux contribution v w
-  __device__ __forceinline__ long long putvw(double v, double w) const { return put(v * w); }
 };
+
+// FP64 products on the integer units: the significand shifted to the top of
+// 64 bits, and the exponent field.  A product is four 32 x 32-bit multiply-adds
+// and a rounding, about 22 instructions where a multiplication holds the FP64
+// pipe for 64 issue slots of its scheduler; the same bits (round to nearest,
+// ties to even).
+struct Sig {
+  unsigned h, l;
+  int e;
+};
+// Zero and subnormal values become 0 (callers that need more test e first).
+__device__ __forceinline__ Sig sig_of(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const int e = (int)((hi >> 20) & 0x7ffu);
+  return {e ? __funnelshift_l(lo, hi, 11) | 0x80000000u : 0u, e ? lo << 11 : 0u, e};
+}
+// a b rounded to 53 bits: significand qh:ql (2^53 when the rounding carried
+// over) with exponent field e.
+__device__ __forceinline__ void sig_mul(const Sig &a, const Sig &b, unsigned &qh, unsigned &ql, int &e) {
+  const unsigned long long p = (unsigned long long)a.l * b.l;
+  const unsigned long long m1 = (unsigned long long)a.l * b.h + (p >> 32);
+  const unsigned long long m2 = (unsigned long long)a.h * b.l + (unsigned)m1;
+  const unsigned long long top = (unsigned long long)a.h * b.h + (m1 >> 32) + (m2 >> 32);
+  const unsigned t1 = (unsigned)(top >> 32), t0 = (unsigned)top, lo = (unsigned)m2;
+  const int n = (int)(~t1 >> 31);  // 1: the product's top bit is clear
+  const unsigned h = __funnelshift_l(t0, t1, n), l = __funnelshift_l(lo, t0, n);
+  const unsigned rest = (lo << n) | (unsigned)p;
+  e = a.e + b.e - 1022 - n;
+  const unsigned up = ((l & 0x7ffu) | (rest != 0u)) + ((l >> 11) & 1u) > 0x400u;
+  const unsigned long long q = ((((unsigned long long)h << 32) | l) >> 11) + up;
+  qh = (unsigned)(q >> 32);
+  ql = (unsigned)q;
+}
+// The rounded product as a factor again.
+__device__ __forceinline__ Sig sig_product(const Sig &a, const Sig &b) {
+  unsigned qh, ql;
+  int e;
+  sig_mul(a, b, qh, ql, e);
+  const unsigned c = qh >> 21;  // 2^53: the low bits are 0
+  qh >>= c;
+  return {__funnelshift_l(ql, qh, 11), ql << 11, e + (int)c};
+}
 
 // FP32: the same integer, rint(v 2^S) with |v 2^S| <= 2^38 (S = 38 on the
 // mixed path), from FP32 adds and multiply-adds only (on sm_103 a
@@ -147,6 +183,14 @@ struct FixWord32 {
   __device__ __forceinline__ long long putvw(float v, float w) const { return (long long)biased(v * s, w); }
 };
 
+// One tile entry's value.
+__device__ __forceinline__ long long entry_value(long long e, const FixScale64 &) { return e; }
+__device__ __forceinline__ long long entry_value(long long e, const FixScale32 &) {
+  return fix_unbias((unsigned)e, (unsigned)((unsigned long long)e >> 32), 1);
+}
+__device__ __forceinline__ long long entry_value(long long e, const FixWord32 &) {
+  return (long long)(int)((unsigned)e - kFixBiasBits);
+}
 // Exact sum of the tile entries q in `m` (bit mask of lanes).
 __device__ __forceinline__ long long group_sum(const long long *row, unsigned m, const FixScale64 &) {
   long long sum = 0;
@@ -275,17 +319,52 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
   long long *tile = reinterpret_cast<long long *>(tile_mem);
   int *nodes = reinterpret_cast<int *>(tile + 32 * kTileStride);
   const T wxl = T(1) - wxh, wyl = T(1) - wyh, wzl = T(1) - wzh;
-  // inactive lanes contribute the zero entry (bias included for FP32)
-  const long long zero_n = fn.put(T(0)), zero_f = ff.putvw(T(0), T(0));
 #pragma unroll
-  for (int b = 0; b < 8; b++) {
-    const T wz = (b & 4) ? wzh : wzl, wy = (b & 2) ? wyh : wyl, wx = (b & 1) ? wxh : wxl;
-    const T w = wz * wy * wx;
-    nodes[b * kTileStride + lane] = corner_node(k, i, j, kk, b);
-    tile[(b + 0) * kTileStride + lane] = active ? fn.put(w) : zero_n;
-    tile[(b + 8) * kTileStride + lane] = active ? ff.putvw(v0, w) : zero_f;
-    tile[(b + 16) * kTileStride + lane] = active ? ff.putvw(v1, w) : zero_f;
-    tile[(b + 24) * kTileStride + lane] = active ? ff.putvw(v2, w) : zero_f;
+  for (int b = 0; b < 8; b++) nodes[b * kTileStride + lane] = corner_node(k, i, j, kk, b);
+  if constexpr (sizeof(T) == 8) {
+    // The weights are at most 1, and the velocity within the bound that the
+    // flux scale is made for, or the call fails: past it the flux is 0.
+    // Inactive lanes have zero weights.  Rolled: unrolled, the pass outgrows
+    // the instruction cache.
+    const Sig sx[2] = {sig_of(wxl), sig_of(wxh)}, sy[2] = {sig_of(wyl), sig_of(wyh)}, sz[2] = {sig_of(wzl), sig_of(wzh)};
+    const T v[3] = {v0, v1, v2};
+    Sig sv[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      sv[d] = sig_of(v[d]);
+      if (sv[d].e > ff.top - 4) sv[d] = Sig{0u, 0u, 0};
+    }
+#pragma unroll 1
+    for (int zy = 0; zy < 4; zy++) {
+      const Sig a = zy & 2 ? sz[1] : sz[0], c = zy & 1 ? sy[1] : sy[0];
+      const Sig wzy = sig_product(a, c);
+#pragma unroll
+      for (int bx = 0; bx < 2; bx++) {
+        const int b = zy * 2 + bx;
+        const Sig w = sig_product(wzy, sx[bx]);
+        tile[b * kTileStride + lane] = active ? fn.round(w.h >> 11, __funnelshift_r(w.l, w.h, 11), w.e) : 0;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+          unsigned qh, ql;
+          int e;
+          sig_mul(sv[d], w, qh, ql, e);
+          const long long r = ff.round(qh, ql, e);
+          tile[(b + 8 + 8 * d) * kTileStride + lane] = !active ? 0 : (__double2hiint(v[d]) < 0 ? -r : r);
+        }
+      }
+    }
+  } else {
+    // inactive lanes contribute the zero entry (its bias included)
+    const long long zero_n = fn.put(T(0)), zero_f = ff.putvw(T(0), T(0));
+#pragma unroll
+    for (int b = 0; b < 8; b++) {
+      const T wz = (b & 4) ? wzh : wzl, wy = (b & 2) ? wyh : wyl, wx = (b & 1) ? wxh : wxl;
+      const T w = wz * wy * wx;
+      tile[(b + 0) * kTileStride + lane] = active ? fn.put(w) : zero_n;
+      tile[(b + 8) * kTileStride + lane] = active ? ff.putvw(v0, w) : zero_f;
+      tile[(b + 16) * kTileStride + lane] = active ? ff.putvw(v1, w) : zero_f;
+      tile[(b + 24) * kTileStride + lane] = active ? ff.putvw(v2, w) : zero_f;
+    }
   }
   const int key = active ? (i | (j << 10) | (kk << 20)) : -1;
   const unsigned peers = __match_any_sync(ECS_FULL_MASK, key);
@@ -298,6 +377,18 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
     const int node = nodes[(lane & 7) * kTileStride];
     if (node >= 0 && sum != 0)
       atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
+    rem = 0;
+  } else if (__all_sync(ECS_FULL_MASK, !active || (peers & (peers - 1u)) == 0u)) {
+    // no two ions in one cell (any order but a sorted one): lane l issues slot
+    // l of one ion after the other, a few independent loads and an atomic each
+#pragma unroll 4
+    for (int q = 0; q < 32; q++) {
+      const long long e = row[q];
+      const long long sum = lane < 8 ? entry_value(e, fn) : entry_value(e, ff);
+      const int node = nodes[(lane & 7) * kTileStride + q];
+      if (node >= 0 && sum != 0)
+        atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
+    }
     rem = 0;
   }
   while (rem) {
@@ -522,7 +613,7 @@ __device__ __forceinline__ void flush_samples(EcsDevStatus *st, float sample, bo
 // Difference numerators at the 8 corners, interpolated with the reference's
 // weight order (src/vector-math.c:645-651): along y with wyh, across the z
 // pair with wxh, across the x pair with wzh.  In 2-D the four corners of the
-// z = 0 plane, along y with wyh, across x with wxh.
+// z = 0 plane, along y with wyh, across x with wxh.  The weights are in [0, 1).
 __device__ __forceinline__ void gather64(const double4_32a *__restrict__ E, const PartK &k, int i,
                                          int j, int kk, rd wx, rd wy, rd wz, rd f[3]) {
   const size_t sx = (size_t)k.Nx + 1, sxy = sx * ((size_t)k.Ny + 1);
@@ -664,17 +755,20 @@ __device__ __forceinline__ void hash64(double px, double py, double pz, double v
 
 // mode bits: 1 push, 2 collide, 4 move, 8 deposit
 //
-// Bound by the FP64 pipe (1/64 of the FP32 rate): what the reference's
-// arithmetic does not need in FP64 (divisions by the cell width, comparisons,
-// conversions, fixed-point rounding) runs on the integer units, and ions that
-// collide are put aside in a queue of their warp (their number, velocity after
-// the push) until 32 of them fill it, instead of holding the other lanes: the
-// FP64 logarithms, square roots and sines of one attempt otherwise cost every
-// second warp as much as its pushes.  64^3, 64 ions a cell, step with
-// collisions: 17.2 -> 6.8 ms.
+// Bound by the FP64 pipe (1/64 of the FP32 rate), which it keeps two thirds
+// busy, and by instruction fetch: what the reference's arithmetic does not need
+// in FP64 (divisions by the cell width, comparisons, conversions, the deposit's
+// products and rounding) runs on the integer units, and ions that collide are
+// put aside in a queue of their warp (their number, velocity after the push)
+// until 32 of them fill it, instead of holding the other lanes: the FP64
+// logarithms, square roots and sines of one attempt otherwise cost every second
+// warp as much as its pushes.  Per warp of ions 384 -> 124 FP64 instructions;
+// 64^3, 64 ions a cell, step with collisions: 17.2 -> 4.8 ms.  The gather's
+// products on the integer units too (104 FP64 instructions) took 5 % longer.
 constexpr int kQueue = 64;  // entries a warp: fewer than 32 left over, and 32 more
 constexpr size_t kQueueBytes = kQueue * (3 * sizeof(double) + sizeof(int));
-__global__ void __launch_bounds__(kBlock, 2) k_particles64(PartK k, int mode, int64_t np,
+constexpr int kBlock64 = 192, kBlocks64 = 3;  // 18 warps an SM: 96 registers, 68 KB of shared memory a block
+__global__ void __launch_bounds__(kBlock64, kBlocks64) k_particles64(PartK k, int mode, int64_t np,
                                                            double *__restrict__ px,
                                                            double *__restrict__ py,
                                                            double *__restrict__ pz,
@@ -1581,8 +1675,8 @@ PartK make_k(const EcsCtx *ctx, double dt) {
     m ^= m >> 16; m *= 0x7feb352du; m ^= m >> 15; m *= 0x846ca68bu; m ^= m >> 16;
     k.stepmix = m ^ k.key1;
   }
-  k.fixn64 = {ldexp(1.0, ctx->shift_n), 1075 - ctx->shift_n};
-  k.fixf64 = {ldexp(1.0, ctx->shift_f), 1075 - ctx->shift_f};
+  k.fixn64 = {1075 - ctx->shift_n};
+  k.fixf64 = {1075 - ctx->shift_f};
   k.fixn32 = {ldexpf(1.0f, ctx->shift_n), ldexpf(1.0f, ctx->shift_n - kFixSplit), -ldexpf(1.0f, kFixSplit - ctx->shift_n)};
   k.fixf32 = {ldexpf(1.0f, ctx->shift_f)};
   // the velocity bound 2^e_v behind the flux scale (ecs_fix_shifts)
@@ -2056,7 +2150,7 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
   if (rc) return rc;
   ctx->pgen++;
   const size_t shm = (size_t)(kBlock / 32) * kTileBytes;
-  const size_t shm64 = (size_t)(kBlock / 32) * (kTileBytes + kQueueBytes);
+  const size_t shm64 = (size_t)(kBlock64 / 32) * (kTileBytes + kQueueBytes);
   static std::atomic<bool> attr_set{false};
   if (!attr_set) {
     cudaFuncSetAttribute(k_particles64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm64);
@@ -2071,8 +2165,9 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
   unsigned int g = grid_blocks(ctx, ctx->np, 3);
   if (ctx->ev[0]) cudaEventRecord(ctx->ev[0], ctx->stream);
   if (ctx->prec == ECS_PREC_FP64) {
-    g = grid_blocks(ctx, ctx->np, 2);  // the blocks that fit the SMs at once
-    k_particles64<<<g, kBlock, shm64, ctx->stream>>>(k, mode, ctx->np, ctx->px, ctx->py, ctx->pz, ctx->vx,
+    // the blocks that fit the SMs at once
+    g = (unsigned)std::min<int64_t>((ctx->np + kBlock64 - 1) / kBlock64, (int64_t)ctx->nsm * kBlocks64);
+    k_particles64<<<g, kBlock64, shm64, ctx->stream>>>(k, mode, ctx->np, ctx->px, ctx->py, ctx->pz, ctx->vx,
                                                 ctx->vy, ctx->vz, ctx->eext64, ctx->acc, ctx->dstat);
   } else if (ctx->tiles_valid) {
     // after an index sort the pass reads the records through the permutation
