@@ -124,6 +124,8 @@ int64_t ecs_ctx_device_bytes(const EcsParams *p, int precision, int64_t cap) {
   // finest; the coarsest level's inverse (<= 128 cells)
   b += (n * (precision == ECS_PREC_FP64 || p->Nz > 128 ? 11 : 7) + n / 4) * t * 8 / 7 + 128 * 128 * t;
   if (precision == ECS_PREC_FP64) {
+    // FP64 row coefficients of the coarser levels (every plane kept: a third of the finest's)
+    if (p->lhs_type != ECS_LHS_IDENTITY) b += n * 8 * 11 * (p->bc[2] == ECS_BC_PERIODIC && p->ndim == 3 ? 1 : 3) / 7;
     b += (2 * m + 1) * n * 8;  // Krylov bases V, Z
     b += cap * 48 + ne * 32;   // ions (6 FP64), E numerators
   } else {

@@ -56,6 +56,7 @@ struct MgLevel {
   T *b = nullptr;      // right-hand side on this level
   T *r = nullptr;      // residual / scratch
   T *t = nullptr;      // smoother scratch
+  T *coef = nullptr;   // FP64: the 11 row coefficients a cell (SoA)
   // z-line factorisation of the (lower, diag, upper) z-tridiagonal part,
   // cyclic closure by Sherman-Morrison (periodic z) or plain (reflecting z).
   T *zl_minv = nullptr, *zl_q = nullptr;

@@ -62,16 +62,31 @@ struct KrylovDev {
 };
 
 // ---- operator ------------------------------------------------------------------
+// A row's 11 coefficients: in FP64 from the arrays of k_coef64 (coef[e * n +
+// c]), where there are any, since forming them takes 39 of the row's 50 FP64
+// operations and FP64 is the scarce resource here (64^3 operator: 25 -> 10 us);
+// in FP32 always from the density, which is 7 words instead of 11.
+template <typename T>
+__device__ __forceinline__ void row_coef(const OpK &o, const T *__restrict__ n, const T *__restrict__ coef,
+                                         const Nbr &q, T v[11]) {
+  if (sizeof(T) == 8 && coef) {
+#pragma unroll
+    for (int e = 0; e < 11; e++) v[e] = __ldg(&coef[(size_t)e * o.g.n + q.c]);
+  } else {
+    row11_n(n, o, q, v);
+  }
+}
+
 // y = A x   (mode 0)     or     y = b - A x   (mode 1)
 template <typename T>
-__global__ void k_apply(OpK o, const T *__restrict__ n, const T *__restrict__ x, const T *__restrict__ b,
-                        T *__restrict__ y, int mode) {
+__global__ void k_apply(OpK o, const T *__restrict__ n, const T *__restrict__ coef, const T *__restrict__ x,
+                        const T *__restrict__ b, T *__restrict__ y, int mode) {
   ECS_PDL_ENTRY();
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const Nbr q = nbr_of(o.g, i, j, k);
   T v[11], xe[11];
-  row11_n(n, o, q, v);
+  row_coef(o, n, coef, q, v);
   row_x(x, q, xe);
   T s = T(0);
 #pragma unroll
@@ -251,14 +266,14 @@ __global__ void k_zline_setup(GridG g, ZCoup<T> zc, const T *__restrict__ n, con
 
 // Right-hand side of the z-line systems: r = b - A_xy xo.
 template <typename T>
-__global__ void k_zline_rhs(OpK o, const T *__restrict__ n, const T *__restrict__ b, const T *__restrict__ xo,
-                            T *__restrict__ r) {
+__global__ void k_zline_rhs(OpK o, const T *__restrict__ n, const T *__restrict__ coef, const T *__restrict__ b,
+                            const T *__restrict__ xo, T *__restrict__ r) {
   ECS_PDL_ENTRY();
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const Nbr q = nbr_of(o.g, i, j, k);
   T v[11], xe[11];
-  row11_n(n, o, q, v);
+  row_coef(o, n, coef, q, v);
   row_x(xo, q, xe);
   T s = b[q.c];
 #pragma unroll
@@ -1562,8 +1577,9 @@ __global__ void k_orth2_scale(size_t n, T *__restrict__ V, KrylovDev *kd, T *__r
 // at every stencil point on the fly, with the rounding of the stored value;
 // a mean is removed only on fully periodic grids, which have no ghosts.
 template <typename T>
-__global__ void k_apply_dyn(OpK o, const T *__restrict__ n, const T *__restrict__ x, const double *__restrict__ mean,
-                            T *__restrict__ Z, T *__restrict__ V, const KrylovDev *__restrict__ kd) {
+__global__ void k_apply_dyn(OpK o, const T *__restrict__ n, const T *__restrict__ coef, const T *__restrict__ x,
+                            const double *__restrict__ mean, T *__restrict__ Z, T *__restrict__ V,
+                            const KrylovDev *__restrict__ kd) {
   ECS_PDL_ENTRY();
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
@@ -1572,7 +1588,7 @@ __global__ void k_apply_dyn(OpK o, const T *__restrict__ n, const T *__restrict_
   const Nbr q = nbr_of(o.g, i, j, k);
   const unsigned c = q.c;
   T v[11], xe[11];
-  row11_n(n, o, q, v);
+  row_coef(o, n, coef, q, v);
   row_x(x, q, xe);
   T s = T(0);
 #pragma unroll
@@ -1852,6 +1868,10 @@ int mg_alloc(EcsCtx *ctx) {
     L.hx = hx; L.hy = hy; L.hz = hz;
     T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_minv, &L.zl_q};
     for (auto a : arr) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
+    if constexpr (sizeof(T) == 8) {
+      if (mg.lv.empty()) L.coef = ctx->coef64;
+      else ECS_CUDA(ctx, cudaMalloc((void **)&L.coef, 11 * L.n * sizeof(T)));
+    }
     if (zl_stored<T>(seg_len<T>(nz))) {
       T **more[] = {&L.zl_a, &L.zl_cp, &L.zl_fb, &L.zl_bb};
       for (auto a : more) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
@@ -1930,18 +1950,6 @@ int ensure_setup_streams(EcsCtx *ctx) {
   return ECS_OK;
 }
 
-// z-line rows and factors of level L on stream s.
-template <typename T>
-int zline_factor(EcsCtx *ctx, MgLevel<T> &L, cudaStream_t s) {
-  const int ncol = L.nx * L.ny;
-  const OpK o = op_level(ctx, L);
-  ecs_launch_pdl(k_zline_rows<T>, blocks3(o.g), threads3(), 0, s, o, L.dens, L.r);  // r is free here
-  ECS_LAUNCHED(ctx);
-  ecs_launch_pdl(k_zline_setup<T>, ecs_div_up(ncol, kColBlock), kColBlock, 0, s, o.g, z_coupling<T>(o), L.dens, L.r, zl_of(L), seg_len<T>(L.nz));
-  ECS_LAUNCHED(ctx);
-  return ECS_OK;
-}
-
 // The 11 FP64 row coefficients of every cell, coef[e * n + c] (e in the
 // order of off_i/off_j/off_k), computed once per operator set-up: FP64
 // arithmetic runs at a small fraction of the FP32 rate on this GPU, and the
@@ -1955,6 +1963,24 @@ __global__ void k_coef64(OpK o, const double *__restrict__ n, double *__restrict
   row11_n(n, o, q, v);
 #pragma unroll
   for (int e = 0; e < 11; e++) coef[(size_t)e * o.g.n + q.c] = v[e];
+}
+
+// z-line rows and factors of level L on stream s.
+template <typename T>
+int zline_factor(EcsCtx *ctx, MgLevel<T> &L, cudaStream_t s) {
+  const int ncol = L.nx * L.ny;
+  const OpK o = op_level(ctx, L);
+  if constexpr (sizeof(T) == 8) {
+    if (&L != &mg_of<T>(ctx).lv[0]) {  // the finest level's are computed beside this
+      ecs_launch_pdl(k_coef64, blocks3(o.g), threads3(), 0, s, o, L.dens, L.coef);
+      ECS_LAUNCHED(ctx);
+    }
+  }
+  ecs_launch_pdl(k_zline_rows<T>, blocks3(o.g), threads3(), 0, s, o, L.dens, L.r);  // r is free here
+  ECS_LAUNCHED(ctx);
+  ecs_launch_pdl(k_zline_setup<T>, ecs_div_up(ncol, kColBlock), kColBlock, 0, s, o.g, z_coupling<T>(o), L.dens, L.r, zl_of(L), seg_len<T>(L.nz));
+  ECS_LAUNCHED(ctx);
+  return ECS_OK;
 }
 
 // Operator set-up of the multigrid levels: level densities, z-line factors,
@@ -2021,7 +2047,7 @@ int sweep(EcsCtx *ctx, MgLevel<T> &L, const T *b, const T *xo, T *xn) {
   const OpK o = op_level(ctx, L);
   const T *r = b;
   if (xo) {
-    ecs_launch_pdl(k_zline_rhs<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, b, xo, L.r);
+    ecs_launch_pdl(k_zline_rhs<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, b, xo, L.r);
     ECS_LAUNCHED(ctx);
     r = L.r;
   }
@@ -2157,7 +2183,7 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
   MgLevel<T> &C = mg.lv[l + 1];
   const OpK o = op_level(ctx, L);
   if ((rc = sweep<T>(ctx, L, b, nullptr, L.t))) return rc;
-  ecs_launch_pdl(k_apply<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.t, b, L.r, 1);
+  ecs_launch_pdl(k_apply<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, L.t, b, L.r, 1);
   ECS_LAUNCHED(ctx);
   const GridG gc = grid_level(ctx, C.nx, C.ny, C.nz);
   ecs_launch_pdl(k_restrict<T>, blocks3(gc), threads3(), 0, ctx->stream, o.g, gc, L.r, C.b);
@@ -2229,7 +2255,7 @@ int cycle_step(EcsCtx *ctx, cudaGraphConditionalHandle cond, int use_graph) {
     if ((rc = launch_reduce<T, kRedMean>(ctx, n, L0.x, (double)n, &kd->mean, cond, use_graph))) return rc;
     mean = &kd->mean;
   }
-  ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.x, mean, Z, V, kd);
+  ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.coef, L0.x, mean, Z, V, kd);
   ECS_LAUNCHED(ctx);
   // classical Gram-Schmidt, two passes
   constexpr int W = kPack<T>;
@@ -2330,7 +2356,9 @@ __global__ void k_residual64(OpK o, const double *__restrict__ coef, const doubl
 
 template <typename T>
 void free_mg(Multigrid<T> &mg) {
-  for (auto &L : mg.lv) {
+  for (size_t l = 0; l < mg.lv.size(); l++) {
+    MgLevel<T> &L = mg.lv[l];
+    if (l > 0 && L.coef) cudaFree(L.coef);  // the finest level's are the context's
     T *arr[] = {L.dens, L.x, L.b, L.r, L.t, L.zl_a, L.zl_cp, L.zl_minv, L.zl_q, L.zl_fb, L.zl_bb, L.zl_a0g, L.zl_qden};
     for (T *a : arr)
       if (a) cudaFree(a);
@@ -2843,7 +2871,7 @@ int ecs_operator_apply64(EcsCtx *ctx, const double *x, double *y) {
     ECS_CUDA(ctx, cudaMemcpyAsync(y, x, ctx->ncell * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
     return ECS_OK;
   }
-  ecs_launch_pdl(k_apply<double>, blocks3(o64.g), threads3(), 0, ctx->stream, o64, op_density(ctx), x, nullptr, y, 0);
+  ecs_launch_pdl(k_apply<double>, blocks3(o64.g), threads3(), 0, ctx->stream, o64, op_density(ctx), nullptr, x, nullptr, y, 0);
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
