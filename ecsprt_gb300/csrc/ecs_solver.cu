@@ -94,6 +94,132 @@ __global__ void k_apply(OpK o, const T *__restrict__ n, const T *__restrict__ co
   y[q.c] = mode ? b[q.c] - s : s;
 }
 
+// ---- FP32 rows four cells a thread ----------------------------------------------
+// Four consecutive x cells of one row: their 18 operands a cell overlap, so a
+// thread loads 10 float4 and 8 words for all four instead of 72 words.  The
+// one-cell kernels are bound by those loads on the large levels (128^3:
+// residual 16.8 -> 8.8 us, z-line right-hand side 12.8 -> 6.8, Arnoldi operator
+// 18.6 -> 10.0, prolongation 12.3 -> 4.8, restriction 6.0 -> 4.2); the same
+// operands give the same bits.  For rows that are a multiple of 4 long (16-byte
+// alignment) and levels of at least kRow4Cells cells: below, a quarter of the
+// threads hides latency worse than the loads cost (32^3 solve 0.675 against
+// 0.666 ms; 48^3 0.930 against 0.943 ms).  x and y are periodic on every grid
+// the solver takes; z may have ghosts.
+constexpr size_t kRow4Cells = 1 << 16;
+struct Row4 {
+  float m, p;  // the cells before and after
+  float4 c;
+  // value d cells (-1, 0, 1) from cell e of the four
+  __device__ __forceinline__ float at(int e) const {
+    return e < 0 ? m : (e == 0 ? c.x : (e == 1 ? c.y : (e == 2 ? c.z : (e == 3 ? c.w : p))));
+  }
+};
+struct Cell4 {
+  unsigned c;          // linear index of the first cell
+  int xm, xp;          // offsets of the cells before the first and after the last
+  int ym, yp, zm, zp;  // row and plane offsets
+  bool vzm, vzp;
+};
+__device__ __forceinline__ float4 ld4(const float *__restrict__ f, unsigned c) {
+  return *reinterpret_cast<const float4 *>(f + c);
+}
+__device__ __forceinline__ Row4 row4(const float *__restrict__ f, const Cell4 &q, int off) {
+  const unsigned c = (unsigned)((int)q.c + off);
+  return {f[(unsigned)((int)c + q.xm)], f[(unsigned)((int)c + q.xp)], ld4(f, c)};
+}
+__device__ __forceinline__ float4 plane4(const float *__restrict__ f, const Cell4 &q, int off, bool valid) {
+  return valid ? ld4(f, (unsigned)((int)q.c + off)) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// Block of row quarters: blockDim.x packs along x, blockDim.y rows.
+__device__ __forceinline__ bool at4(const GridG &g, Cell4 &q) {
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) * 4, j = (int)(blockIdx.y * blockDim.y + threadIdx.y),
+            k = (int)blockIdx.z;
+  if (i >= g.nx || j >= g.ny) return false;
+  const Nbr n = nbr_of(g, i, j, k);
+  q.c = n.c;
+  q.xm = n.xm;
+  q.xp = i + 4 < g.nx ? 4 : 4 - g.nx;
+  q.ym = n.ym; q.yp = n.yp; q.zm = n.zm; q.zp = n.zp;
+  q.vzm = n.vzm; q.vzp = n.vzp;
+  return true;
+}
+static inline dim3 threads4(int nx) {
+  const int w = std::min(nx / 4, 32);
+  return dim3((unsigned)w, (unsigned)(256 / w));
+}
+static inline dim3 blocks4(const GridG &g) {
+  const dim3 t = threads4(g.nx);
+  return dim3((unsigned)((g.nx / 4 + (int)t.x - 1) / (int)t.x), (unsigned)((g.ny + (int)t.y - 1) / (int)t.y), (unsigned)g.nz);
+}
+static inline bool use_row4(const GridG &g) { return g.nx % 4 == 0 && g.n >= kRow4Cells; }
+// The row sums of the four cells: start[e] + sign * sum of v[e'] x[e'] over the
+// row's entries in the order of off_i (in-plane ones only without Z), x less m.
+template <bool Z, bool SUB>
+__device__ __forceinline__ void rows4(const OpK &o, const float *__restrict__ n, const float *__restrict__ x,
+                                      const Cell4 &q, float m, float s[4]) {
+  const Row4 nc = row4(n, q, 0);
+  const float4 nym = ld4(n, (unsigned)((int)q.c + q.ym)), nyp = ld4(n, (unsigned)((int)q.c + q.yp));
+  float4 nzm = make_float4(0.f, 0.f, 0.f, 0.f), nzp = nzm, xzm = nzm, xzp = nzm;
+  const Row4 xc = row4(x, q, 0), xym = row4(x, q, q.ym), xyp = row4(x, q, q.yp);
+  if (Z) {
+    nzm = plane4(n, q, q.zm, q.vzm);
+    nzp = plane4(n, q, q.zp, q.vzp);
+    xzm = plane4(x, q, q.zm, q.vzm);
+    xzp = plane4(x, q, q.zp, q.vzp);
+  }
+  auto f4 = [](const float4 &f, int e) { return e == 0 ? f.x : (e == 1 ? f.y : (e == 2 ? f.z : f.w)); };
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    float v[11];
+    row11_vals(o, nc.at(e), nc.at(e - 1), nc.at(e + 1), f4(nym, e), f4(nyp, e), f4(nzm, e), f4(nzp, e), v);
+    const float xe[11] = {xc.at(e + 1),  xc.at(e - 1),  xyp.at(e),     xym.at(e),     f4(xzp, e), f4(xzm, e),
+                          xyp.at(e + 1), xym.at(e + 1), xyp.at(e - 1), xym.at(e - 1), xc.at(e)};
+#pragma unroll
+    for (int r = 0; r < 11; r++) {
+      if (!Z && (r == 4 || r == 5 || r == 10)) continue;
+      if (SUB) s[e] -= v[r] * xe[r];
+      else s[e] += v[r] * (xe[r] - m);
+    }
+  }
+}
+// y = b - A x (k_apply, mode 1)
+__global__ void __launch_bounds__(256) k_apply4(OpK o, const float *__restrict__ n, const float *__restrict__ x,
+                                                const float *__restrict__ b, float *__restrict__ y) {
+  ECS_PDL_ENTRY();
+  Cell4 q;
+  if (!at4(o.g, q)) return;
+  const float4 bv = ld4(b, q.c);
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  rows4<true, false>(o, n, x, q, 0.f, s);
+  *reinterpret_cast<float4 *>(y + q.c) = make_float4(bv.x - s[0], bv.y - s[1], bv.z - s[2], bv.w - s[3]);
+}
+// r = b - A_xy x (k_zline_rhs)
+__global__ void __launch_bounds__(256) k_zline_rhs4(OpK o, const float *__restrict__ n, const float *__restrict__ b,
+                                                    const float *__restrict__ x, float *__restrict__ r) {
+  ECS_PDL_ENTRY();
+  Cell4 q;
+  if (!at4(o.g, q)) return;
+  const float4 bv = ld4(b, q.c);
+  float s[4] = {bv.x, bv.y, bv.z, bv.w};
+  rows4<false, true>(o, n, x, q, 0.f, s);
+  *reinterpret_cast<float4 *>(r + q.c) = make_float4(s[0], s[1], s[2], s[3]);
+}
+// Z_j = x - mean, V_{j+1} = A Z_j (k_apply_dyn)
+__global__ void __launch_bounds__(256) k_apply_dyn4(OpK o, const float *__restrict__ n, const float *__restrict__ x,
+                                                    const double *__restrict__ mean, float *__restrict__ Z,
+                                                    float *__restrict__ V, const KrylovDev *__restrict__ kd) {
+  ECS_PDL_ENTRY();
+  Cell4 q;
+  if (!at4(o.g, q)) return;
+  const int jj = kd->j;
+  const float m = mean ? (float)mean[0] : 0.f;
+  const float4 xc = ld4(x, q.c);
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  rows4<true, false>(o, n, x, q, m, s);
+  *reinterpret_cast<float4 *>(Z + (size_t)jj * o.g.n + q.c) = make_float4(xc.x - m, xc.y - m, xc.z - m, xc.w - m);
+  *reinterpret_cast<float4 *>(V + (size_t)(jj + 1) * o.g.n + q.c) = make_float4(s[0], s[1], s[2], s[3]);
+}
+
 // ---- z-line smoother --------------------------------------------------------------
 // Column (i,j) carries the z-tridiagonal part of the rows: lo = z- entry,
 // diag = centre, up = z+ entry.  A periodic z closes the cycle, solved with
@@ -500,6 +626,106 @@ __global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__
     }
   }
   f[lin3(gf, i, j, k)] += wi * wj * wk * s;
+}
+
+// The same transfers in FP32, two coarse cells (four fine ones) a thread: the
+// cells' operands overlap, and the fine ones move as float4.
+// k_restrict: coarse cells I, I + 1 (I even) from the fine columns 2I - 1 .. 2I + 3.
+__global__ void __launch_bounds__(256) k_restrict2(GridG gf, GridG gc, const float *__restrict__ f,
+                                                   float *__restrict__ c) {
+  ECS_PDL_ENTRY();
+  const int I = (int)(blockIdx.x * blockDim.x + threadIdx.x) * 2, J = (int)(blockIdx.y * blockDim.y + threadIdx.y),
+            K = (int)blockIdx.z;
+  if (I >= gc.nx || J >= gc.ny) return;
+  const bool semi = semi_z(gf, gc);
+  const Nbr q = nbr_of(gf, 2 * I, 2 * J, semi ? K : 2 * K);
+  const int oz[3] = {q.zm, 0, q.zp}, oy[3] = {q.ym, 0, q.yp};
+  const bool vz[3] = {q.vzm, true, q.vzp};
+  float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+  for (int dk = 0; dk < 3; dk++) {
+    if (semi && dk != 1) continue;
+    const float wk = semi ? 1.f : (dk == 1 ? 0.5f : 0.25f);
+    if (!vz[dk]) continue;  // a ghost plane adds zeros
+#pragma unroll
+    for (int dj = 0; dj < 3; dj++) {
+      const float w = wk * (dj == 1 ? 0.5f : 0.25f);
+      const unsigned r = (unsigned)((int)q.c + oz[dk] + oy[dj]);
+      const float m = f[(unsigned)((int)r + q.xm)];
+      const float4 v = ld4(f, r);
+      s0 += w * 0.25f * m;
+      s0 += w * 0.5f * v.x;
+      s0 += w * 0.25f * v.y;
+      s1 += w * 0.25f * v.y;
+      s1 += w * 0.5f * v.z;
+      s1 += w * 0.25f * v.w;
+    }
+  }
+  *reinterpret_cast<float2 *>(c + lin3(gc, I, J, K)) = make_float2(s0, s1);
+}
+// k_prolong_add: the four fine cells of the coarse cells I, I + 1 (and I + 2).
+__global__ void __launch_bounds__(256) k_prolong_add4(GridG gf, GridG gc, const float *__restrict__ c,
+                                                      float *__restrict__ f) {
+  ECS_PDL_ENTRY();
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x) * 4, j = (int)(blockIdx.y * blockDim.y + threadIdx.y),
+            k = (int)blockIdx.z;
+  if (i >= gf.nx || j >= gf.ny) return;
+  const bool semi = semi_z(gf, gc);
+  const Nbr q = nbr_of(gc, i >> 1, j >> 1, semi ? k : k >> 1);
+  const bool tj = j & 1, tk = !semi && (k & 1);
+  const int x2 = (i >> 1) + 2 < gc.nx ? 2 : 2 - gc.nx;  // the coarse cell after the next
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int a = 0; a < 2; a++) {
+    if (a == 1 && (!tk || !q.vzp)) break;
+#pragma unroll
+    for (int bq = 0; bq < 2; bq++) {
+      if (bq == 1 && !tj) break;
+      const unsigned r = (unsigned)((int)q.c + (a ? q.zp : 0) + (bq ? q.yp : 0));
+      const float2 u = *reinterpret_cast<const float2 *>(c + r);
+      const float w = c[(unsigned)((int)r + x2)];
+      s[0] += u.x;
+      s[1] += u.x;
+      s[1] += u.y;
+      s[2] += u.y;
+      s[3] += u.y;
+      s[3] += w;
+    }
+  }
+  const float wjk = (tj ? 0.5f : 1.f) * (tk ? 0.5f : 1.f);
+  float4 *p = reinterpret_cast<float4 *>(f + lin3(gf, i, j, k));
+  float4 t = *p;
+  t.x += wjk * s[0];
+  t.y += 0.5f * wjk * s[1];
+  t.z += wjk * s[2];
+  t.w += 0.5f * wjk * s[3];
+  *p = t;
+}
+template <typename T>
+int launch_restrict(EcsCtx *ctx, cudaStream_t s, const GridG &gf, const GridG &gc, const T *f, T *c) {
+  bool wide = false;
+  if constexpr (sizeof(T) == 4) {
+    wide = use_row4(gf);
+    if (wide) {
+      const dim3 t = threads4(gf.nx);
+      const dim3 b((unsigned)((gc.nx / 2 + (int)t.x - 1) / (int)t.x), (unsigned)((gc.ny + (int)t.y - 1) / (int)t.y), (unsigned)gc.nz);
+      ecs_launch_pdl(k_restrict2, b, t, 0, s, gf, gc, f, c);
+    }
+  }
+  if (!wide) ecs_launch_pdl(k_restrict<T>, blocks3(gc), threads3(), 0, s, gf, gc, f, c);
+  ECS_LAUNCHED(ctx);
+  return ECS_OK;
+}
+template <typename T>
+int launch_prolong_add(EcsCtx *ctx, cudaStream_t s, const GridG &gf, const GridG &gc, const T *c, T *f) {
+  bool wide = false;
+  if constexpr (sizeof(T) == 4) {
+    wide = use_row4(gf);
+    if (wide) ecs_launch_pdl(k_prolong_add4, blocks4(gf), threads4(gf.nx), 0, s, gf, gc, c, f);
+  }
+  if (!wide) ecs_launch_pdl(k_prolong_add<T>, blocks3(gf), threads3(), 0, s, gf, gc, c, f);
+  ECS_LAUNCHED(ctx);
+  return ECS_OK;
 }
 
 // ---- whole V-cycle of the small levels in one thread block -------------------
@@ -2016,9 +2242,8 @@ int mg_setup(EcsCtx *ctx) {
   ECS_CUDA(ctx, cudaStreamWaitEvent(sa, ctx->sev[0], 0));
   for (size_t l = 1; l < mg.lv.size(); l++) {
     MgLevel<T> &F = mg.lv[l - 1], &C = mg.lv[l];
-    ecs_launch_pdl(k_restrict<T>, blocks3(C.nx, C.ny, C.nz), threads3(), 0, sa, 
-        grid_level(ctx, F.nx, F.ny, F.nz), grid_level(ctx, C.nx, C.ny, C.nz), F.dens, C.dens);
-    ECS_LAUNCHED(ctx);
+    if ((rc = launch_restrict<T>(ctx, sa, grid_level(ctx, F.nx, F.ny, F.nz), grid_level(ctx, C.nx, C.ny, C.nz), F.dens, C.dens)))
+      return rc;
   }
   ECS_CUDA(ctx, cudaEventRecord(ctx->sev[1], sa));
   ECS_CUDA(ctx, cudaStreamWaitEvent(sb, ctx->sev[1], 0));
@@ -2046,7 +2271,14 @@ template <typename T>
 int sweep(EcsCtx *ctx, MgLevel<T> &L, const T *b, const T *xo, T *xn) {
   const OpK o = op_level(ctx, L);
   const T *r = b;
-  if (xo) {
+  bool row4 = false;
+  if constexpr (sizeof(T) == 4) row4 = use_row4(o.g);
+  if (xo && row4) {
+    if constexpr (sizeof(T) == 4)
+      ecs_launch_pdl(k_zline_rhs4, blocks4(o.g), threads4(L.nx), 0, ctx->stream, o, L.dens, b, xo, L.r);
+    ECS_LAUNCHED(ctx);
+    r = L.r;
+  } else if (xo) {
     ecs_launch_pdl(k_zline_rhs<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, b, xo, L.r);
     ECS_LAUNCHED(ctx);
     r = L.r;
@@ -2183,14 +2415,17 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
   MgLevel<T> &C = mg.lv[l + 1];
   const OpK o = op_level(ctx, L);
   if ((rc = sweep<T>(ctx, L, b, nullptr, L.t))) return rc;
-  ecs_launch_pdl(k_apply<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, L.t, b, L.r, 1);
+  bool row4 = false;
+  if constexpr (sizeof(T) == 4) {
+    row4 = use_row4(o.g);
+    if (row4) ecs_launch_pdl(k_apply4, blocks4(o.g), threads4(L.nx), 0, ctx->stream, o, L.dens, L.t, b, L.r);
+  }
+  if (!row4) ecs_launch_pdl(k_apply<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, L.t, b, L.r, 1);
   ECS_LAUNCHED(ctx);
   const GridG gc = grid_level(ctx, C.nx, C.ny, C.nz);
-  ecs_launch_pdl(k_restrict<T>, blocks3(gc), threads3(), 0, ctx->stream, o.g, gc, L.r, C.b);
-  ECS_LAUNCHED(ctx);
+  if ((rc = launch_restrict<T>(ctx, ctx->stream, o.g, gc, L.r, C.b))) return rc;
   if ((rc = vcycle<T>(ctx, l + 1, C.b, C.x))) return rc;
-  ecs_launch_pdl(k_prolong_add<T>, blocks3(o.g), threads3(), 0, ctx->stream, o.g, gc, C.x, L.t);
-  ECS_LAUNCHED(ctx);
+  if ((rc = launch_prolong_add<T>(ctx, ctx->stream, o.g, gc, C.x, L.t))) return rc;
   return sweep<T>(ctx, L, b, L.t, xout);
 }
 
@@ -2255,7 +2490,12 @@ int cycle_step(EcsCtx *ctx, cudaGraphConditionalHandle cond, int use_graph) {
     if ((rc = launch_reduce<T, kRedMean>(ctx, n, L0.x, (double)n, &kd->mean, cond, use_graph))) return rc;
     mean = &kd->mean;
   }
-  ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.coef, L0.x, mean, Z, V, kd);
+  bool row4 = false;
+  if constexpr (sizeof(T) == 4) {
+    row4 = use_row4(o0.g);
+    if (row4) ecs_launch_pdl(k_apply_dyn4, blocks4(o0.g), threads4(L0.nx), 0, ctx->stream, o0, L0.dens, L0.x, mean, Z, V, kd);
+  }
+  if (!row4) ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.coef, L0.x, mean, Z, V, kd);
   ECS_LAUNCHED(ctx);
   // classical Gram-Schmidt, two passes
   constexpr int W = kPack<T>;

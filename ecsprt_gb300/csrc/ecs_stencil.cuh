@@ -83,26 +83,35 @@ __device__ __forceinline__ int off_i(int e) { return (e == 0 || e == 6 || e == 7
 __device__ __forceinline__ int off_j(int e) { return (e == 2 || e == 6 || e == 8) ? 1 : ((e == 3 || e == 7 || e == 9) ? -1 : 0); }
 __device__ __forceinline__ int off_k(int e) { return e == 4 ? 1 : (e == 5 ? -1 : 0); }
 
+// A product that is rounded by itself, and a fused multiply-add.
+__device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 // 11 coefficients of a row in the order above, from the density at the
-// centre and its six face neighbours.
+// centre and its six face neighbours.  The roundings are written out, so that
+// every kernel forms the same bits however the compiler shares the products
+// of neighbouring rows.
 template <typename T>
 __device__ __forceinline__ void row11_vals(const OpK &o, T nijk, T nmjk, T npjk, T nimk, T nipk, T nijm, T nijp,
                                            T v[11]) {
   if (o.unit) nijk = nmjk = npjk = nimk = nipk = nijm = nijp = T(1);
   T sxx, syy, szz, sod;
   op_scales(o, sxx, syy, szz, sod);
-  v[6] = sod * (nipk - npjk);
-  v[7] = sod * (npjk - nimk);
-  v[8] = sod * (nmjk - nipk);
-  v[9] = sod * (nimk - nmjk);
-  v[0] = sxx * (npjk + nijk) + sod * (nipk - nimk);
-  v[1] = sxx * (nijk + nmjk) - sod * (nipk - nimk);
-  v[2] = syy * (nipk + nijk) - sod * (npjk - nmjk);
-  v[3] = syy * (nijk + nimk) + sod * (npjk - nmjk);
-  v[4] = szz * (nijp + nijk);
-  v[5] = szz * (nijk + nijm);
-  v[10] = -(sxx * (npjk + T(2) * nijk + nmjk) + syy * (nipk + T(2) * nijk + nimk) +
-            szz * (nijp + T(2) * nijk + nijm));
+  const T ty = mul_r(sod, nipk - nimk), tx = mul_r(sod, npjk - nmjk);
+  v[6] = mul_r(sod, nipk - npjk);
+  v[7] = mul_r(sod, npjk - nimk);
+  v[8] = mul_r(sod, nmjk - nipk);
+  v[9] = mul_r(sod, nimk - nmjk);
+  v[0] = fma_r(sxx, npjk + nijk, ty);
+  v[1] = fma_r(sxx, nijk + nmjk, -ty);
+  v[2] = fma_r(syy, nipk + nijk, -tx);
+  v[3] = fma_r(syy, nijk + nimk, tx);
+  v[4] = mul_r(szz, nijp + nijk);
+  v[5] = mul_r(szz, nijk + nijm);
+  v[10] = -fma_r(szz, nijp + T(2) * nijk + nijm,
+                 fma_r(sxx, npjk + T(2) * nijk + nmjk, mul_r(syy, nipk + T(2) * nijk + nimk)));
 }
 
 // 11 coefficients of row (k,j,i) in the order above.

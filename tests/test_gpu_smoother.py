@@ -21,6 +21,8 @@ ITERATIONS = {
     (12, 10, 9): 6, (17, 13, 11): 8, (21, 19, 25): 11, (33, 31, 29): 17, (50, 36, 28): 11, (66, 54, 42): 15,
     (9, 25, 100): 15, (64, 64, 9): 24, (16, 16, 160): 10, (30, 30, 30): 9, (48, 48, 48): 9,
     (33, 21, 32, "reflect"): 14, (64, 64, 32, "reflect"): 9, (130, 66, 1): 29, (128, 128, 1): 10,
+    # rows four cells a thread: the smallest level that takes them, rows of one and of 128 packs, ghosts, one plane
+    (128, 128, 4): 43, (132, 100, 68): 14, (4, 256, 128): 81, (512, 128, 4, "reflect"): 8, (256, 256, 1): 10,
 }
 
 
