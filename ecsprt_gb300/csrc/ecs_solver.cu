@@ -1585,29 +1585,66 @@ __global__ void k_sub_value(size_t n, T *__restrict__ v, const double *__restric
 // Dot products are formed 8 slots at a time, then a fixed-order block
 // reduction; slot q of block b goes to partial[q * gridDim.x + b].
 constexpr int kChunk = 8;
+// The warp's 8 sums at once: each exchange halves the slots a lane carries
+// (4 + 2 + 1 + 1 + 1 additions instead of 8 trees of 5, the same tree for every
+// slot).  In FP64 the trees held the pipe for longer than the products: dots of
+// a 64^3 basis 22.9 -> 13.2 us.
+template <typename T>
+__device__ __forceinline__ T warp_sum8(T (&a)[kChunk], int &slot) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = kChunk / 2, s = 16; h >= 1; h /= 2, s /= 2) {
+    const bool up = lane & s;
+#pragma unroll
+    for (int i = 0; i < kChunk / 2; i++)
+      if (i < h) {
+        const T send = up ? a[i] : a[i + h], keep = up ? a[i + h] : a[i];
+        a[i] = keep + __shfl_xor_sync(ECS_FULL_MASK, send, s);
+      }
+  }
+  a[0] += __shfl_xor_sync(ECS_FULL_MASK, a[0], 2);
+  a[0] += __shfl_xor_sync(ECS_FULL_MASK, a[0], 1);
+  slot = (lane & 16 ? 4 : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0);
+  return a[0];
+}
 template <typename T>
 __device__ __forceinline__ void block_chunk(const KSum<T> (&acc)[kChunk], int v0, int nslot,
                                             double *__restrict__ partial) {
   __shared__ double sh[kB / 32][kChunk];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  T v[kChunk];
 #pragma unroll
-  for (int q = 0; q < kChunk; q++) {
-    const T a = warp_sum(acc[q].value());
-    if (lane == 0) sh[warp][q] = (double)a;
-  }
+  for (int q = 0; q < kChunk; q++) v[q] = acc[q].value();
+  int slot;
+  const T t = warp_sum8(v, slot);
+  if ((lane & 3) == 0) sh[warp][slot] = (double)t;
   __syncthreads();
   if (threadIdx.x < kChunk && v0 + (int)threadIdx.x < nslot) {
-    double t = 0.0;
-    for (int w = 0; w < kB / 32; w++) t += sh[w][threadIdx.x];
-    partial[(size_t)(v0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
+    double u = 0.0;
+    for (int w = 0; w < kB / 32; w++) u += sh[w][threadIdx.x];
+    partial[(size_t)(v0 + threadIdx.x) * gridDim.x + blockIdx.x] = u;
   }
   __syncthreads();
 }
 
+// Packs e of V_{v0}..V_{v0 + kHalf - 1} (zeros past the last vector): a few
+// loads are requested before the first is used, where a load a vector inside
+// the sums waited for each in turn.
+constexpr int kHalf = 4;
+template <typename T, int W>
+__device__ __forceinline__ void ld_half(const T *__restrict__ V, size_t n, int v0, int nv, size_t e,
+                                        Pack<T, W> (&v)[kHalf]) {
+#pragma unroll
+  for (int q = 0; q < kHalf; q++) {
+#pragma unroll
+    for (int i = 0; i < W; i++) v[q].v[i] = T(0);
+    if (v0 + q < nv) v[q] = ld_pack<T, W>(V + (size_t)(v0 + q) * n + e * W);
+  }
+}
+
 // Pass 1 of classical Gram-Schmidt: dots of V_0..V_j with w = V_{j+1}.
 // Block partials, then the last block forms h1[q] (one warp a slot).  Packs
-// of W cells; one resident wave of blocks (4 an SM), so that every thread
-// has its loads of several packs in flight.
+// of W cells; one resident wave of blocks (4 an SM).
 template <typename T, int W>
 __global__ void __launch_bounds__(kB, 4) k_dots1(size_t n, const T *__restrict__ V, KrylovDev *__restrict__ kd,
                                                  double *__restrict__ partial) {
@@ -1620,12 +1657,17 @@ __global__ void __launch_bounds__(kB, 4) k_dots1(size_t n, const T *__restrict__
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += stride) {
       const Pack<T, W> we = ld_pack<T, W>(w + e * W);
 #pragma unroll
-      for (int q = 0; q < kChunk; q++)
-        if (v0 + q < nv) {
-          const Pack<T, W> vq = ld_pack<T, W>(V + (size_t)(v0 + q) * n + e * W);
+      for (int h = 0; h < kChunk; h += kHalf) {
+        if (v0 + h >= nv) break;
+        Pack<T, W> v[kHalf];
+        ld_half<T, W>(V, n, v0 + h, nv, e, v);
 #pragma unroll
-          for (int i = 0; i < W; i++) acc[q].add(vq.v[i] * we.v[i]);
-        }
+        for (int q = 0; q < kHalf; q++)
+          if (v0 + h + q < nv) {
+#pragma unroll
+            for (int i = 0; i < W; i++) acc[h + q].add(v[q].v[i] * we.v[i]);
+          }
+      }
     }
     block_chunk(acc, v0, nv, partial);
   }
@@ -1726,9 +1768,9 @@ template <typename T, int W>
 __global__ void __launch_bounds__(kB, 4) k_orth1_dots2(size_t n, T *__restrict__ V, KrylovDev *__restrict__ kd,
                                                        double *__restrict__ partial) {
   ECS_PDL_ENTRY();
-  __shared__ T h[kSlots];
+  __shared__ T hs[kSlots];
   const int nv = kd->j + 1, nslot = nv + 1;
-  if (threadIdx.x < kSlots) h[threadIdx.x] = (int)threadIdx.x < nv ? (T)kd->h1[threadIdx.x] : T(0);
+  if (threadIdx.x < kSlots) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)kd->h1[threadIdx.x] : T(0);
   __syncthreads();
   T *w = V + (size_t)nv * n;
   const size_t nw = n / W, stride = (size_t)gridDim.x * blockDim.x;
@@ -1737,24 +1779,33 @@ __global__ void __launch_bounds__(kB, 4) k_orth1_dots2(size_t n, T *__restrict__
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += stride) {
       Pack<T, W> s = ld_pack<T, W>(w + e * W);
       if (v0 == 0) {
-        for (int q = 0; q < nv; q++) {
-          const Pack<T, W> vq = ld_pack<T, W>(V + (size_t)q * n + e * W);
-          const T hq = h[q];
+        for (int h = 0; h < nv; h += kHalf) {
+          Pack<T, W> v[kHalf];
+          ld_half<T, W>(V, n, h, nv, e, v);
 #pragma unroll
-          for (int i = 0; i < W; i++) s.v[i] -= hq * vq.v[i];
+          for (int q = 0; q < kHalf; q++)
+            if (h + q < nv) {
+              const T hq = hs[h + q];
+#pragma unroll
+              for (int i = 0; i < W; i++) s.v[i] -= hq * v[q].v[i];
+            }
         }
         st_pack<T, W>(w + e * W, s);
       }
 #pragma unroll
-      for (int q = 0; q < kChunk; q++) {
-        const int v = v0 + q;
-        if (v < nv) {
-          const Pack<T, W> vq = ld_pack<T, W>(V + (size_t)v * n + e * W);
+      for (int h = 0; h < kChunk; h += kHalf) {
+        if (v0 + h > nv) break;
+        Pack<T, W> v[kHalf];
+        ld_half<T, W>(V, n, v0 + h, nv, e, v);
 #pragma unroll
-          for (int i = 0; i < W; i++) acc[q].add(vq.v[i] * s.v[i]);
-        } else if (v == nv) {
+        for (int q = 0; q < kHalf; q++) {
+          if (v0 + h + q < nv) {
 #pragma unroll
-          for (int i = 0; i < W; i++) acc[q].add(s.v[i] * s.v[i]);
+            for (int i = 0; i < W; i++) acc[h + q].add(v[q].v[i] * s.v[i]);
+          } else if (v0 + h + q == nv) {
+#pragma unroll
+            for (int i = 0; i < W; i++) acc[h + q].add(s.v[i] * s.v[i]);
+          }
         }
       }
     }
@@ -1786,11 +1837,16 @@ __global__ void k_orth2_scale(size_t n, T *__restrict__ V, KrylovDev *kd, T *__r
   const size_t nw = n / W, stride = (size_t)(gridDim.x - 1) * blockDim.x;
   for (size_t e = (size_t)(blockIdx.x - 1) * blockDim.x + threadIdx.x; e < nw; e += stride) {
     Pack<T, W> s = ld_pack<T, W>(w + e * W);
-    for (int q = 0; q < nv; q++) {
-      const Pack<T, W> vq = ld_pack<T, W>(V + (size_t)q * n + e * W);
-      const T hq = h[q];
+    for (int v0 = 0; v0 < nv; v0 += kHalf) {
+      Pack<T, W> v[kHalf];
+      ld_half<T, W>(V, n, v0, nv, e, v);
 #pragma unroll
-      for (int i = 0; i < W; i++) s.v[i] -= hq * vq.v[i];
+      for (int q = 0; q < kHalf; q++)
+        if (v0 + q < nv) {
+          const T hq = h[v0 + q];
+#pragma unroll
+          for (int i = 0; i < W; i++) s.v[i] -= hq * v[q].v[i];
+        }
     }
 #pragma unroll
     for (int i = 0; i < W; i++) s.v[i] *= sc;
