@@ -47,11 +47,7 @@ __global__ void k_moments(size_t n, const long long *__restrict__ acc, double *_
   }
 }
 
-// ---- RHS: src/rhs.c:321-354 --------------------------------------------------
-struct RhsK {
-  double kappa, hx, hy, hz, hxx, hyy, hzz, E0, cth, cG, scale;
-};
-
+// ---- RHS: src/rhs.c:321-354 (rhs_value) ---------------------------------------
 // Fixed-order sum of `local` over the block into partial[block].
 __device__ __forceinline__ void block_partial(double local, double *sh, double *__restrict__ partial) {
   for (int s = 16; s >= 1; s >>= 1) local += __shfl_xor_sync(ECS_FULL_MASK, local, s);
@@ -76,23 +72,11 @@ __global__ void k_rhs(GridG g, RhsK r, const double *__restrict__ mom, double *_
   if (at3(g.nx, g.ny, i, j, k0)) {
     for (int k = k0; k < g.nz; k += gridDim.z) {
       const Nbr q = nbr_of(g, i, j, k);  // the neighbours' offsets (gval's wrap and ghosts)
-      rd nijk{n[q.c]};
-      rd npjk{nval(n, q, q.xp, q.vxp)}, nmjk{nval(n, q, q.xm, q.vxm)};
-      rd nipk{nval(n, q, q.yp, q.vyp)}, nimk{nval(n, q, q.ym, q.vym)};
-      rd nijp{nval(n, q, q.zp, q.vzp)}, nijm{nval(n, q, q.zm, q.vzm)};
-      rd two{2.0}, one{1.0}, kap{r.kappa};
-      rd dndx = rd{r.hx} * (npjk - nmjk);
-      rd dndy = rd{r.hy} * (nipk - nimk);
-      rd d2ndxx = rd{r.hxx} * ((npjk - two * nijk) + nmjk);
-      rd d2ndyy = rd{r.hyy} * ((nipk - two * nijk) + nimk);
-      rd d2ndzz = rd{r.hzz} * ((nijp - two * nijk) + nijm);
-      rd dGxdx = rd{r.hx} * (rd{nval(Gx, q, q.xp, q.vxp)} - rd{nval(Gx, q, q.xm, q.vxm)});
-      rd dGydy = rd{r.hy} * (rd{nval(Gy, q, q.yp, q.vyp)} - rd{nval(Gy, q, q.ym, q.vym)});
-      rd dGzdz = rd{r.hz} * (rd{nval(Gz, q, q.zp, q.vzp)} - rd{nval(Gz, q, q.zm, q.vzm)});
-      rd Eterm = (dndy - kap * dndx) * rd{r.E0};
-      rd Pterm = rd{r.cth} * ((d2ndxx + d2ndyy) + (one + kap * kap) * d2ndzz);
-      rd Gterm = rd{r.cG} * ((dGxdx + dGydy) + dGzdz);
-      double v = (rd{r.scale} * ((Eterm + Pterm) + Gterm)).v;
+      const double v = rhs_value(
+          r, rd{n[q.c]}, rd{nval(n, q, q.xp, q.vxp)}, rd{nval(n, q, q.xm, q.vxm)}, rd{nval(n, q, q.yp, q.vyp)},
+          rd{nval(n, q, q.ym, q.vym)}, rd{nval(n, q, q.zp, q.vzp)}, rd{nval(n, q, q.zm, q.vzm)},
+          rd{nval(Gx, q, q.xp, q.vxp)}, rd{nval(Gx, q, q.xm, q.vxm)}, rd{nval(Gy, q, q.yp, q.vyp)},
+          rd{nval(Gy, q, q.ym, q.vym)}, rd{nval(Gz, q, q.zp, q.vzp)}, rd{nval(Gz, q, q.zm, q.vzm)});
       b[q.c] = v;
       local += v;
     }
@@ -207,11 +191,7 @@ int ecs_grid_rhs(EcsCtx *ctx) {
   if (p.rhs_type == ECS_RHS_SINUSOIDAL) {
     k_rhs_sin<<<grid, threads3(), 0, ctx->stream>>>(g, p.ndim, p.dx, p.dy, p.dz, p.n0, p.scale, ctx->rhs, ctx->red);
   } else {
-    RhsK r;
-    r.kappa = p.kappa_e;
-    r.hx = 1.0 / (2.0 * p.dx); r.hy = 1.0 / (2.0 * p.dy); r.hz = 1.0 / (2.0 * p.dz);
-    r.hxx = 1.0 / (p.dx * p.dx); r.hyy = 1.0 / (p.dy * p.dy); r.hzz = 1.0 / (p.dz * p.dz);
-    r.E0 = p.E0; r.cth = p.cth; r.cG = p.cG; r.scale = p.scale;
+    const RhsK r = make_rhs(p, p.dz);
     k_rhs<<<grid, threads3(), 0, ctx->stream>>>(g, r, ctx->mom, ctx->rhs, ctx->red);
   }
   ECS_LAUNCHED(ctx);

@@ -11,11 +11,12 @@
 // buffers; this entry point needs only a small reduction scratch, which lives
 // in a file-scope __device__ array instead of an allocation.
 //
-// Scratch: ECS_NOALLOC_RHS_MAX_BLOCKS FP64 block partial sums plus one slot
-// for the mean (32 KiB + 8 B), present on every device that loads the
-// library until the process exits.  Each thread block reduces
-// ECS_NOALLOC_RHS_CELLS_PER_BLOCK cells, so grids of at most
-// ECS_NOALLOC_RHS_MAX_CELLS cells (256 x 256 x 128) are accepted.
+// Scratch: ECS_NOALLOC_RHS_MAX_BLOCKS FP64 block partial sums plus a slot for
+// the mean and one for the reduction's completion count (32 KiB + 16 B),
+// present on every device that loads the library until the process exits.
+// Each thread block reduces at most ECS_NOALLOC_RHS_CELLS_PER_BLOCK cells, so
+// grids of at most ECS_NOALLOC_RHS_MAX_CELLS cells (256 x 256 x 128) are
+// accepted.
 //
 // Every call shares the array: each call writes every partial and the mean
 // before it reads them, so nothing from an earlier call is used, but two
@@ -32,67 +33,47 @@
 #include <algorithm>
 #include <mutex>
 
-#include "ecs_internal.cuh"
+#include "ecs_stencil.cuh"
 
 #define ECS_NOALLOC_RHS_MAX_BLOCKS 4096
 #define ECS_NOALLOC_RHS_CELLS_PER_BLOCK 2048
 #define ECS_NOALLOC_RHS_MAX_CELLS (ECS_NOALLOC_RHS_MAX_BLOCKS * ECS_NOALLOC_RHS_CELLS_PER_BLOCK)
 #define ECS_NOALLOC_MAX_DEVICES 64
 
-// [0, MAX_BLOCKS): block partial sums of b; [MAX_BLOCKS]: the mean of b.
-static __device__ __align__(256) double g_rhs_scratch[ECS_NOALLOC_RHS_MAX_BLOCKS + 1];
+// [0, MAX_BLOCKS): block partial sums of b; [MAX_BLOCKS]: the mean of b;
+// [MAX_BLOCKS + 1]: blocks done (0 between calls).
+static __device__ __align__(256) double g_rhs_scratch[ECS_NOALLOC_RHS_MAX_BLOCKS + 2];
 
 namespace {
 
 constexpr int kThreads = 256;
-
-struct rdn {
-  double v;
-};
-__device__ __forceinline__ rdn operator+(rdn a, rdn b) { return {__dadd_rn(a.v, b.v)}; }
-__device__ __forceinline__ rdn operator-(rdn a, rdn b) { return {__dsub_rn(a.v, b.v)}; }
-__device__ __forceinline__ rdn operator*(rdn a, rdn b) { return {__dmul_rn(a.v, b.v)}; }
 
 struct RhsNoAllocK {
   int nx, ny, nz;
   int bc[3];
   int ndim;
   size_t n;
-  double kappa, hx, hy, hz, hxx, hyy, hzz, E0, cth, cG, scale;
-  double dx, dy, dz, n0;  // -rhs sinusoidal
+  RhsK r;
+  double scale, dx, dy, dz, n0;  // -rhs sinusoidal
 };
 
-// Moment c of node (k,j,i) from FluidNode{n,Gx,Gy,Gz} storage, with the
-// reference's ghost semantics (periodic wrap, zero outside ghosted axes).
-__device__ __forceinline__ double node_moment(const double *__restrict__ m, const RhsNoAllocK &g, int k,
-                                              int j, int i, int c) {
-  if (i < 0 || i >= g.nx) { if (g.bc[0]) return 0.0; i = i < 0 ? i + g.nx : i - g.nx; }
-  if (j < 0 || j >= g.ny) { if (g.bc[1]) return 0.0; j = j < 0 ? j + g.ny : j - g.ny; }
-  if (k < 0 || k >= g.nz) { if (g.bc[2]) return 0.0; k = k < 0 ? k + g.nz : k - g.nz; }
-  return m[(((size_t)k * g.ny + j) * g.nx + i) * 4 + c];
-}
-
-// b of the full RHS (src/rhs.c:321-354) at node (k, j, i).  A 2-D grid is
-// one node deep with a unit, periodic z cell, so every z term is exactly 0.
+// b of the full RHS (src/rhs.c:321-354) at node (k, j, i) from
+// FluidNode{n,Gx,Gy,Gz} storage, with the reference's ghost semantics
+// (periodic wrap, zero outside ghosted axes).  A 2-D grid is one node deep
+// with a unit, periodic z cell, so every z term is exactly 0.
 __device__ __forceinline__ double full_rhs(const double *__restrict__ mom, const RhsNoAllocK &g, int k, int j,
                                            int i) {
-  rdn nijk{node_moment(mom, g, k, j, i, 0)};
-  rdn npjk{node_moment(mom, g, k, j, i + 1, 0)}, nmjk{node_moment(mom, g, k, j, i - 1, 0)};
-  rdn nipk{node_moment(mom, g, k, j + 1, i, 0)}, nimk{node_moment(mom, g, k, j - 1, i, 0)};
-  rdn nijp{node_moment(mom, g, k + 1, j, i, 0)}, nijm{node_moment(mom, g, k - 1, j, i, 0)};
-  rdn two{2.0}, one{1.0}, kap{g.kappa};
-  rdn dndx = rdn{g.hx} * (npjk - nmjk);
-  rdn dndy = rdn{g.hy} * (nipk - nimk);
-  rdn d2ndxx = rdn{g.hxx} * ((npjk - two * nijk) + nmjk);
-  rdn d2ndyy = rdn{g.hyy} * ((nipk - two * nijk) + nimk);
-  rdn d2ndzz = rdn{g.hzz} * ((nijp - two * nijk) + nijm);
-  rdn dGxdx = rdn{g.hx} * (rdn{node_moment(mom, g, k, j, i + 1, 1)} - rdn{node_moment(mom, g, k, j, i - 1, 1)});
-  rdn dGydy = rdn{g.hy} * (rdn{node_moment(mom, g, k, j + 1, i, 2)} - rdn{node_moment(mom, g, k, j - 1, i, 2)});
-  rdn dGzdz = rdn{g.hz} * (rdn{node_moment(mom, g, k + 1, j, i, 3)} - rdn{node_moment(mom, g, k - 1, j, i, 3)});
-  rdn Eterm = (dndy - kap * dndx) * rdn{g.E0};
-  rdn Pterm = rdn{g.cth} * ((d2ndxx + d2ndyy) + (one + kap * kap) * d2ndzz);
-  rdn Gterm = rdn{g.cG} * ((dGxdx + dGydy) + dGzdz);
-  return (rdn{g.scale} * ((Eterm + Pterm) + Gterm)).v;
+  GridG gg;
+  gg.nx = g.nx; gg.ny = g.ny; gg.nz = g.nz;
+  for (int d = 0; d < 3; d++) gg.bc[d] = g.bc[d];
+  const Nbr q = nbr_of(gg, i, j, k);
+  auto at = [&](int off, bool valid, int c) {
+    return rd{valid ? mom[(size_t)(unsigned)((int)q.c + off) * 4 + c] : 0.0};
+  };
+  return rhs_value(g.r, at(0, true, 0), at(q.xp, q.vxp, 0), at(q.xm, q.vxm, 0), at(q.yp, q.vyp, 0),
+                   at(q.ym, q.vym, 0), at(q.zp, q.vzp, 0), at(q.zm, q.vzm, 0), at(q.xp, q.vxp, 1),
+                   at(q.xm, q.vxm, 1), at(q.yp, q.vyp, 2), at(q.ym, q.vym, 2), at(q.zp, q.vzp, 3),
+                   at(q.zm, q.vzm, 3));
 }
 
 // b of -rhs sinusoidal (src/rhs.c:82-148; 2-D src/rhs.c:26-79): n0 cos(2 pi
@@ -107,50 +88,57 @@ __device__ __forceinline__ double sin_rhs(const RhsNoAllocK &g, int k, int j, in
   return __dmul_rn(__dmul_rn(g.n0, val), g.scale);
 }
 
-// One block per ECS_NOALLOC_RHS_CELLS_PER_BLOCK consecutive cells; each
-// block writes its partial sum of b into partials[blockIdx.x].
+// One block per `cells` consecutive cells (256 on small grids, so that the
+// FP64 work spreads over the SMs: with 2048 always, a 32^3 grid ran on 16 of
+// them); each block writes its partial sum of b into partials[blockIdx.x], and
+// the one that finishes last forms the mean from the partials in a fixed order
+// (strided per thread, warp tree, then the warps in order).  No block waits on
+// another.
 template <bool kSinusoidal>
-__global__ void __launch_bounds__(kThreads) k_rhs_noalloc(RhsNoAllocK g, const double *__restrict__ mom,
+__global__ void __launch_bounds__(kThreads) k_rhs_noalloc(RhsNoAllocK g, int cells, const double *__restrict__ mom,
                                                           double *__restrict__ b, double *__restrict__ partials) {
   __shared__ double sh[kThreads / 32];
+  __shared__ int last;
   double local = 0.0;
-  const size_t c0 = (size_t)blockIdx.x * ECS_NOALLOC_RHS_CELLS_PER_BLOCK;
-  for (int q = threadIdx.x; q < ECS_NOALLOC_RHS_CELLS_PER_BLOCK; q += blockDim.x) {
-    const size_t c = c0 + q;
-    if (c >= g.n) break;
-    const int i = (int)(c % g.nx), j = (int)((c / g.nx) % g.ny), k = (int)(c / ((size_t)g.nx * g.ny));
+  const unsigned c0 = blockIdx.x * (unsigned)cells, n = (unsigned)g.n;
+  for (unsigned c = c0 + threadIdx.x; c < n && c < c0 + (unsigned)cells; c += kThreads) {
+    const unsigned r = c / (unsigned)g.nx;
+    const int i = (int)(c - r * (unsigned)g.nx), j = (int)(r % (unsigned)g.ny), k = (int)(r / (unsigned)g.ny);
     const double v = kSinusoidal ? sin_rhs(g, k, j, i) : full_rhs(mom, g, k, j, i);
     b[c] = v;
     local += v;
   }
-  for (int s = 16; s >= 1; s >>= 1) local += __shfl_xor_sync(ECS_FULL_MASK, local, s);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = local;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < kThreads / 32; w++) t += sh[w];
-    partials[blockIdx.x] = t;
-  }
-}
-
-// The mean, once: one block sums the nb partials in a fixed order (strided
-// per thread, warp tree, then the warps in order) into partials[MAX_BLOCKS].
-__global__ void __launch_bounds__(1024) k_mean_noalloc(int nb, double n, double *__restrict__ partials) {
-  __shared__ double sh[32];
-  double t = 0.0;
-  for (int q = threadIdx.x; q < nb; q += blockDim.x) t += partials[q];
-  for (int s = 16; s >= 1; s >>= 1) t += __shfl_xor_sync(ECS_FULL_MASK, t, s);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  auto block_sum = [&](double t) {
+    for (int s = 16; s >= 1; s >>= 1) t += __shfl_xor_sync(ECS_FULL_MASK, t, s);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = t;
+    __syncthreads();
     double u = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) u += sh[w];
-    partials[ECS_NOALLOC_RHS_MAX_BLOCKS] = u / n;
+    if (threadIdx.x == 0)
+      for (int w = 0; w < kThreads / 32; w++) u += sh[w];
+    return u;
+  };
+  const double mine = block_sum(local);
+  unsigned int *done = reinterpret_cast<unsigned int *>(partials + ECS_NOALLOC_RHS_MAX_BLOCKS + 1);
+  if (threadIdx.x == 0) {
+    partials[blockIdx.x] = mine;
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x - 1;
+    __threadfence();
   }
+  __syncthreads();
+  if (!last) return;
+  double t = 0.0;
+  for (unsigned q = threadIdx.x; q < gridDim.x; q += kThreads) t += __ldcg(partials + q);
+  const double u = block_sum(t);
+  if (threadIdx.x == 0) partials[ECS_NOALLOC_RHS_MAX_BLOCKS] = u / (double)g.n;
 }
 
-__global__ void __launch_bounds__(kThreads) k_sub_mean_noalloc(size_t n, double *__restrict__ b,
-                                                               const double *__restrict__ partials) {
+// b -= mean.  Also puts the completion count back to 0, whatever a call that
+// overlapped this one has left there, so that the next call starts clean.
+__global__ void __launch_bounds__(kThreads) k_sub_mean_noalloc(size_t n, double *__restrict__ b, double *partials) {
+  if (blockIdx.x == 0 && threadIdx.x == 0)
+    *reinterpret_cast<unsigned int *>(partials + ECS_NOALLOC_RHS_MAX_BLOCKS + 1) = 0u;
   const double mean = partials[ECS_NOALLOC_RHS_MAX_BLOCKS];
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
     b[c] -= mean;
@@ -224,19 +212,17 @@ extern "C" int ecs_rhs_noalloc(const EcsParams *params, const double *d_moments,
   for (int d = 0; d < 3; d++) g.bc[d] = p.bc[d] == ECS_BC_PERIODIC ? 0 : 1;
   g.ndim = p.ndim;
   g.n = n;
-  g.kappa = p.kappa_e;
-  g.hx = 1.0 / (2.0 * p.dx); g.hy = 1.0 / (2.0 * p.dy); g.hz = 1.0 / (2.0 * p.dz);
-  g.hxx = 1.0 / (p.dx * p.dx); g.hyy = 1.0 / (p.dy * p.dy); g.hzz = 1.0 / (p.dz * p.dz);
-  g.E0 = p.E0; g.cth = p.cth; g.cG = p.cG; g.scale = p.scale;
+  g.r = make_rhs(p, p.dz);
+  g.scale = p.scale;
   g.dx = p.dx; g.dy = p.dy; g.dz = p.dz; g.n0 = p.n0;
-  const int nb = (int)((n + ECS_NOALLOC_RHS_CELLS_PER_BLOCK - 1) / ECS_NOALLOC_RHS_CELLS_PER_BLOCK);
+  const int cells = (int)std::max<size_t>(kThreads, ((n + ECS_NOALLOC_RHS_MAX_BLOCKS - 1) / ECS_NOALLOC_RHS_MAX_BLOCKS +
+                                                     kThreads - 1) / kThreads * kThreads);
+  const int nb = (int)((n + cells - 1) / cells);
   if (p.rhs_type == ECS_RHS_SINUSOIDAL)
-    k_rhs_noalloc<true><<<nb, kThreads, 0, s>>>(g, d_moments, d_rhs, scratch);
+    k_rhs_noalloc<true><<<nb, kThreads, 0, s>>>(g, cells, d_moments, d_rhs, scratch);
   else
-    k_rhs_noalloc<false><<<nb, kThreads, 0, s>>>(g, d_moments, d_rhs, scratch);
+    k_rhs_noalloc<false><<<nb, kThreads, 0, s>>>(g, cells, d_moments, d_rhs, scratch);
   if ((rc = launched("rhs"))) return rc;
-  k_mean_noalloc<<<1, 1024, 0, s>>>(nb, (double)n, scratch);
-  if ((rc = launched("mean"))) return rc;
   k_sub_mean_noalloc<<<nb_elem, kThreads, 0, s>>>(n, d_rhs, scratch);
   return launched("mean removal");
 }

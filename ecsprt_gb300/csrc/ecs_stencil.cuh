@@ -3,6 +3,8 @@
 // and the 11-coefficient operator row of src/lhs.c:366-423.
 #pragma once
 
+#include <math.h>
+
 #include "ecs_internal.cuh"
 
 // FP64 arithmetic with every operation separately rounded (no contraction),
@@ -202,4 +204,59 @@ static inline OpK make_op(const EcsParams &p, int nx, int ny, int nz, double hx,
 }
 static inline GridG make_grid(const EcsParams &p, int nx, int ny, int nz) {
   return make_op(p, nx, ny, nz, 1.0, 1.0, 1.0).g;
+}
+
+// ---- right-hand side (src/rhs.c:321-354) -------------------------------------
+// The reference's operation order, every operation separately rounded.  The
+// row is bound by the FP64 pipe (1/64 of the FP32 rate), so what FP64
+// arithmetic cannot change runs on the integer units: products with a power of
+// two (1/(2 dx), 1/dx^2 of a power-of-two spacing, 2 n) are exponent
+// additions, 1 + kappa^2 is formed on the host, and without a background field
+// its term, an exact zero for finite densities, is left out.  128^3 and
+// dx = 1: 42 -> 25 FP64 operations a cell.
+constexpr int kNoPow2 = 1 << 20;
+struct RhsK {
+  double kappa, opk2, hx, hy, hz, hxx, hyy, hzz, E0, cth, cG, scale;
+  int px, py, pz, pxx, pyy, pzz;  // h = 2^p exactly, or kNoPow2
+};
+static inline int pow2_of(double h) {
+  int e = 0;
+  return frexp(h, &e) == 0.5 && e >= -62 && e <= 64 ? e - 1 : kNoPow2;
+}
+static inline RhsK make_rhs(const EcsParams &p, double dz) {
+  RhsK r;
+  volatile double k2 = p.kappa_e * p.kappa_e;  // rounded by itself
+  r.kappa = p.kappa_e;
+  r.opk2 = 1.0 + k2;
+  r.hx = 1.0 / (2.0 * p.dx); r.hy = 1.0 / (2.0 * p.dy); r.hz = 1.0 / (2.0 * dz);
+  r.hxx = 1.0 / (p.dx * p.dx); r.hyy = 1.0 / (p.dy * p.dy); r.hzz = 1.0 / (dz * dz);
+  r.px = pow2_of(r.hx); r.py = pow2_of(r.hy); r.pz = pow2_of(r.hz);
+  r.pxx = pow2_of(r.hxx); r.pyy = pow2_of(r.hyy); r.pzz = pow2_of(r.hzz);
+  r.E0 = p.E0; r.cth = p.cth; r.cG = p.cG; r.scale = p.scale;
+  return r;
+}
+// h v for h = 2^p (any h when p is kNoPow2).
+__device__ __forceinline__ rd scale2(double h, int p, rd v) {
+  const int hi = __double2hiint(v.v), e = (hi >> 20) & 0x7ff;
+  if (p == kNoPow2 || (unsigned)(e - 128) > 1792u) return e == 0 && ((hi << 1) | __double2loint(v.v)) == 0 ? v : rd{h} * v;
+  return rd{__hiloint2double(hi + p * (1 << 20), __double2loint(v.v))};
+}
+// b from the density at the node and its six neighbours and the flux at the
+// two neighbours along its own axis.
+__device__ __forceinline__ double rhs_value(const RhsK &r, rd nijk, rd npjk, rd nmjk, rd nipk, rd nimk, rd nijp, rd nijm,
+                                            rd gxp, rd gxm, rd gyp, rd gym, rd gzp, rd gzm) {
+  const rd n2 = scale2(2.0, 1, nijk);
+  const rd d2ndxx = scale2(r.hxx, r.pxx, (npjk - n2) + nmjk);
+  const rd d2ndyy = scale2(r.hyy, r.pyy, (nipk - n2) + nimk);
+  const rd d2ndzz = scale2(r.hzz, r.pzz, (nijp - n2) + nijm);
+  const rd dGxdx = scale2(r.hx, r.px, gxp - gxm);
+  const rd dGydy = scale2(r.hy, r.py, gyp - gym);
+  const rd dGzdz = scale2(r.hz, r.pz, gzp - gzm);
+  rd t = rd{r.cth} * ((d2ndxx + d2ndyy) + rd{r.opk2} * d2ndzz);
+  if (r.E0 != 0.0) {
+    const rd dndx = scale2(r.hx, r.px, npjk - nmjk), dndy = scale2(r.hy, r.py, nipk - nimk);
+    t = (dndy - rd{r.kappa} * dndx) * rd{r.E0} + t;
+  }
+  const rd Gterm = rd{r.cG} * ((dGxdx + dGydy) + dGzdz);
+  return (rd{r.scale} * (t + Gterm)).v;
 }

@@ -205,7 +205,7 @@ int ecs_lhs_apply_host(EcsCtx *ctx, const double *x, double *y);
    may be NULL, unless -rhs full) and d_rhs (device, [Nz][Ny][Nx]) belong to
    the caller; the work is queued on `stream` (a cudaStream_t, NULL for the
    default stream).  The parameters are checked as ecs_ctx_create checks
-   them.  Its reduction scratch is a fixed __device__ array of 32 KiB + 8 B
+   them.  Its reduction scratch is a fixed __device__ array of 32 KiB + 16 B
    held by every device that loads the library, so grids of more than
    8,388,608 nodes (256 x 256 x 128) are rejected with ECS_ERR_INVALID.  The
    first call on a device looks up the array's device address
