@@ -1154,10 +1154,14 @@ __global__ void __launch_bounds__(kBlock, 3) k_particles32(PartK k, int mode, in
 // way when a sort follows.
 //
 // Loads: each thread's next ion record is loaded into registers (one
-// 256-bit load) while it works on the current one, with the permutation
-// entry of the one after that loaded a step earlier, so the memory latency
-// of a record overlaps the arithmetic of the previous ion.  All sums are
-// exact integers, so the moments equal those of k_particles32 bit for bit.
+// 256-bit load) while it works on the current one, so the memory latency
+// of a record overlaps the arithmetic of the previous ion.  The lanes' ions are
+// a segment apart, so a 4-byte permutation entry an ion would take a line of
+// its own in the L1 data pipe, the busiest unit, as a whole record does: the
+// chunk's entries are read as whole lines into shared memory first (128^3, 64
+// ions a cell: the pass after a sort 3.39 -> 3.29 ms; the sort keys written the
+// same way gave nothing).  All sums are exact integers, so the moments equal
+// those of k_particles32 bit for bit.
 
 // Block shape of the tile kernel: one block a tile.
 constexpr int kTileThreads = 256;
@@ -1236,6 +1240,9 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM) k_tiles32(Part
   __shared__ int dcnt[kWCells];       // window deposits a cell (bias removal)
   __shared__ float2 ewxy[kEXY * kWZ];  // x, y difference numerators of the window's nodes (padded strides)
   __shared__ float ewz[kWPad];         // z numerators, at the deposit window's strides
+  // the chunk's permutation entries; one word of padding in 64 keeps lanes a
+  // segment of 64 apart in different banks
+  __shared__ int32_t entry[kWindowMax + kWindowMax / 64 + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool collide = (mode & 2) && k.collide;
   unsigned int nacc = 0, nref = 0;  // collision counters of this thread, flushed at the end
@@ -1262,6 +1269,8 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM) k_tiles32(Part
       float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb4 = na;  // the next record
       if (mend > 0) ld_record(src + 2 * src_pos(0), na, nb4);
       if (mend > 1) sp_next = src_pos(1);
+      if (perm)
+        for (int e = threadIdx.x; e < L; e += blockDim.x) entry[e + (e >> 6)] = __ldg(perm + ca + e);
       if ((mode & 1) && ca == a) {  // window nodes outside the extended grid are never read
         const int sx = k.Nx + 1, sxy = sx * (k.Ny + 1);
         for (int e = threadIdx.x; e < kWNodes; e += blockDim.x) {
@@ -1283,7 +1292,10 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM) k_tiles32(Part
         const float4 ra = na, rb = nb4;
         if (m + 1 < mend) {  // the next record, in flight while this one is worked on
           ld_record(src + 2 * sp_next, na, nb4);
-          if (m + 2 < mend) sp_next = src_pos(m + 2);
+          if (m + 2 < mend) {
+            const int e = qi0 + m + 2;
+            sp_next = perm ? (int64_t)entry[e + (e >> 6)] : (int64_t)ca + e;
+          }
         }
         IonState q = ion_state(Ion{__float_as_int(ra.x), ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, __float_as_int(rb.w)});
         const int64_t ip = (int64_t)ca + qi0 + m;
