@@ -154,7 +154,7 @@ struct EcsCtx {
   double *phi = nullptr;            // potential [ncell]
   double4_32a *eext64 = nullptr;        // difference numerators on extended nodes
   float4 *eext32 = nullptr;
-  long long *acc = nullptr;         // fixed-point moments [4][ncell]
+  long long *acc = nullptr;         // fixed-point moments, [4][ncell] or [ncell][4] (ecs_acc_interleaved)
   double *mom = nullptr;            // FP64 moments SoA [4][ncell]
   double *rhs = nullptr;            // [ncell]
   double *red = nullptr;            // reduction scratch (FP64)
@@ -352,6 +352,17 @@ int ecs_grid_eext(EcsCtx *ctx);          // difference numerators from phi
 int ecs_grid_moments(EcsCtx *ctx);       // fixed-point -> FP64 moments
 int ecs_grid_rhs(EcsCtx *ctx);           // RHS (+ mean removal) from moments
 int ecs_grid_clear_acc(EcsCtx *ctx);
+// Layout of the deposit accumulators.  A global reduction costs the L1 data
+// pipe a pass per 32-byte sector, so the passes that add an ion's fields node
+// by node (FP64, 2-D) keep a node's four side by side: 8 sectors an ion
+// instead of about 20 in 3-D (64^3 FP64, 64 ions a cell: 4.39 -> 4.36 ms, the
+// arithmetic bounds it), 4 instead of 7.5 in 2-D (256^2 mixed, 64 ions a cell:
+// 222 -> 175 us).  The tile kernel adds
+// rows of nodes a field at a time and keeps the fields apart (7 nodes of a
+// row in 2 to 3 sectors).
+static inline bool ecs_acc_interleaved(const EcsCtx *ctx) {
+  return ctx->prec == ECS_PREC_FP64 || ctx->p.ndim == 2;
+}
 int ecs_solver_alloc(EcsCtx *ctx);       // reductions, Krylov bases, control block
 int ecs_solver_setup(EcsCtx *ctx);       // multigrid hierarchy from the density
 // setup = 1: compute the RHS and set up the operator first (the step's field

@@ -252,6 +252,8 @@ struct PartK {
   int Nx, Ny, Nz;
   int bc[3];
   size_t ncell;
+  int acc_shift;     // accumulator of field f at node c: acc[(c << acc_shift) + f acc_field]
+  size_t acc_field;
   double dx, dy, dz;
   double lo[3], hi[3], L[3];  // grid bounds (x0, x1, Lx per axis)
   double dinv[3];             // 1 / cell width, rounded
@@ -291,6 +293,11 @@ __device__ __forceinline__ int corner_node(const PartK &k, int i, int j, int kk,
   if (jj >= k.Ny) { if (k.bc[1]) return -1; jj -= k.Ny; }
   if (zz >= k.Nz) { if (k.bc[2]) return -1; zz -= k.Nz; }
   return (zz * k.Ny + jj) * k.Nx + ii;  // at most 2^30 nodes
+}
+
+// Where field f of a node is accumulated (EcsCtx::acc_interleaved).
+__device__ __forceinline__ size_t acc_index(const PartK &k, int f, int node) {
+  return ((size_t)node << k.acc_shift) + (size_t)f * k.acc_field;
 }
 
 // Deposit one particle's CIC contributions (src/moments.c:162-205): weights
@@ -376,7 +383,7 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
     const long long sum = lane < 8 ? full_sum(row, fn) : full_sum(row, ff);
     const int node = nodes[(lane & 7) * kTileStride];
     if (node >= 0 && sum != 0)
-      atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
+      atomicAdd((unsigned long long *)&acc[acc_index(k, lane >> 3, node)], (unsigned long long)sum);
     rem = 0;
   } else if (__all_sync(ECS_FULL_MASK, !active || (peers & (peers - 1u)) == 0u)) {
     // no two ions in one cell (any order but a sorted one): lane l issues slot
@@ -387,7 +394,7 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
       const long long sum = lane < 8 ? entry_value(e, fn) : entry_value(e, ff);
       const int node = nodes[(lane & 7) * kTileStride + q];
       if (node >= 0 && sum != 0)
-        atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
+        atomicAdd((unsigned long long *)&acc[acc_index(k, lane >> 3, node)], (unsigned long long)sum);
     }
     rem = 0;
   }
@@ -398,7 +405,7 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
     const long long sum = lane < 8 ? group_sum(row, grp, fn) : group_sum(row, grp, ff);
     const int node = nodes[(lane & 7) * kTileStride + lead];
     if (node >= 0 && sum != 0)
-      atomicAdd((unsigned long long *)&acc[(size_t)(lane >> 3) * k.ncell + node], (unsigned long long)sum);
+      atomicAdd((unsigned long long *)&acc[acc_index(k, lane >> 3, node)], (unsigned long long)sum);
   }
   __syncwarp();
 }
@@ -411,7 +418,7 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
 // a half, so that 12 of 16 lanes work and 16 iterations do; few cells
 // (kFlatGroups or fewer: ions in cell order) are summed first, each half its
 // own lanes' ions.  k_particles32 at 256^2 cells, 64 ions a cell: any order
-// 293 -> 222 us, cell order 161 -> 103 us.
+// 293 -> 222 us (175 with interleaved accumulators), cell order 161 -> 103 us.
 constexpr int kFlatGroups = 8;
 __device__ __forceinline__ void deposit_flat(long long *__restrict__ acc, unsigned char *tile_mem, const PartK &k,
                                              bool active, int i, int j, float wxh, float wyh, float v0, float v1) {
@@ -437,7 +444,7 @@ __device__ __forceinline__ void deposit_flat(long long *__restrict__ acc, unsign
   // lanes 12 to 15 of a half follow the rows of lanes 0 to 3
   const unsigned *row = words + (slot % 12) * kTileStride, *row_l = words + (12 + (slot & 3)) * kTileStride;
   const int *node_of = nodes + (slot & 3) * kTileStride;
-  unsigned long long *dst = reinterpret_cast<unsigned long long *>(acc) + (size_t)(slot >> 2) * k.ncell;
+  unsigned long long *dst = reinterpret_cast<unsigned long long *>(acc) + acc_index(k, slot >> 2, 0);
   if (__popc(leads) > kFlatGroups) {
     if (adds) {
 #pragma unroll 4
@@ -445,7 +452,7 @@ __device__ __forceinline__ void deposit_flat(long long *__restrict__ acc, unsign
         const int h = (int)(row[q] - kFixBiasBits), l = dens ? (int)(row_l[q] - kFixBiasBits) : 0;
         const long long sum = dens ? fix_join(h, l) : (long long)h;
         const int node = node_of[q];
-        if (node >= 0 && sum != 0) atomicAdd(dst + node, (unsigned long long)sum);
+        if (node >= 0 && sum != 0) atomicAdd(dst + ((size_t)node << k.acc_shift), (unsigned long long)sum);
       }
     }
   } else {
@@ -472,7 +479,7 @@ __device__ __forceinline__ void deposit_flat(long long *__restrict__ acc, unsign
       const unsigned bias = (unsigned)__popc(grp) * kFixBiasBits;
       const long long sum = dens ? fix_join((int)(hs - bias), (int)(ls - bias)) : (long long)(int)(hs - bias);
       const int node = node_of[lead];
-      if (adds && half == 0 && node >= 0 && sum != 0) atomicAdd(dst + node, (unsigned long long)sum);
+      if (adds && half == 0 && node >= 0 && sum != 0) atomicAdd(dst + ((size_t)node << k.acc_shift), (unsigned long long)sum);
     }
   }
   __syncwarp();
@@ -1723,6 +1730,8 @@ PartK make_k(const EcsCtx *ctx, double dt) {
   k.Nx = p.Nx; k.Ny = p.Ny; k.Nz = p.Nz;
   for (int d = 0; d < 3; d++) k.bc[d] = p.bc[d] == ECS_BC_PERIODIC ? ECS_BC_PERIODIC : ECS_BC_INJECT_REFLECT;
   k.ncell = ctx->ncell;
+  k.acc_shift = ecs_acc_interleaved(ctx) ? 2 : 0;
+  k.acc_field = ecs_acc_interleaved(ctx) ? 1 : ctx->ncell;
   k.dx = p.dx; k.dy = p.dy; k.dz = p.dz;
   k.lo[0] = p.x0; k.lo[1] = p.y0; k.lo[2] = p.z0;
   k.hi[0] = p.x1; k.hi[1] = p.y1; k.hi[2] = p.z1;
