@@ -317,6 +317,7 @@ int ecs_moments_upload(EcsCtx *ctx, const double *m) {
   ECS_CUDA(ctx, cudaFreeAsync(stage, ctx->stream));
   ECS_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   ctx->moments_ready = true;
+  ctx->mom_quanta = false;
   ctx->lhs_ready = false;
   return ECS_OK;
 }

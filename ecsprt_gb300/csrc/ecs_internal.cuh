@@ -189,6 +189,10 @@ struct EcsCtx {
   cudaEvent_t ev_solve[2] = {nullptr, nullptr};
   bool lhs_ready = false;
   bool moments_ready = false;
+  // the moments are a mixed deposit's, whole multiples of 2^-shift_n and
+  // 2^-shift_f: a choice of kernels, which check every value all the same (a
+  // graph captured under one answer is right under the other)
+  bool mom_quanta = false;
   bool eext_ready = false;          // difference numerators valid for the current phi
   int warm_start = 0;               // ecs_step starts the solve from the previous phi
 

@@ -91,29 +91,105 @@ __device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// ---- exact sums in integers ------------------------------------------------
+// FP64 adds issue at 1/64 of the FP32 rate.  Moments that come from the mixed
+// deposit are whole multiples of 2^-S, and sums and differences of a few of
+// them are exact in FP64 too; so they can be formed in int64 and converted
+// (exactly: below 2^53) on the integer units, with the same bits.  Any other
+// value takes the FP64 operations (all of them where S is kNoQuanta).
+constexpr int kNoQuanta = -1;
+constexpr int kQuantaBits = 50;  // |a| < 2^50: sums of up to four stay below 2^52
+// a = v 2^S; false unless that is whole and below 2^kQuantaBits.
+__device__ __forceinline__ bool quanta_of(double v, int S, long long &a) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const int r = 1075 - S - (int)((hi >> 20) & 0x7ffu);  // the significand's right shift
+  const unsigned mh = (hi & 0xfffffu) | 0x100000u;
+  const int tz = lo ? __ffs((int)lo) - 1 : 31 + __ffs((int)mh);
+  const unsigned long long m = (((unsigned long long)mh << 32) | lo) >> (r & 63);
+  const bool zero = (hi | lo) == 0u;  // -0 is left to the FP64 operations
+  a = zero ? 0 : ((int)hi < 0 ? -(long long)m : (long long)m);
+  return zero || (r >= 53 - kQuantaBits && r <= tz);
+}
+// a 2^-S for |a| < 2^53.
+__device__ __forceinline__ double from_quanta(long long a, int S) {
+  const unsigned long long m = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
+  const int lz = __clzll((long long)m);
+  // the leading bit adds one to the exponent field
+  const unsigned long long b = ((unsigned long long)(1023 + 62 - lz - S) << 52) + ((m << (lz & 63)) >> 11);
+  return m == 0 ? 0.0 : __longlong_as_double((long long)(b | ((unsigned long long)a & 0x8000000000000000ull)));
+}
+
 // 11 coefficients of a row in the order above, from the density at the
-// centre and its six face neighbours.  The roundings are written out, so that
+// centre and its six face neighbours: the sums and differences (RowSums),
+// then their products.  The roundings are written out, so that
 // every kernel forms the same bits however the compiler shares the products
 // of neighbouring rows.
+template <typename T>
+struct RowSums {
+  T dy, dx;                      // n(y+) - n(y-), n(x+) - n(x-)
+  T d6, d7, d8, d9;              // of the four off-diagonals
+  T xp, xm, yp, ym, zp, zm;      // face sums
+  T x2, y2, z2;                  // n+ + 2 n + n-
+};
+template <typename T>
+__device__ __forceinline__ void row11_products(const OpK &o, const RowSums<T> &u, T v[11]) {
+  T sxx, syy, szz, sod;
+  op_scales(o, sxx, syy, szz, sod);
+  const T ty = mul_r(sod, u.dy), tx = mul_r(sod, u.dx);
+  v[6] = mul_r(sod, u.d6);
+  v[7] = mul_r(sod, u.d7);
+  v[8] = mul_r(sod, u.d8);
+  v[9] = mul_r(sod, u.d9);
+  v[0] = fma_r(sxx, u.xp, ty);
+  v[1] = fma_r(sxx, u.xm, -ty);
+  v[2] = fma_r(syy, u.yp, -tx);
+  v[3] = fma_r(syy, u.ym, tx);
+  v[4] = mul_r(szz, u.zp);
+  v[5] = mul_r(szz, u.zm);
+  v[10] = -fma_r(szz, u.z2, fma_r(sxx, u.x2, mul_r(syy, u.y2)));
+}
 template <typename T>
 __device__ __forceinline__ void row11_vals(const OpK &o, T nijk, T nmjk, T npjk, T nimk, T nipk, T nijm, T nijp,
                                            T v[11]) {
   if (o.unit) nijk = nmjk = npjk = nimk = nipk = nijm = nijp = T(1);
-  T sxx, syy, szz, sod;
-  op_scales(o, sxx, syy, szz, sod);
-  const T ty = mul_r(sod, nipk - nimk), tx = mul_r(sod, npjk - nmjk);
-  v[6] = mul_r(sod, nipk - npjk);
-  v[7] = mul_r(sod, npjk - nimk);
-  v[8] = mul_r(sod, nmjk - nipk);
-  v[9] = mul_r(sod, nimk - nmjk);
-  v[0] = fma_r(sxx, npjk + nijk, ty);
-  v[1] = fma_r(sxx, nijk + nmjk, -ty);
-  v[2] = fma_r(syy, nipk + nijk, -tx);
-  v[3] = fma_r(syy, nijk + nimk, tx);
-  v[4] = mul_r(szz, nijp + nijk);
-  v[5] = mul_r(szz, nijk + nijm);
-  v[10] = -fma_r(szz, nijp + T(2) * nijk + nijm,
-                 fma_r(sxx, npjk + T(2) * nijk + nmjk, mul_r(syy, nipk + T(2) * nijk + nimk)));
+  RowSums<T> u;
+  u.dy = nipk - nimk;
+  u.dx = npjk - nmjk;
+  u.d6 = nipk - npjk;
+  u.d7 = npjk - nimk;
+  u.d8 = nmjk - nipk;
+  u.d9 = nimk - nmjk;
+  u.xp = npjk + nijk;
+  u.xm = nijk + nmjk;
+  u.yp = nipk + nijk;
+  u.ym = nijk + nimk;
+  u.zp = nijp + nijk;
+  u.zm = nijk + nijm;
+  u.x2 = npjk + T(2) * nijk + nmjk;
+  u.y2 = nipk + T(2) * nijk + nimk;
+  u.z2 = nijp + T(2) * nijk + nijm;
+  row11_products(o, u, v);
+}
+// The same from densities a 2^-S.
+__device__ __forceinline__ void row11_quanta(const OpK &o, int S, long long a, long long xm, long long xp, long long ym,
+                                             long long yp, long long zm, long long zp, double v[11]) {
+  RowSums<double> u;
+  u.dy = from_quanta(yp - ym, S);
+  u.dx = from_quanta(xp - xm, S);
+  u.d6 = from_quanta(yp - xp, S);
+  u.d7 = from_quanta(xp - ym, S);
+  u.d8 = from_quanta(xm - yp, S);
+  u.d9 = from_quanta(ym - xm, S);
+  u.xp = from_quanta(xp + a, S);
+  u.xm = from_quanta(a + xm, S);
+  u.yp = from_quanta(yp + a, S);
+  u.ym = from_quanta(a + ym, S);
+  u.zp = from_quanta(zp + a, S);
+  u.zm = from_quanta(a + zm, S);
+  u.x2 = from_quanta(xp + 2 * a + xm, S);
+  u.y2 = from_quanta(yp + 2 * a + ym, S);
+  u.z2 = from_quanta(zp + 2 * a + zm, S);
+  row11_products(o, u, v);
 }
 
 // 11 coefficients of row (k,j,i) in the order above.
@@ -241,6 +317,16 @@ __device__ __forceinline__ rd scale2(double h, int p, rd v) {
   if (p == kNoPow2 || (unsigned)(e - 128) > 1792u) return e == 0 && ((hi << 1) | __double2loint(v.v)) == 0 ? v : rd{h} * v;
   return rd{__hiloint2double(hi + p * (1 << 20), __double2loint(v.v))};
 }
+// b from the derivatives; with a background field also those of the density
+// along x and y (dndx(), dndy()).
+template <typename X, typename Y>
+__device__ __forceinline__ double rhs_combine(const RhsK &r, rd d2ndxx, rd d2ndyy, rd d2ndzz, rd dGxdx, rd dGydy,
+                                              rd dGzdz, X dndx, Y dndy) {
+  rd t = rd{r.cth} * ((d2ndxx + d2ndyy) + rd{r.opk2} * d2ndzz);
+  if (r.E0 != 0.0) t = (dndy() - rd{r.kappa} * dndx()) * rd{r.E0} + t;
+  const rd Gterm = rd{r.cG} * ((dGxdx + dGydy) + dGzdz);
+  return (rd{r.scale} * (t + Gterm)).v;
+}
 // b from the density at the node and its six neighbours and the flux at the
 // two neighbours along its own axis.
 __device__ __forceinline__ double rhs_value(const RhsK &r, rd nijk, rd npjk, rd nmjk, rd nipk, rd nimk, rd nijp, rd nijm,
@@ -252,11 +338,6 @@ __device__ __forceinline__ double rhs_value(const RhsK &r, rd nijk, rd npjk, rd 
   const rd dGxdx = scale2(r.hx, r.px, gxp - gxm);
   const rd dGydy = scale2(r.hy, r.py, gyp - gym);
   const rd dGzdz = scale2(r.hz, r.pz, gzp - gzm);
-  rd t = rd{r.cth} * ((d2ndxx + d2ndyy) + rd{r.opk2} * d2ndzz);
-  if (r.E0 != 0.0) {
-    const rd dndx = scale2(r.hx, r.px, npjk - nmjk), dndy = scale2(r.hy, r.py, nipk - nimk);
-    t = (dndy - rd{r.kappa} * dndx) * rd{r.E0} + t;
-  }
-  const rd Gterm = rd{r.cG} * ((dGxdx + dGydy) + dGzdz);
-  return (rd{r.scale} * (t + Gterm)).v;
+  return rhs_combine(r, d2ndxx, d2ndyy, d2ndzz, dGxdx, dGydy, dGzdz, [&] { return scale2(r.hx, r.px, npjk - nmjk); },
+                     [&] { return scale2(r.hy, r.py, nipk - nimk); });
 }
