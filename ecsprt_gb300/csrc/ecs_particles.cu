@@ -1234,17 +1234,24 @@ __global__ void __launch_bounds__(kBlock, 3) k_particles32(PartK k, int mode, in
 // words (bits(bias) + value; the bias of every contribution is taken out at
 // the flush from per-cell counts of the window's ions), and the window is
 // added to the global int64 accumulators once per chunk.  The chunk is split
-// into 32 consecutive segments, one per lane, so the lanes of a warp work on
-// different cells and rarely on the same node.  Ions outside the window
+// into 16 consecutive segments, one per pair of lanes, so that the pairs of a
+// warp work on different cells and rarely on the same node.  The lanes of a
+// pair take every other ion and so share the lines of the records they read
+// and write (a line's pass through the L1 data pipe an access); usually in the
+// same cell, they add its corners in opposite x order, which keeps them on
+// different nodes and, with the sorted segments at x = 0 and 2 (then 1 and 3),
+// the warp on 32 banks (128^3, 64 ions a cell: counting pass 3.62 -> 3.47 ms,
+// pass after a sort 3.28 -> 3.23; without collisions 3.47 -> 3.22 and 3.01 ->
+// 2.86).  Ions outside the window
 // (moved farther, or wrapped around a periodic edge) deposit straight into
 // the global accumulators.  The cells of the moved ions are counted the same
 // way when a sort follows.
 //
 // Loads: each thread's next ion record is loaded into registers (one
 // 256-bit load) while it works on the current one, so the memory latency
-// of a record overlaps the arithmetic of the previous ion.  The lanes' ions are
-// a segment apart, so a 4-byte permutation entry an ion would take a line of
-// its own in the L1 data pipe, the busiest unit, as a whole record does: the
+// of a record overlaps the arithmetic of the previous ion.  The pairs' ions are
+// a segment apart, so a 4-byte permutation entry would take a line of
+// its own in the L1 data pipe, the busiest unit, as two whole records do: the
 // chunk's entries are read as whole lines into shared memory first (128^3, 64
 // ions a cell: the pass after a sort 3.39 -> 3.29 ms; the sort keys written the
 // same way gave nothing).  All sums are exact integers, so the moments equal
@@ -1267,7 +1274,7 @@ __device__ __forceinline__ bool in_cell_window(int li, int lj, int lk) {
 __device__ __forceinline__ void tile_finish(const PartK &k, int mode, EcsDevStatus *st, IonState &q, int64_t ip,
                                             const TileCtx &tc, unsigned (*win)[kWPad], int *dcnt, int *wcnt,
                                             long long *__restrict__ acc, int32_t *__restrict__ count,
-                                            int32_t *__restrict__ keys, float4 *dst) {
+                                            int32_t *__restrict__ keys, float4 *dst, int flip) {
   ion_move(k, mode, st, q);
   const int li = q.i - tc.wx0, lj = q.j - tc.wy0, lk = q.kk - tc.wz0;
   const bool inwin = in_cell_window(li, lj, lk);
@@ -1286,11 +1293,14 @@ __device__ __forceinline__ void tile_finish(const PartK &k, int mode, EcsDevStat
     const float vxs = q.vx * s, vys = q.vy * s, vzs = q.vz * s;  // exact: s is a power of two
     if (inwin && fabsf(q.vx) <= k.vwinf && fabsf(q.vy) <= k.vwinf && fabsf(q.vz) <= k.vwinf) {
       const int n0 = lk * kSZ + lj * kSY + li;
+      // the two lanes of a pair start at opposite x corners
+      const int na = n0 + flip, nz = n0 + 1 - flip;
+      const float wa = flip ? wxh : wxl, wb = flip ? wxl : wxh;
       atomicAdd(&dcnt[(lk * kCY + lj) * kCX + li], 1);
 #pragma unroll
       for (int bc = 0; bc < 8; bc++) {
-        const float w = wzy[bc >> 1] * ((bc & 1) ? wxh : wxl);
-        const int nb = n0 + (bc >> 2) * kSZ + ((bc >> 1) & 1) * kSY + (bc & 1);
+        const float w = wzy[bc >> 1] * ((bc & 1) ? wb : wa);
+        const int nb = ((bc & 1) ? nz : na) + (bc >> 2) * kSZ + ((bc >> 1) & 1) * kSY;
         const float h = __fmaf_rn(w, k.fixn32.s_hi, kFixBias);
         const float r = __fmaf_rn(__fsub_rn(h, kFixBias), k.fixn32.s_back, w);
         atomicAdd(&win[0][nb], __float_as_uint(h));
@@ -1341,13 +1351,15 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM) k_tiles32(Part
     if (a == b) continue;
     for (int ca = a; ca < b; ca += kWindowMax) {
       const int L = min(kWindowMax, b - ca);
-      const int seg = (L + 31) >> 5;               // lane segment
-      const int sub = (seg + kTileThreads / 32 - 1) / (kTileThreads / 32);  // a warp's run inside each segment
-      // this thread's ions: m = 0 .. sub-1 at qi = lane * seg + warp * sub + m
-      const int qi0 = lane * seg + warp * sub;
-      const int mend = min(sub, min(seg - warp * sub, L - qi0));  // active iterations (may be <= 0)
+      // 16 segments of 2 seg ions, a pair of lanes each: the lanes of a pair take
+      // every other ion, a warp a run of each segment
+      const int seg = (L + 31) >> 5;
+      const int sub = (seg + kTileThreads / 32 - 1) / (kTileThreads / 32);
+      // this thread's ions: m = 0 .. mend-1 at qi0 + 2 m
+      const int qi0 = 2 * ((lane >> 1) * seg + warp * sub) + (lane & 1);
+      const int mend = min(sub, min(seg - warp * sub, (L - qi0 + 1) >> 1));  // may be <= 0
       auto src_pos = [&](int m) -> int64_t {
-        const int64_t ip = (int64_t)ca + qi0 + m;
+        const int64_t ip = (int64_t)ca + qi0 + 2 * m;
         return perm ? (int64_t)__ldg(perm + ip) : ip;
       };
       // the chunk's first record (and the permutation entry of the second)
@@ -1380,15 +1392,15 @@ __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM) k_tiles32(Part
         if (m + 1 < mend) {  // the next record, in flight while this one is worked on
           ld_record(src + 2 * sp_next, na, nb4);
           if (m + 2 < mend) {
-            const int e = qi0 + m + 2;
+            const int e = qi0 + 2 * m + 4;
             sp_next = perm ? (int64_t)entry[e + (e >> 6)] : (int64_t)ca + e;
           }
         }
         IonState q = ion_state(Ion{__float_as_int(ra.x), ra.y, ra.z, ra.w, rb.x, rb.y, rb.z, __float_as_int(rb.w)});
-        const int64_t ip = (int64_t)ca + qi0 + m;
+        const int64_t ip = (int64_t)ca + qi0 + 2 * m;
         if (mode & 1) ion_push(k, E, q, ewxy, ewz, tc.wx0, tc.wy0, tc.wz0);
         if (collide) collide_ion<float>(k, (uint32_t)q.id, kIdTag, (uint32_t)q.id, q.vx, q.vy, q.vz, nacc, nref);
-        tile_finish(k, mode, st, q, ip, tc, win, dcnt, wcnt, acc, count, keys, dst);
+        tile_finish(k, mode, st, q, ip, tc, win, dcnt, wcnt, acc, count, keys, dst, lane & 1);
       }
       __syncthreads();
       // window -> global accumulators
