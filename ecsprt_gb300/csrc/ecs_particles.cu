@@ -982,10 +982,11 @@ __device__ __forceinline__ int32_t ion_cell(const float4 *ions, int64_t ip) {
   return __ldcs(reinterpret_cast<const int32_t *>(ions) + 8 * ip);
 }
 // Sort key of cell (i, j, k): tile-major (tiles of ECS_TILE_X x ECS_TILE_Y x
-// ECS_TILE_Z cells, x fastest), then the cell within its tile.
-__device__ __forceinline__ int tile_key(int i, int j, int k, const TileG &t) {
-  const int tile = ((k / ECS_TILE_Z) * t.nty + j / ECS_TILE_Y) * t.ntx + i / ECS_TILE_X;
-  return tile * ECS_TILE_CELLS + ((k % ECS_TILE_Z) * ECS_TILE_Y + j % ECS_TILE_Y) * ECS_TILE_X + i % ECS_TILE_X;
+// ECS_TILE_Z cells, x fastest), then the cell within its tile.  Unsigned: a
+// signed division by a power of two costs two instructions more.
+__device__ __forceinline__ int tile_key(unsigned i, unsigned j, unsigned k, const TileG &t) {
+  const unsigned tile = ((k / ECS_TILE_Z) * t.nty + j / ECS_TILE_Y) * t.ntx + i / ECS_TILE_X;
+  return (int)(tile * ECS_TILE_CELLS + ((k % ECS_TILE_Z) * ECS_TILE_Y + j % ECS_TILE_Y) * ECS_TILE_X + i % ECS_TILE_X);
 }
 __device__ __forceinline__ int cell_key(int32_t c, const TileG &t) {
   return tile_key(c & 1023, (c >> 10) & 1023, (c >> 20) & 1023, t);
@@ -1148,24 +1149,32 @@ __device__ __forceinline__ void ion_push(const PartK &k, const float4 *__restric
 }
 
 // Move + boundary conditions (src/positions.c:436-472, src/boundaries.c:6-34)
-// in the pass's mode, then the velocity checks.
-__device__ __forceinline__ void ion_move(const PartK &k, int mode, EcsDevStatus *st, IonState &q) {
+// in the pass's mode, then the velocity checks.  Returns whether every
+// velocity component is within vwinf, which is below the bound vmaxf: one
+// test passes nearly every ion.
+__device__ __forceinline__ bool ion_move(const PartK &k, int mode, EcsDevStatus *st, IonState &q) {
   if (mode & 4) {
     q.i += advance(q.ox, q.vx * k.dtc[0]);
     q.j += advance(q.oy, q.vy * k.dtc[1]);
     q.kk += advance(q.oz, q.vz * k.dtc[2]);
-    const bool inside = bound_axis(k.bc[0], k.Nx, q.i, q.ox, q.vx) & bound_axis(k.bc[1], k.Ny, q.j, q.oy, q.vy) &
-                        bound_axis(k.bc[2], k.Nz, q.kk, q.oz, q.vz);
-    if (!inside) {
-      atomicOr(&st->flags, ECS_FLAG_RANGE);
-      q.i = min(max(q.i, 0), k.Nx - 1);
-      q.j = min(max(q.j, 0), k.Ny - 1);
-      q.kk = min(max(q.kk, 0), k.Nz - 1);
+    if ((unsigned)q.i >= (unsigned)k.Nx || (unsigned)q.j >= (unsigned)k.Ny || (unsigned)q.kk >= (unsigned)k.Nz) {
+      const bool inside = bound_axis(k.bc[0], k.Nx, q.i, q.ox, q.vx) & bound_axis(k.bc[1], k.Ny, q.j, q.oy, q.vy) &
+                          bound_axis(k.bc[2], k.Nz, q.kk, q.oz, q.vz);
+      if (!inside) {
+        atomicOr(&st->flags, ECS_FLAG_RANGE);
+        q.i = min(max(q.i, 0), k.Nx - 1);
+        q.j = min(max(q.j, 0), k.Ny - 1);
+        q.kk = min(max(q.kk, 0), k.Nz - 1);
+      }
     }
   }
-  if (!(isfinite(q.vx) && isfinite(q.vy) && isfinite(q.vz))) atomicOr(&st->flags, ECS_FLAG_NONFINITE);
-  if ((mode & 8) && !(fabsf(q.vx) <= k.vmaxf && fabsf(q.vy) <= k.vmaxf && fabsf(q.vz) <= k.vmaxf))
-    atomicOr(&st->flags, ECS_FLAG_RANGE);
+  const bool slow = fabsf(q.vx) <= k.vwinf && fabsf(q.vy) <= k.vwinf && fabsf(q.vz) <= k.vwinf;
+  if (!slow) {
+    if (!(isfinite(q.vx) && isfinite(q.vy) && isfinite(q.vz))) atomicOr(&st->flags, ECS_FLAG_NONFINITE);
+    if ((mode & 8) && !(fabsf(q.vx) <= k.vmaxf && fabsf(q.vy) <= k.vmaxf && fabsf(q.vz) <= k.vmaxf))
+      atomicOr(&st->flags, ECS_FLAG_RANGE);
+  }
+  return slow;
 }
 
 // Push, collisions (src/collisions.c:9-167; keyed by the ion's identity) and
@@ -1275,7 +1284,7 @@ __device__ __forceinline__ void tile_finish(const PartK &k, int mode, EcsDevStat
                                             const TileCtx &tc, unsigned (*win)[kWPad], int *dcnt, int *wcnt,
                                             long long *__restrict__ acc, int32_t *__restrict__ count,
                                             int32_t *__restrict__ keys, float4 *dst, int flip) {
-  ion_move(k, mode, st, q);
+  const bool slow = ion_move(k, mode, st, q);
   const int li = q.i - tc.wx0, lj = q.j - tc.wy0, lk = q.kk - tc.wz0;
   const bool inwin = in_cell_window(li, lj, lk);
   if (count) {
@@ -1291,7 +1300,7 @@ __device__ __forceinline__ void tile_finish(const PartK &k, int mode, EcsDevStat
     const float wzy[4] = {wzl * wyl, wzl * wyh, wzh * wyl, wzh * wyh};
     const float s = k.fixf32.s;
     const float vxs = q.vx * s, vys = q.vy * s, vzs = q.vz * s;  // exact: s is a power of two
-    if (inwin && fabsf(q.vx) <= k.vwinf && fabsf(q.vy) <= k.vwinf && fabsf(q.vz) <= k.vwinf) {
+    if (inwin && slow) {
       const int n0 = lk * kSZ + lj * kSY + li;
       // the two lanes of a pair start at opposite x corners
       const int na = n0 + flip, nz = n0 + 1 - flip;
