@@ -605,6 +605,65 @@ __global__ void k_restrict(GridG gf, GridG gc, const T *__restrict__ f, T *__res
   c[lin3(gc, I, J, K)] = s;
 }
 
+// The residual r = b - A x and its restriction in one kernel: a block forms the
+// residuals that its CX x CY x CZ coarse cells read in shared memory, those of
+// the rim again in its neighbours (405 for the 256 own ones; 306 for 256 when z
+// is not coarsened, Z = kZSemi, 153 for 128 in 2-D, kZFlat), and no residual goes
+// through memory.  A launch and a round trip less where latency is all that
+// counts (rule: residual_restrict_fused).  Same operations as k_apply and
+// k_restrict.  x and y are periodic and even on every level that is coarsened,
+// and so is z where it is coarsened.
+enum { kZFull = 0, kZSemi = 1, kZFlat = 2 };
+template <int Z>
+struct RrTile {
+  static constexpr int CX = Z == kZFull ? 4 : 8, CY = 4, CZ = Z == kZFlat ? 1 : 2;
+  static constexpr int FX = 2 * CX + 1, FY = 2 * CY + 1, FZ = Z == kZFull ? 2 * CZ + 1 : CZ;
+  static constexpr int kThreads = (FX * FY * FZ + 31) / 32 * 32;
+};
+template <typename T, int Z>
+__global__ void __launch_bounds__(RrTile<Z>::kThreads) k_residual_restrict(OpK o, GridG gc, const T *__restrict__ n,
+                                                                           const T *__restrict__ coef,
+                                                                           const T *__restrict__ x,
+                                                                           const T *__restrict__ b, T *__restrict__ c) {
+  ECS_PDL_ENTRY();
+  typedef RrTile<Z> R;
+  __shared__ T res[R::FZ][R::FY][R::FX];
+  const int I0 = blockIdx.x * R::CX, J0 = blockIdx.y * R::CY, K0 = blockIdx.z * R::CZ;
+  const int t = threadIdx.x, fx = t % R::FX, fy = t / R::FX % R::FY, fz = t / (R::FX * R::FY);
+  if (fz < R::FZ) {
+    int i = 2 * I0 - 1 + fx, j = 2 * J0 - 1 + fy, k = Z == kZFull ? 2 * K0 - 1 + fz : K0 + fz;
+    if (i < o.g.nx && j < o.g.ny && k < o.g.nz) {  // past the last coarse cell: not read
+      i = i < 0 ? o.g.nx - 1 : i;
+      j = j < 0 ? o.g.ny - 1 : j;
+      k = k < 0 ? o.g.nz - 1 : k;
+      const Nbr q = nbr_of(o.g, i, j, k);
+      T v[11], xe[11];
+      row_coef(o, n, coef, q, v);
+      row_x(x, q, xe);
+      T s = T(0);
+#pragma unroll
+      for (int e = 0; e < 11; e++) s += v[e] * xe[e];
+      res[fz][fy][fx] = b[q.c] - s;
+    }
+  }
+  __syncthreads();
+  const int ci = t % R::CX, cj = t / R::CX % R::CY, ck = t / (R::CX * R::CY);
+  if (ck >= R::CZ || I0 + ci >= gc.nx || J0 + cj >= gc.ny || K0 + ck >= gc.nz) return;
+  T s = T(0);
+#pragma unroll
+  for (int dk = Z == kZSemi ? 1 : 0; dk < (Z == kZSemi ? 2 : 3); dk++) {
+    const T wk = Z == kZSemi ? T(1) : (dk == 1 ? T(0.5) : T(0.25));
+    const int rk = Z == kZFull ? 2 * ck + dk : ck;  // flat: one plane is every neighbour along z
+#pragma unroll
+    for (int dj = 0; dj < 3; dj++) {
+      const T wj = dj == 1 ? T(0.5) : T(0.25);
+#pragma unroll
+      for (int di = 0; di < 3; di++) s += wk * wj * (di == 1 ? T(0.5) : T(0.25)) * res[rk][2 * cj + dj][2 * ci + di];
+    }
+  }
+  c[lin3(gc, I0 + ci, J0 + cj, K0 + ck)] = s;
+}
+
 // f += P c, trilinear: the coarse cells through the neighbour offsets of the
 // coarse cell (i/2, j/2, k/2); a term of the second cell along an axis is
 // added only for an odd index, x innermost, then y, then z.
@@ -733,6 +792,41 @@ int launch_restrict(EcsCtx *ctx, cudaStream_t s, const GridG &gf, const GridG &g
     ecs_launch_pdl(semi_z(gf, gc) ? k_restrict<T, true> : k_restrict<T, false>, blocks3(gc), threads3(), 0, s, gf, gc, f, c);
   ECS_LAUNCHED(ctx);
   return ECS_OK;
+}
+template <typename T, int Z>
+void launch_residual_restrict(EcsCtx *ctx, const OpK &o, const GridG &gc, const MgLevel<T> &L, const T *b, T *c) {
+  typedef RrTile<Z> R;
+  const dim3 g((unsigned)((gc.nx + R::CX - 1) / R::CX), (unsigned)((gc.ny + R::CY - 1) / R::CY),
+               (unsigned)((gc.nz + R::CZ - 1) / R::CZ));
+  ecs_launch_pdl(k_residual_restrict<T, Z>, g, R::kThreads, 0, ctx->stream, o, gc, (const T *)L.dens, (const T *)L.coef,
+                 (const T *)L.t, b, c);
+}
+// Levels whose residual and restriction are one kernel.  3-D: 32^3 solve 0.585
+// -> 0.561 ms, FP64 40 x 24 x 20 1.263 -> 1.216; on a 64^3 level the rim's second
+// residuals cost more than the launch (64^3 solve 0.744 with two kernels, 0.760
+// fused).  In 2-D the rim is smaller: 256^2 solve 0.748 -> 0.710 with the levels
+// below 256^2 and 2 to 3 % more with it.
+inline bool residual_restrict_fused(const GridG &g) {
+  return g.n < (g.nz == 1 ? (size_t)1 << 17 : (size_t)1 << 16);
+}
+// c = restriction of b - A L.t
+template <typename T>
+int residual_restrict(EcsCtx *ctx, MgLevel<T> &L, const OpK &o, const GridG &gc, const T *b, T *c) {
+  if (residual_restrict_fused(o.g)) {
+    if (o.g.nz == 1) launch_residual_restrict<T, kZFlat>(ctx, o, gc, L, b, c);
+    else if (semi_z(o.g, gc)) launch_residual_restrict<T, kZSemi>(ctx, o, gc, L, b, c);
+    else launch_residual_restrict<T, kZFull>(ctx, o, gc, L, b, c);
+    ECS_LAUNCHED(ctx);
+    return ECS_OK;
+  }
+  bool row4 = false;
+  if constexpr (sizeof(T) == 4) {
+    row4 = use_row4(o.g);
+    if (row4) ecs_launch_pdl(k_apply4, blocks4(o.g), threads4(L.nx), 0, ctx->stream, o, L.dens, L.t, b, L.r);
+  }
+  if (!row4) ecs_launch_pdl(k_apply<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, L.t, b, L.r, 1);
+  ECS_LAUNCHED(ctx);
+  return launch_restrict<T>(ctx, ctx->stream, o.g, gc, L.r, c);
 }
 template <typename T>
 int launch_prolong_add(EcsCtx *ctx, cudaStream_t s, const GridG &gf, const GridG &gc, const T *c, T *f) {
@@ -2507,15 +2601,8 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
   MgLevel<T> &C = mg.lv[l + 1];
   const OpK o = op_level(ctx, L);
   if ((rc = sweep<T>(ctx, L, b, nullptr, L.t))) return rc;
-  bool row4 = false;
-  if constexpr (sizeof(T) == 4) {
-    row4 = use_row4(o.g);
-    if (row4) ecs_launch_pdl(k_apply4, blocks4(o.g), threads4(L.nx), 0, ctx->stream, o, L.dens, L.t, b, L.r);
-  }
-  if (!row4) ecs_launch_pdl(k_apply<T>, blocks3(o.g), threads3(), 0, ctx->stream, o, L.dens, L.coef, L.t, b, L.r, 1);
-  ECS_LAUNCHED(ctx);
   const GridG gc = grid_level(ctx, C.nx, C.ny, C.nz);
-  if ((rc = launch_restrict<T>(ctx, ctx->stream, o.g, gc, L.r, C.b))) return rc;
+  if ((rc = residual_restrict<T>(ctx, L, o, gc, b, C.b))) return rc;
   if ((rc = vcycle<T>(ctx, l + 1, C.b, C.x))) return rc;
   if ((rc = launch_prolong_add<T>(ctx, ctx->stream, o.g, gc, C.x, L.t))) return rc;
   return sweep<T>(ctx, L, b, L.t, xout);
