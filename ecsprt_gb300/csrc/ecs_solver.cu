@@ -668,14 +668,9 @@ __global__ void __launch_bounds__(RrTile<Z>::kThreads) k_residual_restrict(OpK o
 // coarse cell (i/2, j/2, k/2); a term of the second cell along an axis is
 // added only for an odd index, x innermost, then y, then z.
 template <typename T, bool SEMI>
-__global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__restrict__ f) {
-  ECS_PDL_ENTRY();
-  int i, j, k;
-  if (!at3(gf.nx, gf.ny, i, j, k)) return;
+__device__ __forceinline__ T prolonged(const GridG &gc, const T *__restrict__ c, T old, int i, int j, int k) {
   const Nbr q = nbr_of(gc, i >> 1, j >> 1, SEMI ? k : k >> 1);
   const bool t[3] = {(i & 1) != 0, (j & 1) != 0, !SEMI && (k & 1)};
-  const unsigned e0 = lin3(gf, i, j, k);
-  const T old = f[e0];
   T v[8];
 #pragma unroll
   for (int e = 0; e < 8; e++) {
@@ -690,7 +685,15 @@ __global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__
     s = add ? s + v[e] : s;
   }
   const T wi = t[0] ? T(0.5) : T(1), wj = t[1] ? T(0.5) : T(1), wk = t[2] ? T(0.5) : T(1);
-  f[e0] = old + wi * wj * wk * s;
+  return old + wi * wj * wk * s;
+}
+template <typename T, bool SEMI>
+__global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__restrict__ f) {
+  ECS_PDL_ENTRY();
+  int i, j, k;
+  if (!at3(gf.nx, gf.ny, i, j, k)) return;
+  const unsigned e0 = lin3(gf, i, j, k);
+  f[e0] = prolonged<T, SEMI>(gc, c, f[e0], i, j, k);
 }
 
 // The same transfers in FP32, two coarse cells (four fine ones) a thread: the
@@ -793,6 +796,58 @@ int launch_restrict(EcsCtx *ctx, cudaStream_t s, const GridG &gf, const GridG &g
   ECS_LAUNCHED(ctx);
   return ECS_OK;
 }
+// FP32: x2 = x + P c and the right-hand side of the z-line systems, r = b - A_xy
+// x2, in one kernel: a block prolongs its TX x TY x TZ cells and the rim that
+// their rows read (432 values for 256 cells, 180 for 128 in 2-D) into shared
+// memory.  x2 is another array than x, whose rim the neighbouring blocks read.
+// Same operations as k_prolong_add and k_zline_rhs.
+template <bool FLAT>
+struct PrTile {
+  static constexpr int TX = 16, TY = FLAT ? 8 : 4, TZ = FLAT ? 1 : 4;
+  static constexpr int HX = TX + 2, HY = TY + 2;
+  static constexpr int kThreads = (HX * HY * TZ + 31) / 32 * 32;
+};
+template <bool SEMI, bool FLAT>
+__global__ void __launch_bounds__(PrTile<FLAT>::kThreads) k_prolong_rhs(OpK o, GridG gc, const float *__restrict__ n,
+                                                                        const float *__restrict__ b,
+                                                                        const float *__restrict__ c,
+                                                                        const float *__restrict__ x,
+                                                                        float *__restrict__ x2, float *__restrict__ r) {
+  ECS_PDL_ENTRY();
+  typedef PrTile<FLAT> R;
+  __shared__ float xs[R::TZ][R::HY][R::HX];
+  const int i0 = blockIdx.x * R::TX, j0 = blockIdx.y * R::TY, k0 = blockIdx.z * R::TZ;
+  const int t = threadIdx.x;
+  // this thread's own cell: its row is requested before the barrier
+  const int oi = t % R::TX, oj = t / R::TX % R::TY, ok = t / (R::TX * R::TY);
+  const bool own = ok < R::TZ && i0 + oi < o.g.nx && j0 + oj < o.g.ny && k0 + ok < o.g.nz;
+  float v[11], s = 0.f;
+  unsigned cell = 0;
+  if (own) {
+    const Nbr q = nbr_of(o.g, i0 + oi, j0 + oj, k0 + ok);
+    cell = q.c;
+    row11_n(n, o, q, v);
+    s = b[q.c];
+  }
+  const int hx = t % R::HX, hy = t / R::HX % R::HY, hz = t / (R::HX * R::HY);
+  const int i1 = i0 + hx - 1, j1 = j0 + hy - 1, k = k0 + hz;
+  if (hz < R::TZ && i1 <= o.g.nx && j1 <= o.g.ny && k < o.g.nz) {
+    const int i = i1 < 0 ? o.g.nx - 1 : (i1 == o.g.nx ? 0 : i1), j = j1 < 0 ? o.g.ny - 1 : (j1 == o.g.ny ? 0 : j1);
+    const unsigned e = lin3(o.g, i, j, k);
+    const float y = prolonged<float, SEMI>(gc, c, x[e], i, j, k);
+    xs[hz][hy][hx] = y;
+    if (hx >= 1 && hx <= R::TX && hy >= 1 && hy <= R::TY && i1 < o.g.nx && j1 < o.g.ny) x2[e] = y;
+  }
+  __syncthreads();
+  if (!own) return;
+#pragma unroll
+  for (int e = 0; e < 10; e++) {
+    if (e == 4 || e == 5) continue;
+    s -= v[e] * xs[ok][oj + 1 + off_j(e)][oi + 1 + off_i(e)];
+  }
+  r[cell] = s;
+}
+
 template <typename T, int Z>
 void launch_residual_restrict(EcsCtx *ctx, const OpK &o, const GridG &gc, const MgLevel<T> &L, const T *b, T *c) {
   typedef RrTile<Z> R;
@@ -2453,13 +2508,16 @@ int mg_setup(EcsCtx *ctx) {
   return ECS_OK;
 }
 
+// One sweep xn = xo + omega (...); `rhs_done`: its right-hand side is in L.r.
 template <typename T>
-int sweep(EcsCtx *ctx, MgLevel<T> &L, const T *b, const T *xo, T *xn) {
+int sweep(EcsCtx *ctx, MgLevel<T> &L, const T *b, const T *xo, T *xn, bool rhs_done = false) {
   const OpK o = op_level(ctx, L);
   const T *r = b;
   bool row4 = false;
   if constexpr (sizeof(T) == 4) row4 = use_row4(o.g);
-  if (xo && row4) {
+  if (rhs_done) {
+    r = L.r;
+  } else if (xo && row4) {
     if constexpr (sizeof(T) == 4)
       ecs_launch_pdl(k_zline_rhs4, blocks4(o.g), threads4(L.nx), 0, ctx->stream, o, L.dens, b, xo, L.r);
     ECS_LAUNCHED(ctx);
@@ -2559,12 +2617,28 @@ int launch_coarse_sweeps(EcsCtx *ctx, MgLevel<T> &L, const CoarseShape &cs, cons
   return ECS_OK;
 }
 
-// One V(1,1) cycle on level l: xout = M(l) b, zero initial guess.  Levels of
-// at most kSmallCells cells run as one single-block kernel.
+// x2 = L.x, the coarse correction xc added to L.t, and the right-hand side in L.r.
+int launch_prolong_rhs(EcsCtx *ctx, MgLevel<float> &L, const OpK &o, const GridG &gc, const float *b, const float *xc) {
+  const bool flat = o.g.nz == 1;
+  const auto kernel = flat ? k_prolong_rhs<false, true> : (semi_z(o.g, gc) ? k_prolong_rhs<true, false> : k_prolong_rhs<false, false>);
+  const int ty = flat ? PrTile<true>::TY : PrTile<false>::TY, tz = flat ? PrTile<true>::TZ : PrTile<false>::TZ;
+  const dim3 g((unsigned)((L.nx + PrTile<true>::TX - 1) / PrTile<true>::TX), (unsigned)((L.ny + ty - 1) / ty),
+               (unsigned)((L.nz + tz - 1) / tz));
+  ecs_launch_pdl(kernel, g, flat ? PrTile<true>::kThreads : PrTile<false>::kThreads, 0, ctx->stream, o, gc,
+                 (const float *)L.dens, b, xc, (const float *)L.t, L.x, L.r);
+  ECS_LAUNCHED(ctx);
+  return ECS_OK;
+}
+
+// One V(1,1) cycle on level l: *x = M(l) b (one of the level's arrays), zero
+// initial guess.  Levels of at most kSmallCells cells run as one single-block
+// kernel.
 template <typename T>
-int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
+int vcycle(EcsCtx *ctx, size_t l, const T *b, const T **x) {
   Multigrid<T> &mg = mg_of<T>(ctx);
   MgLevel<T> &L = mg.lv[l];
+  T *xout = L.x;
+  *x = xout;
   int rc;
   if (L.n <= kSmallCells && mg.lv.size() - l <= (size_t)kMaxSmall && small_layout<T>(mg, l, nullptr) <= kSmallSmem) {
     SmallCycle<T> sc;
@@ -2603,8 +2677,19 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, T *xout) {
   if ((rc = sweep<T>(ctx, L, b, nullptr, L.t))) return rc;
   const GridG gc = grid_level(ctx, C.nx, C.ny, C.nz);
   if ((rc = residual_restrict<T>(ctx, L, o, gc, b, C.b))) return rc;
-  if ((rc = vcycle<T>(ctx, l + 1, C.b, C.x))) return rc;
-  if ((rc = launch_prolong_add<T>(ctx, ctx->stream, o.g, gc, C.x, L.t))) return rc;
+  const T *xc = nullptr;
+  if ((rc = vcycle<T>(ctx, l + 1, C.b, &xc))) return rc;
+  // FP32: one kernel where the residual and its restriction are (32^3 solve 0.536
+  // -> 0.513 ms, 64^3 0.746 -> 0.738, 256^2 in 2-D 0.673 -> 0.656).  FP64 would lose
+  // (64^3 1.633 -> 1.642): the rim's sums cost its narrow pipe what the launch does.
+  if constexpr (sizeof(T) == 4) {
+    if (residual_restrict_fused(o.g)) {
+      if ((rc = launch_prolong_rhs(ctx, L, o, gc, b, xc))) return rc;
+      *x = L.t;
+      return sweep<T>(ctx, L, b, L.x, L.t, true);
+    }
+  }
+  if ((rc = launch_prolong_add<T>(ctx, ctx->stream, o.g, gc, xc, L.t))) return rc;
   return sweep<T>(ctx, L, b, L.t, xout);
 }
 
@@ -2662,19 +2747,20 @@ int cycle_step(EcsCtx *ctx, cudaGraphConditionalHandle cond, int use_graph) {
   const OpK o0 = op_level(ctx, L0);
   T *V = basis_v<T>(ctx), *Z = basis_z<T>(ctx);
   int rc;
-  // z = M v_j  (vin = L0.b holds v_j, the V-cycle writes L0.x)
-  if ((rc = vcycle<T>(ctx, 0, L0.b, L0.x))) return rc;
+  // z = M v_j  (vin = L0.b holds v_j)
+  const T *zv = nullptr;
+  if ((rc = vcycle<T>(ctx, 0, L0.b, &zv))) return rc;
   const double *mean = nullptr;
   if (fully_periodic(ctx)) {  // the operator's null space: project out the mean
-    if ((rc = launch_reduce<T, kRedMean>(ctx, n, L0.x, (double)n, &kd->mean, cond, use_graph))) return rc;
+    if ((rc = launch_reduce<T, kRedMean>(ctx, n, zv, (double)n, &kd->mean, cond, use_graph))) return rc;
     mean = &kd->mean;
   }
   bool row4 = false;
   if constexpr (sizeof(T) == 4) {
     row4 = use_row4(o0.g);
-    if (row4) ecs_launch_pdl(k_apply_dyn4, blocks4(o0.g), threads4(L0.nx), 0, ctx->stream, o0, L0.dens, L0.x, mean, Z, V, kd);
+    if (row4) ecs_launch_pdl(k_apply_dyn4, blocks4(o0.g), threads4(L0.nx), 0, ctx->stream, o0, L0.dens, zv, mean, Z, V, kd);
   }
-  if (!row4) ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.coef, L0.x, mean, Z, V, kd);
+  if (!row4) ecs_launch_pdl(k_apply_dyn<T>, blocks3(o0.g), threads3(), 0, ctx->stream, o0, L0.dens, L0.coef, zv, mean, Z, V, kd);
   ECS_LAUNCHED(ctx);
   // classical Gram-Schmidt, two passes
   constexpr int W = kPack<T>;
