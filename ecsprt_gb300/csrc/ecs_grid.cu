@@ -114,7 +114,7 @@ __global__ void k_rhs(GridG g, RhsK r, const double *__restrict__ mom, double *_
 }
 
 // The same with the differences of moments that are whole quanta (2^-Sn,
-// 2^-Sf) formed in integers: 21 -> 12 FP64 operations a cell.  Launched for
+// 2^-Sf) formed in integers: 25 -> 16 FP64 operations a cell.  Launched for
 // moments of a mixed deposit (EcsCtx::mom_quanta); a cell with any other value
 // takes the FP64 operations here too, at a loss (the whole ecs_rhs at 128^3,
 // dx = 1: 134 -> 111 us; moments without quanta 145 against k_rhs's 134).

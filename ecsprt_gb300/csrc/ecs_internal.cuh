@@ -361,9 +361,8 @@ int ecs_grid_clear_acc(EcsCtx *ctx);
 // by node (FP64, 2-D) keep a node's four side by side: 8 sectors an ion
 // instead of about 20 in 3-D (64^3 FP64, 64 ions a cell: 4.39 -> 4.36 ms, the
 // arithmetic bounds it), 4 instead of 7.5 in 2-D (256^2 mixed, 64 ions a cell:
-// 222 -> 175 us).  The tile kernel adds
-// rows of nodes a field at a time and keeps the fields apart (7 nodes of a
-// row in 2 to 3 sectors).
+// 222 -> 175 us).  The tile kernel adds rows of nodes a field at a time and
+// keeps the fields apart (7 nodes of a row in 2 to 3 sectors).
 static inline bool ecs_acc_interleaved(const EcsCtx *ctx) {
   return ctx->prec == ECS_PREC_FP64 || ctx->p.ndim == 2;
 }

@@ -417,10 +417,10 @@ __global__ void k_zline_rhs(OpK o, const T *__restrict__ n, const T *__restrict_
 // large ones.  FP32 with segments of 8 reads 5 words a cell instead of 9, and
 // its last operands are requested before the first barrier, so that two
 // memory latencies cover the solve.  Every thread runs the carried-value scan
-// over the segments itself (two barriers instead of four): 5.3 -> 3.9 us at
-// 32^3, 21.5 -> 15 us at 128^3.  Each phase keeps only the arrays that it
+// over the segments itself (two barriers instead of four): 9.1 -> 4.7 us at
+// 32^3, 21.4 -> 13.2 us at 128^3 (launch list).  Each phase keeps only the arrays that it
 // needs, so that two blocks of 512 threads fit an SM (with everything held
-// from the start, one block an SM: 7.5 against 6.4 us at 96^3).
+// from the start, one block an SM, it took 1.1 us more at 96^3).
 template <typename T, int S>
 __global__ void __launch_bounds__(32 * kMaxSeg, zl_stored<T>(S) ? 1 : 2)
     k_zline_seg(GridG g, ZCoup<T> zc, const T *__restrict__ n, ZlP<T> z, const T *__restrict__ r,
@@ -909,8 +909,8 @@ int launch_prolong_add(EcsCtx *ctx, cudaStream_t s, const GridG &gf, const GridG
 // and multiply-adds each.  The kernel runs each piece of its code once or a
 // few times per launch, so instruction fetch and the phases' latency bound it.
 // With the rows, wraps and index divisions redone in every phase and the
-// columns' recurrences through shared memory it took 24 us for 8^3 + 4^3 and
-// 70 us for a 6^3 coarsest level of 21 sweeps (FP32); 10 and 26 us in this
+// columns' recurrences through shared memory it took 27 us for 8^3 + 4^3 (FP64
+// 42) and 70 us for a 6^3 coarsest level of 21 sweeps; 11 (27) and 18 us in this
 // form.
 template <typename T>
 struct SmallLevel {
