@@ -81,7 +81,7 @@ __device__ __forceinline__ void row_coef(const OpK &o, const T *__restrict__ n, 
 template <typename T>
 __global__ void k_apply(OpK o, const T *__restrict__ n, const T *__restrict__ coef, const T *__restrict__ x,
                         const T *__restrict__ b, T *__restrict__ y, int mode) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const Nbr q = nbr_of(o.g, i, j, k);
@@ -273,7 +273,7 @@ static inline ZCoup<T> z_coupling(const OpK &o) {
 // z-line set-up.
 template <typename T>
 __global__ void k_zline_rows(OpK o, const T *__restrict__ n, T *__restrict__ dg) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const Nbr q = nbr_of(o.g, i, j, k);
@@ -287,7 +287,7 @@ __global__ void k_zline_rows(OpK o, const T *__restrict__ n, T *__restrict__ dg)
 template <typename T>
 __global__ void k_zline_setup(GridG g, ZCoup<T> zc, const T *__restrict__ n, const T *__restrict__ dg, ZlP<T> z,
                               int S) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   const int ncol = g.nx * g.ny;
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= ncol) return;
@@ -394,7 +394,7 @@ __global__ void k_zline_setup(GridG g, ZCoup<T> zc, const T *__restrict__ n, con
 template <typename T>
 __global__ void k_zline_rhs(OpK o, const T *__restrict__ n, const T *__restrict__ coef, const T *__restrict__ b,
                             const T *__restrict__ xo, T *__restrict__ r) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const Nbr q = nbr_of(o.g, i, j, k);
@@ -425,7 +425,7 @@ template <typename T, int S>
 __global__ void __launch_bounds__(32 * kMaxSeg, zl_stored<T>(S) ? 1 : 2)
     k_zline_seg(GridG g, ZCoup<T> zc, const T *__restrict__ n, ZlP<T> z, const T *__restrict__ r,
                 const T *__restrict__ xo, T *__restrict__ xn, T omega) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   constexpr bool kStored = zl_stored<T>(S);
   __shared__ T sA[kMaxSeg][33], sB[kMaxSeg][33], sC[kMaxSeg][33], sD[kMaxSeg][33];
   __shared__ T sLast[32];
@@ -576,7 +576,7 @@ __host__ __device__ __forceinline__ bool semi_z(const GridG &gf, const GridG &gc
 // offsets of the fine cell (2I, 2J, 2K) (or (2I, 2J, K)).
 template <typename T, bool SEMI>
 __global__ void k_restrict(GridG gf, GridG gc, const T *__restrict__ f, T *__restrict__ c) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   int I, J, K;
   if (!at3(gc.nx, gc.ny, I, J, K)) return;
   const Nbr q = nbr_of(gf, 2 * I, 2 * J, SEMI ? K : 2 * K);
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(RrTile<Z>::kThreads) k_residual_restrict(OpK o
                                                                            const T *__restrict__ coef,
                                                                            const T *__restrict__ x,
                                                                            const T *__restrict__ b, T *__restrict__ c) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   typedef RrTile<Z> R;
   __shared__ T res[R::FZ][R::FY][R::FX];
   const int I0 = blockIdx.x * R::CX, J0 = blockIdx.y * R::CY, K0 = blockIdx.z * R::CZ;
@@ -689,7 +689,7 @@ __device__ __forceinline__ T prolonged(const GridG &gc, const T *__restrict__ c,
 }
 template <typename T, bool SEMI>
 __global__ void k_prolong_add(GridG gf, GridG gc, const T *__restrict__ c, T *__restrict__ f) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   int i, j, k;
   if (!at3(gf.nx, gf.ny, i, j, k)) return;
   const unsigned e0 = lin3(gf, i, j, k);
@@ -1088,7 +1088,7 @@ __device__ __noinline__ void blk_sweep(const SmallLevel<T> &L, int ints_off, int
 template <typename T>
 __global__ void __launch_bounds__(kSmallThreads) k_vcycle_small(SmallCycle<T> sc, const T *__restrict__ b_in,
                                                                 T *__restrict__ x_out, int coarse_sweeps, T omega) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   extern __shared__ unsigned char small_smem[];
   T *sm = reinterpret_cast<T *>(small_smem);
   unsigned *ints = reinterpret_cast<unsigned *>(sm + sc.ints);
@@ -1248,7 +1248,7 @@ template <typename T, int EW, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1)
     k_coarse_sweeps(OpK o, ZCoup<T> zc, const T *__restrict__ dens, ZlP<T> z, const T *__restrict__ b,
                     T *__restrict__ xout, int rows, int sweeps, T omega) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   constexpr int S = kClusterSeg;
   extern __shared__ __align__(16) unsigned char coarse_smem[];
   cg::cluster_group cl = cg::this_cluster();
@@ -1474,7 +1474,7 @@ __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k)
 template <typename T, int ROWS, int TPR, bool SWAP>
 __global__ void __launch_bounds__(ROWS *TPR) k_coarse_inverse(OpK o, const T *__restrict__ dens, int regularize,
                                                               T *__restrict__ invT) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   constexpr int COLS = ROWS / TPR, RPL = ROWS / 32;  // columns a thread, rows a lane (pivot search)
   __shared__ T colbuf[2][ROWS];
   __shared__ T prow[2][ROWS];
@@ -1746,7 +1746,7 @@ __device__ __forceinline__ void slot_totals(const double *partial, int ns, int n
 // v -= value[0]
 template <typename T>
 __global__ void k_sub_value(size_t n, T *__restrict__ v, const double *__restrict__ value) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   const double m = value[0];
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
     v[e] = (T)((double)v[e] - m);
@@ -1819,7 +1819,7 @@ __device__ __forceinline__ void ld_half(const T *__restrict__ V, size_t n, int v
 template <typename T, int W>
 __global__ void __launch_bounds__(kB, 4) k_dots1(size_t n, const T *__restrict__ V, KrylovDev *__restrict__ kd,
                                                  double *__restrict__ partial) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   const int nv = kd->j + 1;
   const T *w = V + (size_t)nv * n;
   const size_t nw = n / W, stride = (size_t)gridDim.x * blockDim.x;
@@ -1938,7 +1938,7 @@ __device__ __noinline__ void arnoldi_rotate(KrylovDev *kd, cudaGraphConditionalH
 template <typename T, int W>
 __global__ void __launch_bounds__(kB, 4) k_orth1_dots2(size_t n, T *__restrict__ V, KrylovDev *__restrict__ kd,
                                                        double *__restrict__ partial) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   __shared__ T hs[kSlots];
   const int nv = kd->j + 1, nslot = nv + 1;
   if (threadIdx.x < kSlots) hs[threadIdx.x] = (int)threadIdx.x < nv ? (T)kd->h1[threadIdx.x] : T(0);
@@ -1993,7 +1993,7 @@ __global__ void __launch_bounds__(kB, 4) k_orth1_dots2(size_t n, T *__restrict__
 template <typename T, int W>
 __global__ void k_orth2_scale(size_t n, T *__restrict__ V, KrylovDev *kd, T *__restrict__ vin,
                               cudaGraphConditionalHandle cond, int use_graph) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   if (blockIdx.x == 0) {
     arnoldi_rotate(kd, cond, use_graph);
     return;
@@ -2033,7 +2033,7 @@ template <typename T>
 __global__ void k_apply_dyn(OpK o, const T *__restrict__ n, const T *__restrict__ coef, const T *__restrict__ x,
                             const double *__restrict__ mean, T *__restrict__ Z, T *__restrict__ V,
                             const KrylovDev *__restrict__ kd) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   int i, j, k;
   if (!at3(o.g.nx, o.g.ny, i, j, k)) return;
   const int jj = kd->j;
@@ -2128,7 +2128,7 @@ template <typename T, int W, int M>
 __global__ void __launch_bounds__(kB) k_reduce(size_t nw, const T *__restrict__ v, double *__restrict__ partial,
                                                double div, double *out, KrylovDev *kd,
                                                cudaGraphConditionalHandle cond, int use_graph, RefineArgs ra) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   KSum<T> acc;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nw; e += (size_t)gridDim.x * blockDim.x) {
     const Pack<T, W> p = ld_pack<T, W>(v + e * W);
@@ -2198,7 +2198,7 @@ __global__ void __launch_bounds__(kB) k_scale_beta(size_t nw, const double *__re
 template <typename T>
 __global__ void k_cycle_start(size_t n, const T *__restrict__ b, T *__restrict__ V, T *__restrict__ vin,
                               const KrylovDev *__restrict__ kd) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   const T sc = (T)kd->inv_scale;
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const T v = b[e] * sc;
@@ -2214,7 +2214,7 @@ template <typename T, int W, bool MEAN>
 __global__ void __launch_bounds__(kB) k_cycle_finish(size_t nw, size_t n, const T *__restrict__ Z, KrylovDev *kd,
                                                      const double *__restrict__ scale, double *__restrict__ phi,
                                                      double *__restrict__ partial, double *mean) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   __shared__ T y[kKrylovMax];
   const int nj = kd->nits;
   const double a = scale ? scale[0] : 1.0;
@@ -2390,7 +2390,7 @@ constexpr T kOmega() { return T(0.8); }
 // weighting) and the z-line factorisation of every level.
 template <typename T>
 __global__ void k_density_in(size_t n, const double *__restrict__ mom, T *__restrict__ d) {
-  ECS_PDL_ENTRY();
+  ECS_PDL_ENTRY_FOR(T);
   for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
     d[e] = (T)mom[e];
 }
