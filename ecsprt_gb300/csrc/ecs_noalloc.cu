@@ -19,9 +19,12 @@
 // accepted.
 //
 // Every call shares the array: each call writes every partial and the mean
-// before it reads them, so nothing from an earlier call is used, but two
-// calls that overlap on the GPU (different streams without ordering) race on
-// it.
+// before it reads them, and the block that finishes last puts the completion
+// count back to 0, so a call needs nothing of the calls before it.  Two calls
+// that overlap on the GPU (different streams without ordering) race on it:
+// either may then subtract a mean of mixed partials or an earlier call's mean.
+// A call ordered after both is right again (k_sub_mean_noalloc clears the
+// count).
 //
 // The array's device address is looked up once per device, the first time a
 // call runs with that device current, and cached for the life of the
@@ -131,11 +134,14 @@ __global__ void __launch_bounds__(kThreads) k_rhs_noalloc(RhsNoAllocK g, int cel
   double t = 0.0;
   for (unsigned q = threadIdx.x; q < gridDim.x; q += kThreads) t += __ldcg(partials + q);
   const double u = block_sum(t);
-  if (threadIdx.x == 0) partials[ECS_NOALLOC_RHS_MAX_BLOCKS] = u / (double)g.n;
+  if (threadIdx.x == 0) {
+    partials[ECS_NOALLOC_RHS_MAX_BLOCKS] = u / (double)g.n;
+    *done = 0u;  // here, not in the next kernel alone: that launch can fail
+  }
 }
 
-// b -= mean.  Also puts the completion count back to 0, whatever a call that
-// overlapped this one has left there, so that the next call starts clean.
+// b -= mean.  Also clears the completion count, whatever calls that overlapped
+// this one have left there, so that the next call starts clean.
 __global__ void __launch_bounds__(kThreads) k_sub_mean_noalloc(size_t n, double *__restrict__ b, double *partials) {
   if (blockIdx.x == 0 && threadIdx.x == 0)
     *reinterpret_cast<unsigned int *>(partials + ECS_NOALLOC_RHS_MAX_BLOCKS + 1) = 0u;

@@ -212,8 +212,9 @@ int ecs_lhs_apply_host(EcsCtx *ctx, const double *x, double *y);
    (cudaGetSymbolAddress) and keeps it for the life of the process; make
    that first call before any stream capture, and do not call it on a device
    after cudaDeviceReset.  Every call shares the one scratch array: calls
-   that overlap on the GPU (unordered streams) race.  Errors are reported by
-   ecs_last_error(NULL). */
+   that overlap on the GPU (unordered streams) race, and their results may
+   have any mean, one of an earlier call's among them; calls ordered after
+   them are right again.  Errors are reported by ecs_last_error(NULL). */
 int ecs_rhs_noalloc(const EcsParams *params, const double *d_moments, double *d_rhs, void *stream);
 
 /* One time step of src/pic.c:244-258: push, collide (if mn > 0), move + BC,
