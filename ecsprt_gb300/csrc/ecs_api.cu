@@ -114,31 +114,30 @@ int64_t ecs_ctx_device_bytes(const EcsParams *p, int precision, int64_t cap) {
   const int64_t n = (int64_t)p->Nx * p->Ny * p->Nz;
   const int64_t ne = (int64_t)(p->Nx + 1) * (p->Ny + 1) * (p->Nz + 1);
   const int64_t m = 30;  // Krylov basis vectors (FGMRES restart)
-  const int64_t t = precision == ECS_PREC_FP64 ? 8 : 4;  // solver arithmetic
-  int64_t b = 0;
-  b += n * 8 * (1 + 4 + 1) + n * 8 * 4;  // phi, moments, rhs; fixed-point accumulators
-  b += n * 8 + (m + 2) * 4096 * 8;       // FP64 residual, reductions
-  if (p->lhs_type != ECS_LHS_IDENTITY) b += n * 8 * 11;  // FP64 row coefficients of the residuals
-  // multigrid: 7 cell arrays (11 in FP64 and for columns of more than 128
-  // cells) and 2 plane arrays a level, levels summing to at most 8/7 of the
-  // finest; the coarsest level's inverse (<= 128 cells)
-  b += (n * (precision == ECS_PREC_FP64 || p->Nz > 128 ? 11 : 7) + n / 4) * t * 8 / 7 + 128 * 128 * t;
-  if (precision == ECS_PREC_FP64) {
-    // FP64 row coefficients of the coarser levels (every plane kept: a third of the finest's)
-    if (p->lhs_type != ECS_LHS_IDENTITY) b += n * 8 * 11 * (p->bc[2] == ECS_BC_PERIODIC && p->ndim == 3 ? 1 : 3) / 7;
-    b += (2 * m + 1) * n * 8;  // Krylov bases V, Z
-    b += cap * 48 + ne * 32;   // ions (6 FP64), E numerators
-  } else {
-    b += (2 * m + 2) * n * 4;  // Krylov bases V, Z, the normalised residual
-    b += cap * 72 + ne * 16;   // ions (two 32-byte record buffers, sort keys, permutation), E numerators
-    const int64_t keys = (int64_t)((p->Nx + ECS_TILE_X - 1) / ECS_TILE_X) * ((p->Ny + ECS_TILE_Y - 1) / ECS_TILE_Y) *
-                         ((p->Nz + ECS_TILE_Z - 1) / ECS_TILE_Z) * ECS_TILE_CELLS;
-    b += keys * 4 * 2 + keys / 1024 * 4;  // sort counts and offsets
+  const bool fp64 = precision == ECS_PREC_FP64;
+  DeviceBytes b;
+  for (int f : {1, 4, 4, 1, 1}) b.add(n * 8 * f);  // phi, moments, fixed-point accumulators, rhs, FP64 residual
+  b.add((m + 2) * 4096 * 8);                       // reductions
+  if (p->lhs_type != ECS_LHS_IDENTITY) {
+    b.add(n * 8 * 11);  // FP64 row coefficients of the residuals
+    ecs_mg_bytes(*p, precision, b);
   }
-  if (cap > 0) b += (2 + EcsCtx::kStageDn) * 2 * ecs_stage_stride(ecs_stage_ions(cap)) * 8;  // host-transfer staging
-  // allocation rounding (about 40 allocations) and instantiated CUDA graphs
-  b += (int64_t)8 << 20;
-  return b;
+  b.add((m + 1) * n * (fp64 ? 8 : 4));               // Krylov basis V
+  b.add((fp64 ? m * 8 : (m + 1) * 4) * n);           // Z; mixed: and the normalised residual
+  b.add(ne * (fp64 ? 32 : 16));                      // E numerators
+  int64_t ions = cap * (fp64 ? 48 : 72);  // 6 FP64; mixed: two 32-byte record buffers, sort keys, permutation
+  if (!fp64) {
+    const int64_t tiles = (int64_t)((p->Nx + ECS_TILE_X - 1) / ECS_TILE_X) * ((p->Ny + ECS_TILE_Y - 1) / ECS_TILE_Y) *
+                          ((p->Nz + ECS_TILE_Z - 1) / ECS_TILE_Z);
+    for (int q = 0; q < 2; q++) b.add(tiles * ECS_TILE_CELLS * 4);  // sort counts and offsets
+    b.add((2 * tiles + 1) * 4);                                     // tile tables of ecs_step_host
+  }
+  if (cap > 0) ions += (2 + EcsCtx::kStageDn) * 2 * ecs_stage_stride(ecs_stage_ions(cap)) * 8;  // host-transfer staging
+  // the pages of the ion arrays (9 at most, about a MiB each), small control
+  // blocks, instantiated CUDA graphs.  Contexts of 16^3 to 256 x 256 x 128, without
+  // ions and with 4 a cell, held 2 to 22 MiB less than this says; FP64 and 2-D ones
+  // with ions 15 to 154 MiB, the staging of ecs_step_host that they do without.
+  return b.total + ions + ((int64_t)16 << 20);
 }
 
 int ecs_ctx_create(const EcsParams *params, int precision, int64_t np_capacity, void *stream, EcsCtx **out) {

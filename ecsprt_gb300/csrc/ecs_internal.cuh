@@ -66,6 +66,12 @@ struct MgLevel {
   T *zl_a0g = nullptr, *zl_qden = nullptr;  // per-column Sherman-Morrison scalars
 };
 
+// Sizes of a multigrid level.
+struct MgDims {
+  int nx, ny, nz;
+  double hx, hy, hz;
+};
+
 // Thread-block cluster that runs the sweeps of the coarsest level (ctas = 0:
 // none).
 struct CoarseShape {
@@ -378,6 +384,17 @@ int ecs_grid_clear_acc(EcsCtx *ctx);
 static inline bool ecs_acc_interleaved(const EcsCtx *ctx) {
   return ctx->prec == ECS_PREC_FP64 || ctx->p.ndim == 2;
 }
+// Device bytes of a set of cudaMalloc arrays: each of more than 1 MiB takes
+// whole 2 MiB pages, smaller ones share them (512-byte steps).  A 100 x 72 x 50
+// context held 18 MiB more than the sum of its arrays.
+struct DeviceBytes {
+  int64_t total = 0;
+  void add(int64_t bytes) {
+    const int64_t step = bytes > ((int64_t)1 << 20) ? (int64_t)2 << 20 : 512;
+    total += (bytes + step - 1) / step * step;
+  }
+};
+void ecs_mg_bytes(const EcsParams &p, int precision, DeviceBytes &b);  // the multigrid hierarchy's arrays
 int ecs_solver_alloc(EcsCtx *ctx);       // reductions, Krylov bases, control block
 int ecs_solver_setup(EcsCtx *ctx);       // multigrid hierarchy from the density
 // setup = 1: compute the RHS and set up the operator first (the step's field

@@ -2308,42 +2308,25 @@ Multigrid<float> &mg_of<float>(EcsCtx *ctx) { return ctx->mg32; }
 template <typename T>
 int coarse_attrs(EcsCtx *ctx, CoarseShape &cs);
 
-template <typename T>
-int mg_alloc(EcsCtx *ctx) {
-  Multigrid<T> &mg = mg_of<T>(ctx);
-  if (mg.built) return ECS_OK;
-  int nx = ctx->p.Nx, ny = ctx->p.Ny, nz = ctx->p.Nz;
-  double hx = ctx->p.dx, hy = ctx->p.dy, hz = ctx->p.dz;
+// The levels of the hierarchy, finest first.
+std::vector<MgDims> mg_dims(const EcsParams &p) {
+  std::vector<MgDims> lv;
+  int nx = p.Nx, ny = p.Ny, nz = p.Nz;
+  double hx = p.dx, hy = p.dy, hz = p.dz;
   for (;;) {
-    MgLevel<T> L;
-    L.nx = nx; L.ny = ny; L.nz = nz;
-    L.n = (size_t)nx * ny * nz;
-    L.hx = hx; L.hy = hy; L.hz = hz;
-    T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_minv, &L.zl_q};
-    for (auto a : arr) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
-    if constexpr (sizeof(T) == 8) {
-      if (mg.lv.empty()) L.coef = ctx->coef64;
-      else ECS_CUDA(ctx, cudaMalloc((void **)&L.coef, 11 * L.n * sizeof(T)));
-    }
-    if (zl_stored<T>(seg_len<T>(nz))) {
-      T **more[] = {&L.zl_a, &L.zl_cp, &L.zl_fb, &L.zl_bb};
-      for (auto a : more) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
-    }
-    ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_a0g, (size_t)nx * ny * sizeof(T)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_qden, (size_t)nx * ny * sizeof(T)));
-    mg.lv.push_back(L);
+    lv.push_back({nx, ny, nz, hx, hy, hz});
     // A 2-D grid (nz = 1) coarsens in x and y only.  So does a grid with a
     // reflecting z: its ghost planes one spacing outside the walls do not
     // nest under z coarsening, and the z-line smoother resolves z on every
     // level, so the levels keep all planes down to one column (x y = 1 x 1,
     // whose Nz cells the coarsest inverse solves directly).
     const bool flat = nz == 1;
-    const bool semi = !flat && ctx->p.bc[2] != ECS_BC_PERIODIC;
+    const bool semi = !flat && p.bc[2] != ECS_BC_PERIODIC;
     if (semi) {
-      if (nx % 2 || ny % 2 || mg.lv.size() >= 12) break;
+      if (nx % 2 || ny % 2 || lv.size() >= 12) break;
     } else {
       bool even = (nx % 2 == 0) && (ny % 2 == 0) && (flat || nz % 2 == 0);
-      if (!even || std::min(nx, std::min(ny, flat ? nx : nz)) < 8 || mg.lv.size() >= 12) break;
+      if (!even || std::min(nx, std::min(ny, flat ? nx : nz)) < 8 || lv.size() >= 12) break;
     }
     nx /= 2; ny /= 2;
     hx *= 2; hy *= 2;
@@ -2351,6 +2334,47 @@ int mg_alloc(EcsCtx *ctx) {
       nz /= 2;
       hz *= 2;
     }
+  }
+  return lv;
+}
+
+// What mg_alloc allocates for these levels.
+template <typename T>
+void mg_bytes(const std::vector<MgDims> &lv, DeviceBytes &b) {
+  for (size_t l = 0; l < lv.size(); l++) {
+    const int64_t plane = (int64_t)lv[l].nx * lv[l].ny, n = plane * lv[l].nz;
+    for (int q = 0; q < (zl_stored<T>(seg_len<T>(lv[l].nz)) ? 11 : 7); q++) b.add(n * sizeof(T));
+    for (int q = 0; q < 2; q++) b.add(plane * sizeof(T));
+    if (sizeof(T) == 8 && l > 0) b.add(11 * n * sizeof(T));
+  }
+  const MgDims &c = lv.back();
+  const int64_t nc = (int64_t)c.nx * c.ny * c.nz;
+  if (nc <= kDirectMax) b.add(nc * nc * sizeof(T));
+}
+
+// An array added here goes into mg_bytes too.
+template <typename T>
+int mg_alloc(EcsCtx *ctx) {
+  Multigrid<T> &mg = mg_of<T>(ctx);
+  if (mg.built) return ECS_OK;
+  for (const MgDims &d : mg_dims(ctx->p)) {
+    MgLevel<T> L;
+    L.nx = d.nx; L.ny = d.ny; L.nz = d.nz;
+    L.n = (size_t)d.nx * d.ny * d.nz;
+    L.hx = d.hx; L.hy = d.hy; L.hz = d.hz;
+    T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_minv, &L.zl_q};
+    for (auto a : arr) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
+    if constexpr (sizeof(T) == 8) {
+      if (mg.lv.empty()) L.coef = ctx->coef64;
+      else ECS_CUDA(ctx, cudaMalloc((void **)&L.coef, 11 * L.n * sizeof(T)));
+    }
+    if (zl_stored<T>(seg_len<T>(L.nz))) {
+      T **more[] = {&L.zl_a, &L.zl_cp, &L.zl_fb, &L.zl_bb};
+      for (auto a : more) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
+    }
+    ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_a0g, (size_t)L.nx * L.ny * sizeof(T)));
+    ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_qden, (size_t)L.nx * L.ny * sizeof(T)));
+    mg.lv.push_back(L);
   }
   const size_t nc = mg.lv.back().n;
   if (nc <= (size_t)kDirectMax) {
@@ -3212,6 +3236,12 @@ bool host_pinned(const void *p) {
 // ============================================================================
 // entry points used by ecs_api.cu and ecs_grid.cu
 // ============================================================================
+void ecs_mg_bytes(const EcsParams &p, int precision, DeviceBytes &b) {
+  const std::vector<MgDims> lv = mg_dims(p);
+  if (precision == ECS_PREC_FP64) mg_bytes<double>(lv, b);
+  else mg_bytes<float>(lv, b);
+}
+
 int ecs_solver_alloc(EcsCtx *ctx) {
   size_t n = ctx->ncell;
   int m = ctx->krylov_m;
