@@ -1966,9 +1966,20 @@ __global__ void k_init_ions(InitK ik, PartK k, int64_t n, int fp64, float4 *__re
 // ============================================================================
 // entry points used by ecs_api.cu
 // ============================================================================
+// Dynamic shared memory of the order-free particle kernels.
+static constexpr size_t kShm32 = (size_t)(kBlock / 32) * kTileBytes;
+static constexpr size_t kShm64 = (size_t)(kBlock64 / 32) * (kTileBytes + kQueueBytes);
+
 int ecs_particles_alloc(EcsCtx *ctx) {
   size_t n = (size_t)ctx->cap;
   if (n == 0) n = 1;
+  // above 48 KB: asked for on the device of every context (the attribute is
+  // a device's, so a flag for the process would leave the others out)
+  if (ctx->prec == ECS_PREC_FP64)
+    ECS_CUDA(ctx, cudaFuncSetAttribute(k_particles64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShm64));
+  else
+    ECS_CUDA(ctx, cudaFuncSetAttribute(ctx->p.ndim == 2 ? k_particles32<true> : k_particles32<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kShm32));
   if (ctx->prec == ECS_PREC_FP64) {
     double **arr[6] = {&ctx->px, &ctx->py, &ctx->pz, &ctx->vx, &ctx->vy, &ctx->vz};
     for (auto a : arr) ECS_CUDA(ctx, cudaMalloc((void **)a, n * sizeof(double)));
@@ -2278,15 +2289,6 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
   int rc = pass_params(ctx, dt, mode, k);
   if (rc) return rc;
   ctx->pgen++;
-  const size_t shm = (size_t)(kBlock / 32) * kTileBytes;
-  const size_t shm64 = (size_t)(kBlock64 / 32) * (kTileBytes + kQueueBytes);
-  static std::atomic<bool> attr_set{false};
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_particles64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm64);
-    cudaFuncSetAttribute(k_particles32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    cudaFuncSetAttribute(k_particles32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    attr_set = true;
-  }
   int32_t *count = nullptr;
   if (count_for_sort && ctx->prec == ECS_PREC_MIXED) {
     ECS_CUDA(ctx, cudaMemsetAsync(ctx->sort_count, 0, ctx->nkeys * sizeof(int32_t), ctx->stream));
@@ -2297,7 +2299,7 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
   if (ctx->prec == ECS_PREC_FP64) {
     // the blocks that fit the SMs at once
     g = (unsigned)std::min<int64_t>((ctx->np + kBlock64 - 1) / kBlock64, (int64_t)ctx->nsm * kBlocks64);
-    k_particles64<<<g, kBlock64, shm64, ctx->stream>>>(k, mode, ctx->np, ctx->px, ctx->py, ctx->pz, ctx->vx,
+    k_particles64<<<g, kBlock64, kShm64, ctx->stream>>>(k, mode, ctx->np, ctx->px, ctx->py, ctx->pz, ctx->vx,
                                                 ctx->vy, ctx->vz, ctx->eext64, ctx->acc, ctx->dstat);
   } else if (ctx->tiles_valid) {
     // after an index sort the pass reads the records through the permutation
@@ -2317,10 +2319,10 @@ static int launch_particles(EcsCtx *ctx, double dt, int mode, bool count_for_sor
     rc = settle_order(ctx);
     if (rc) return rc;
     if (k.ndim == 2)
-      k_particles32<true><<<g, kBlock, shm, ctx->stream>>>(
+      k_particles32<true><<<g, kBlock, kShm32, ctx->stream>>>(
           k, mode, ctx->np, ctx->ions[ctx->cur], ctx->eext32, ctx->acc, count, ctx->sort_keys, ctx->dstat);
     else
-      k_particles32<false><<<g, kBlock, shm, ctx->stream>>>(k, mode, ctx->np, ctx->ions[ctx->cur], ctx->eext32,
+      k_particles32<false><<<g, kBlock, kShm32, ctx->stream>>>(k, mode, ctx->np, ctx->ions[ctx->cur], ctx->eext32,
                                                             ctx->acc, count, ctx->sort_keys, ctx->dstat);
   }
   ECS_LAUNCHED(ctx);

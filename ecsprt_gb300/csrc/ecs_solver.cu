@@ -928,6 +928,7 @@ struct SmallCycle {
   SmallLevel<T> lv[kMaxSmall];
 };
 constexpr size_t kSmallCells = 512;
+constexpr size_t kSmallSmem = 200 * 1024;  // its shared memory at most
 constexpr int kSmallThreads = (int)kSmallCells;
 // Planes that a column's thread keeps in registers; deeper columns (a
 // reflecting z is not coarsened) run their recurrences through shared memory.
@@ -2357,6 +2358,8 @@ template <typename T>
 int mg_alloc(EcsCtx *ctx) {
   Multigrid<T> &mg = mg_of<T>(ctx);
   if (mg.built) return ECS_OK;
+  // on the device of every context: a flag for the process would leave others out
+  ECS_CUDA(ctx, cudaFuncSetAttribute(k_vcycle_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
   for (const MgDims &d : mg_dims(ctx->p)) {
     MgLevel<T> L;
     L.nx = d.nx; L.ny = d.ny; L.nz = d.nz;
@@ -2567,8 +2570,6 @@ int sweep(EcsCtx *ctx, MgLevel<T> &L, const T *b, const T *xo, T *xn, bool rhs_d
   return ECS_OK;
 }
 
-constexpr size_t kSmallSmem = 200 * 1024;  // shared memory of the single-block cycle
-
 // Layout of a single-block cycle over levels l.. in shared memory (offsets in
 // sc, if given): per level 4 vectors, 11 row coefficients and 4 z-line factor
 // arrays, 2 column arrays, and 3 words a cell of neighbour offsets at the end.
@@ -2675,11 +2676,6 @@ int vcycle(EcsCtx *ctx, size_t l, const T *b, const T **x) {
       S.o = op_level(ctx, M);
       S.dens = M.dens;
       S.minv = M.zl_minv; S.q = M.zl_q; S.a0g = M.zl_a0g; S.qden = M.zl_qden;
-    }
-    static std::atomic<bool> attr_set[2];  // zero-initialised: false
-    if (!attr_set[sizeof(T) == 8]) {
-      ECS_CUDA(ctx, cudaFuncSetAttribute(k_vcycle_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
-      attr_set[sizeof(T) == 8] = true;
     }
     ecs_launch_pdl(k_vcycle_small<T>, 1, kSmallThreads, bytes, ctx->stream, sc, b, xout, kCoarseSweeps, kOmega<T>());
     ECS_LAUNCHED(ctx);
