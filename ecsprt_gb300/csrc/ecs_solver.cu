@@ -3436,6 +3436,9 @@ int ecs_solver_free(EcsCtx *ctx) {
 // ---- stand-alone solve requests ---------------------------------------------
 int ecs_request_launch(EcsCtx *ctx, const double *density, double *phi, const double flux_scale[3], double rtol,
                        int max_it) {
+  // before the graph is built: it keeps the kernels that this picks, and a
+  // request's density is no deposit's
+  ctx->mom_quanta = false;
   int rc = ctx->prec == ECS_PREC_FP64 ? build_request_graph<double>(ctx, flux_scale, rtol, max_it)
                                       : build_request_graph<float>(ctx, flux_scale, rtol, max_it);
   if (rc) return rc;
@@ -3459,7 +3462,6 @@ int ecs_request_launch(EcsCtx *ctx, const double *density, double *phi, const do
   ECS_CUDA(ctx, cudaGraphLaunch(rg.exec, ctx->stream));
   ECS_CUDA(ctx, cudaEventRecord(ctx->ev_solve[1], ctx->stream));
   ctx->moments_ready = true;
-  ctx->mom_quanta = false;
   ctx->lhs_ready = true;
   ctx->eext_ready = false;
   return ECS_OK;
