@@ -2514,11 +2514,12 @@ int ecs_part_fused(EcsCtx *ctx, double dt, int do_collide, int *sorted) {
 //   uploads   fixed chunks of stage_n ions: copies in on xs[1], conversion
 //             into the records on xs_up (two staging buffers), all issued
 //             at once;
-//   the pass  by ranges of whole tiles (at most stage_n ions) on the
-//             context's stream, each range after the upload chunks it reads
-//             have been converted;
-//   downloads by the same ranges: conversion on xs_conv, copies out on
-//             xs[0] (three staging buffers).
+//   the pass  by ranges of whole tiles (at most stage_n ions, or one tile
+//             of more) on the context's stream, each range after the upload
+//             chunks it reads have been converted;
+//   downloads by the same ranges, in pieces of at most stage_n ions:
+//             conversion on xs_conv, copies out on xs[0] (three staging
+//             buffers).
 // The copies in never wait for the copies out, so both directions of the
 // host link stay busy.  After a cell sort (pending permutation) the pass
 // gathers each range's ions from their old positions (the host arrays'
@@ -2619,8 +2620,6 @@ int ecs_part_host_pass(EcsCtx *ctx, double *pos, double *vel, int64_t np, double
   if ((rc = host_tile_tables(ctx, ntiles, gather))) return rc;
   const int32_t *tb = ctx->tile_bounds;
   if (tb[ntiles] != np) return ECS_ERR_STATE;
-  for (int t = 0; t < ntiles; t++)
-    if (tb[t + 1] - tb[t] > chunk) return ECS_ERR_STATE;  // a tile larger than a staging chunk
   const int64_t nup = ecs_div_up(np, chunk);
   if (!ctx->stage_dn[0]) {
     ECS_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->xs_conv, cudaStreamNonBlocking));
@@ -2717,13 +2716,14 @@ int ecs_part_host_pass(EcsCtx *ctx, double *pos, double *vel, int64_t np, double
     done[r] = 1;
     for (int d = r; d <= r + 1 && d < R; d++) {
       if (out[d] || !done[d] || (d > 0 && !done[d - 1])) continue;
-      const int qd = (int)(c % ND);
-      ECS_CUDA(ctx, cudaEventRecord(ctx->xev_tiled[qd], ctx->stream));
-      ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs_conv, ctx->xev_tiled[qd], 0));
-      if (c >= ND) ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs_conv, ctx->xev_dn_copy[qd], 0));  // staging out free
-      if ((rc = host_span_out(ctx, k, pos, vel, np, rg[d].A, rg[d].n, dst, qd))) return rc;
+      for (int64_t a = 0; a < rg[d].n; a += chunk, c++) {
+        const int qd = (int)(c % ND);
+        ECS_CUDA(ctx, cudaEventRecord(ctx->xev_tiled[qd], ctx->stream));
+        ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs_conv, ctx->xev_tiled[qd], 0));
+        if (c >= ND) ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs_conv, ctx->xev_dn_copy[qd], 0));  // staging out free
+        if ((rc = host_span_out(ctx, k, pos, vel, np, rg[d].A + a, std::min(chunk, rg[d].n - a), dst, qd))) return rc;
+      }
       out[d] = 1;
-      c++;
     }
   }
   if (waited < nup - 1) ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, ctx->xev_upc[nup - 1], 0));
