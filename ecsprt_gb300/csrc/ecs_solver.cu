@@ -3248,14 +3248,16 @@ int ecs_solver_alloc(EcsCtx *ctx) {
     ECS_CUDA(ctx, cudaMallocHost((void **)&ctx->h_dots, (size_t)(m + 2) * sizeof(double)));
     ECS_CUDA(ctx, cudaMalloc((void **)&ctx->r64, n * sizeof(double)));
     ECS_CUDA(ctx, cudaMalloc(&ctx->kdev, sizeof(KrylovDev)));
-    ECS_CUDA(ctx, cudaMemset(ctx->kdev, 0, sizeof(KrylovDev)));
+    // zeroed on the context's stream: the default stream is not ordered with
+    // it, and behind a host step's transfers its memset ran during the first solve
+    ECS_CUDA(ctx, cudaMemsetAsync(ctx->kdev, 0, sizeof(KrylovDev), ctx->stream));
     ECS_CUDA(ctx, cudaMallocHost(&ctx->kdev_host, sizeof(KrylovDev)));
     ECS_CUDA(ctx, cudaMallocHost(&ctx->kctl_host, sizeof(KrylovDev)));
     memset(ctx->kdev_host, 0, sizeof(KrylovDev));
     memset(ctx->kctl_host, 0, sizeof(KrylovDev));
     if (!identity_lhs(ctx)) ECS_CUDA(ctx, cudaMalloc((void **)&ctx->coef64, 11 * n * sizeof(double)));
     ECS_CUDA(ctx, cudaMalloc(&ctx->rdev, sizeof(RefineDev)));
-    ECS_CUDA(ctx, cudaMemset(ctx->rdev, 0, sizeof(RefineDev)));
+    ECS_CUDA(ctx, cudaMemsetAsync(ctx->rdev, 0, sizeof(RefineDev), ctx->stream));
     ECS_CUDA(ctx, cudaMallocHost(&ctx->rdev_host, sizeof(RefineDev)));
     memset(ctx->rdev_host, 0, sizeof(RefineDev));
   }
