@@ -3,6 +3,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 
 #include "ecs_internal.cuh"
@@ -27,9 +28,10 @@ int ecs_cuda_check(EcsCtx *ctx, cudaError_t e, const char *what) {
 
 namespace {
 
-__global__ void k_moments_aos(size_t n, const double *__restrict__ mom, double *__restrict__ out) {
+// n cells of fields `plane` apart
+__global__ void k_moments_aos(size_t n, size_t plane, const double *__restrict__ mom, double *__restrict__ out) {
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
-    for (int d = 0; d < 4; d++) out[4 * c + d] = mom[(size_t)d * n + c];
+    for (int d = 0; d < 4; d++) out[4 * c + d] = mom[(size_t)d * plane + c];
 }
 __global__ void k_moments_soa(size_t n, const double *__restrict__ in, double *__restrict__ mom) {
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x)
@@ -324,7 +326,7 @@ int ecs_moments_upload(EcsCtx *ctx, const double *m) {
 static int moments_to_host(EcsCtx *ctx, double *m) {
   double *stage = nullptr;
   ECS_CUDA(ctx, cudaMallocAsync((void **)&stage, ctx->ncell * 4 * sizeof(double), ctx->stream));
-  k_moments_aos<<<blocks(ctx, ctx->ncell), 256, 0, ctx->stream>>>(ctx->ncell, ctx->mom, stage);
+  k_moments_aos<<<blocks(ctx, ctx->ncell), 256, 0, ctx->stream>>>(ctx->ncell, ctx->ncell, ctx->mom, stage);
   ECS_LAUNCHED(ctx);
   ECS_CUDA(ctx, cudaMemcpyAsync(m, stage, ctx->ncell * 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   ECS_CUDA(ctx, cudaFreeAsync(stage, ctx->stream));
@@ -332,22 +334,26 @@ static int moments_to_host(EcsCtx *ctx, double *m) {
   return ECS_OK;
 }
 
-// The same without waiting, for ecs_step_host after its pipelined pass: the
-// conversion into the free upload staging buffer on the context's stream,
-// the copy behind the ions' download (xs[0], waited for with them).  *sent
-// stays false when the staging buffer is too small (then use the above).
-static int moments_to_host_async(EcsCtx *ctx, double *m, bool *sent) {
-  *sent = false;
-  const size_t bytes = ctx->ncell * 4 * sizeof(double);
-  if (!ctx->stage[0] || !ctx->xs[0] || bytes > (size_t)ecs_stage_stride(ctx->stage_n) * 2 * sizeof(double))
-    return ECS_OK;
+// The same without waiting, for ecs_step_host after its pipelined pass: in
+// pieces through the two upload staging buffers, which are free then,
+// converted on xs_conv and copied behind the ions' download (xs[0]), both
+// waited for with it.
+static int moments_to_host_async(EcsCtx *ctx, double *m) {
+  const size_t n = ctx->ncell, piece = (size_t)ecs_stage_stride(ctx->stage_n) * 2 / 4;  // cells
   if (!ctx->ev_mom) ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->ev_mom, cudaEventDisableTiming));
-  k_moments_aos<<<blocks(ctx, ctx->ncell), 256, 0, ctx->stream>>>(ctx->ncell, ctx->mom, ctx->stage[0]);
-  ECS_LAUNCHED(ctx);
   ECS_CUDA(ctx, cudaEventRecord(ctx->ev_mom, ctx->stream));
-  ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs[0], ctx->ev_mom, 0));
-  ECS_CUDA(ctx, cudaMemcpyAsync(m, ctx->stage[0], bytes, cudaMemcpyDeviceToHost, ctx->xs[0]));
-  *sent = true;
+  ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs_conv, ctx->ev_mom, 0));
+  for (size_t c = 0, u = 0; c < n; c += piece, u++) {
+    const int q = (int)(u & 1);
+    const size_t cells = std::min(piece, n - c);
+    if (u >= 2) ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs_conv, ctx->xev_copy[q], 0));  // buffer q copied out
+    k_moments_aos<<<blocks(ctx, cells), 256, 0, ctx->xs_conv>>>(cells, n, ctx->mom + c, ctx->stage[q]);
+    ECS_LAUNCHED(ctx);
+    ECS_CUDA(ctx, cudaEventRecord(ctx->xev_kern[q], ctx->xs_conv));
+    ECS_CUDA(ctx, cudaStreamWaitEvent(ctx->xs[0], ctx->xev_kern[q], 0));
+    ECS_CUDA(ctx, cudaMemcpyAsync(m + 4 * c, ctx->stage[q], cells * 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->xs[0]));
+    ECS_CUDA(ctx, cudaEventRecord(ctx->xev_copy[q], ctx->xs[0]));
+  }
   return ECS_OK;
 }
 
@@ -525,7 +531,8 @@ int ecs_step_host(EcsCtx *ctx, double *pos, double *vel, int64_t np, double dt, 
     if ((rc = ecs_grid_moments(ctx))) return rc;
     if ((rc = ecs_part_status_async(ctx))) return rc;
     // the moments go out behind the ions' download while the solve runs
-    if (moments_out && (rc = moments_to_host_async(ctx, moments_out, &moments_sent))) return rc;
+    if (moments_out && (rc = moments_to_host_async(ctx, moments_out))) return rc;
+    moments_sent = true;
   }
   EcsSolveStats st;
   StepStatus ss = {};
