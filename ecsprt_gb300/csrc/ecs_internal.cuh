@@ -257,8 +257,9 @@ int ecs_validate_params(const EcsParams *p);
 // thirty-second of the capacity, so that the first chunk's upload and the last
 // one's download are a small part of the whole, but at most 2^22 ions and at
 // least 2^19 (copies of some 12 MB; an eighth of a smaller capacity, at least
-// 2^16).  64^3, 64 ions a cell: a host step takes 7.0-7.8 ms with an eighth,
-// 6.5-6.9 with a thirty-second.
+// 2^16).  Host steps with an eighth and with a thirty-second, in turn, medians
+// of six runs of 32: 64^3 x 64 ions a cell 6.78-6.98 and 6.32-6.50 ms, 96^3 x 32
+// 11.2-12.2 and 10.1-10.4, 128^3 x 16 13.5-14.7 and 12.4.
 inline int64_t ecs_stage_ions(int64_t cap) {
   int64_t n = cap / 8;
   if (n > ((int64_t)1 << 19)) n = cap / 32 > ((int64_t)1 << 19) ? cap / 32 : (int64_t)1 << 19;
@@ -304,9 +305,12 @@ __device__ __forceinline__ void ecs_pdl_trigger() { asm volatile("griddepcontrol
 // or more (about a quarter of the SMs) let their successor in when they end.
 // Its early blocks gain nothing beside kernels of 10 us and more and take slots
 // from their later blocks: FP64 solves of 64^3 1.621 -> 1.511 ms, 80 x 72 x 64
-// 3.27 -> 3.06, 37 x 50 x 61 6.95 -> 5.32, 256^2 in 2-D 1.28 -> 1.18; up to 1 %
-// slower at 10,000 cells, where all are short.  FP32 kernels, 3 to 5 us most of
-// them, lose without it: 128^3 1.481 against 1.522 ms.
+// 3.27 -> 3.06, 37 x 50 x 61 6.95 -> 5.32, 256^2 in 2-D 1.28 -> 1.18.  The line at
+// 17, 40, 100 or 152 blocks: 48^3 1.665, 1.666, 1.690, 1.690 ms; 64^3 1.801, 1.793,
+// 1.792, 1.828; 64 x 48 x 33 with walls 2.825, 2.820, 2.845, 2.846; 128 x 100
+// 2.560, 2.545, 2.547, 2.547; grids of 10,000 cells, where all kernels are
+// short, do not feel it (20 x 16 x 30 1.817 on every line).  FP32 kernels, 3 to
+// 5 us most of them, lose without the trigger: 128^3 1.481 against 1.522 ms.
 #define ECS_PDL_ENTRY_FOR(T)                                                                     \
   do {                                                                                           \
     ecs_pdl_wait();                                                                              \

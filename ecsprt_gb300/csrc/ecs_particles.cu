@@ -419,6 +419,9 @@ __device__ __forceinline__ void deposit_warp(long long *__restrict__ acc, unsign
 // (kFlatGroups or fewer: ions in cell order) are summed first, each half its
 // own lanes' ions.  k_particles32 at 256^2 cells, 64 ions a cell: any order
 // 293 -> 222 us (175 with interleaved accumulators), cell order 161 -> 103 us.
+// The line at 4, 8 or 16 cells a warp: 134, 198, 198 us with 8 cells a warp (runs
+// of 4 ions), 16, 20, 20 us at 4 ions a cell in cell order (8 cells too); 172 in
+// any order and 92 in cell order wherever it lies.
 constexpr int kFlatGroups = 8;
 __device__ __forceinline__ void deposit_flat(long long *__restrict__ acc, unsigned char *tile_mem, const PartK &k,
                                              bool active, int i, int j, float wxh, float wyh, float v0, float v1) {

@@ -856,11 +856,17 @@ void launch_residual_restrict(EcsCtx *ctx, const OpK &o, const GridG &gc, const 
   ecs_launch_pdl(k_residual_restrict<T, Z>, g, R::kThreads, 0, ctx->stream, o, gc, (const T *)L.dens, (const T *)L.coef,
                  (const T *)L.t, b, c);
 }
-// Levels whose residual and restriction are one kernel.  3-D: 32^3 solve 0.585
-// -> 0.561 ms, FP64 40 x 24 x 20 1.263 -> 1.216; on a 64^3 level the rim's second
+// Levels whose residual and restriction are one kernel (and, in FP32, their
+// prolongation and right-hand side, k_prolong_rhs).  3-D: 32^3 solve 0.585 ->
+// 0.561 ms, FP64 40 x 24 x 20 1.263 -> 1.216; on a 64^3 level the rim's second
 // residuals cost more than the launch (64^3 solve 0.744 with two kernels, 0.760
 // fused).  In 2-D the rim is smaller: 256^2 solve 0.748 -> 0.710 with the levels
-// below 256^2 and 2 to 3 % more with it.
+// below 256^2 and 2 to 3 % more with it.  Where the line lies (whole solves;
+// no level fused, this line, the line at twice and at three (2-D: eight) times
+// the cells):
+// 40^3 0.849, 0.786, 0.781-0.789 ms, 40 x 40 x 42 (67,200 cells) 0.957, 0.956, 0.966;
+// 48^3 0.840, 0.805, 0.805; 56^3 0.909, 0.868, 0.868, 0.875; 2-D 320 x 400 1.124,
+// 1.039; 400^2 1.610, 1.523, 1.511; 512^2 1.086, 1.020, 1.016, 1.029.
 inline bool residual_restrict_fused(const GridG &g) {
   return g.n < (g.nz == 1 ? (size_t)1 << 17 : (size_t)1 << 16);
 }
@@ -1404,7 +1410,10 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Cluster of the sweeps of an nx x ny x nz level: one CTA up to 2048 cells,
 // then a CTA for each 2048 (a sweep of that many cells takes about as long as
 // the cluster barrier), at most sixteen and one a row; 0 CTAs when the level
-// does not fit (or its columns are cut into longer segments).
+// does not fit (or its columns are cut into longer segments).  Solves with
+// 1024, 2048 and 4096 cells a CTA: 20 x 18 x 22 0.736, 0.736, 0.736 ms; 26^3 0.740,
+// 0.751, 0.836; 30^3 0.741, 0.801, 0.925; 34^3 0.953, 0.948, 1.109; 42 x 38 x 34
+// 1.011, 1.209, 1.428; 66 x 54 x 42 1.496, 1.493, 1.659; 100 x 72 x 50 2.55 each.
 static CoarseShape coarse_shape(int nx, int ny, int nz) {
   CoarseShape s;
   if (nz > kClusterSeg * kMaxSeg) return s;
