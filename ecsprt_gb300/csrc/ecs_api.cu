@@ -22,6 +22,7 @@ int ecs_fail(EcsCtx *ctx, int code, const char *fmt, ...) {
 }
 
 int ecs_cuda_check(EcsCtx *ctx, cudaError_t e, const char *what) {
+  cudaGetLastError();  // reported here: the thread's next launch must not find it
   return ecs_fail(ctx, e == cudaErrorMemoryAllocation ? ECS_ERR_NOMEM : ECS_ERR_CUDA, "%s: %s", what,
                   cudaGetErrorString(e));
 }
@@ -183,6 +184,7 @@ int ecs_ctx_create(const EcsParams *params, int precision, int64_t np_capacity, 
     if (a_ != cudaSuccess) {                                                      \
       ecs_fail(nullptr, ECS_ERR_NOMEM, "cudaMalloc %zu bytes: %s", (size_t)(bytes), \
                cudaGetErrorString(a_));                                           \
+      cudaGetLastError();                                                         \
       ecs_ctx_destroy(ctx);                                                       \
       return ECS_ERR_NOMEM;                                                       \
     }                                                                             \
@@ -196,6 +198,7 @@ int ecs_ctx_create(const EcsParams *params, int precision, int64_t np_capacity, 
   else CREATE_ALLOC(ctx->eext32, ctx->next * sizeof(float4));
 #undef CREATE_ALLOC
   if (cudaMallocHost((void **)&ctx->hstat, sizeof(EcsDevStatus)) != cudaSuccess) {
+    cudaGetLastError();
     ecs_fail(nullptr, ECS_ERR_NOMEM, "pinned allocation failed");
     ecs_ctx_destroy(ctx);
     return ECS_ERR_NOMEM;

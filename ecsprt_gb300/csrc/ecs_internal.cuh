@@ -278,6 +278,24 @@ int ecs_cuda_check(EcsCtx *ctx, cudaError_t e, const char *what);
     cudaError_t e_ = (call);                                       \
     if (e_ != cudaSuccess) return ecs_cuda_check((ctx), e_, #call); \
   } while (0)
+// Buffers allocated on first use: a no-op where p is set, and a failure leaves
+// it unset, so that the call can be made again.
+template <typename T>
+inline int ecs_dev_alloc(EcsCtx *ctx, T *&p, size_t bytes) {
+  if (p) return ECS_OK;
+  void *q = nullptr;
+  ECS_CUDA(ctx, cudaMalloc(&q, bytes));
+  p = static_cast<T *>(q);
+  return ECS_OK;
+}
+template <typename T>
+inline int ecs_pinned_alloc(EcsCtx *ctx, T *&p, size_t bytes) {
+  if (p) return ECS_OK;
+  void *q = nullptr;
+  ECS_CUDA(ctx, cudaMallocHost(&q, bytes));
+  p = static_cast<T *>(q);
+  return ECS_OK;
+}
 #define ECS_LAUNCHED(ctx)                                                   \
   do {                                                                      \
     (ctx)->launches++;                                                      \

@@ -2017,17 +2017,25 @@ int ecs_particles_free(EcsCtx *ctx) {
 // (ecs_stage_ions) through two staging buffers, so that the copy of one
 // chunk overlaps the conversion kernel of the other.
 
+static int ensure_event(EcsCtx *ctx, cudaEvent_t &e) {
+  if (!e) ECS_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return ECS_OK;
+}
+static int ensure_stream(EcsCtx *ctx, cudaStream_t &s) {
+  if (!s) ECS_CUDA(ctx, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  return ECS_OK;
+}
+
 static int ensure_xfer(EcsCtx *ctx) {
-  if (ctx->stage[0]) return ECS_OK;
-  for (int q = 0; q < 2; q++) {
-    ECS_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->xs[q], cudaStreamNonBlocking));
-    ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->xev_copy[q], cudaEventDisableTiming));
-    ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->xev_kern[q], cudaEventDisableTiming));
-  }
-  ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->xev_ready, cudaEventDisableTiming));
+  if (ctx->stage_n) return ECS_OK;  // set last: everything is there
   const int64_t n = ecs_stage_ions(ctx->cap);
+  int rc;
   for (int q = 0; q < 2; q++)
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->stage[q], (size_t)ecs_stage_stride(n) * 2 * sizeof(double)));
+    if ((rc = ensure_stream(ctx, ctx->xs[q])) || (rc = ensure_event(ctx, ctx->xev_copy[q])) ||
+        (rc = ensure_event(ctx, ctx->xev_kern[q])) ||
+        (rc = ecs_dev_alloc(ctx, ctx->stage[q], (size_t)ecs_stage_stride(n) * 2 * sizeof(double))))
+      return rc;
+  if ((rc = ensure_event(ctx, ctx->xev_ready))) return rc;
   ctx->stage_n = n;
   return ECS_OK;
 }
@@ -2588,11 +2596,11 @@ static int host_tile_tables(EcsCtx *ctx, int ntiles, bool gather) {
   const bool want_b = !ctx->bounds_valid;
   if (!want_b && !gather) return ECS_OK;
   const size_t nb = (size_t)ntiles + 1, words = nb + (size_t)ntiles;
-  if (!ctx->tile_tables_dev) {
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->tile_tables_dev, words * sizeof(int32_t)));
-    ECS_CUDA(ctx, cudaMallocHost((void **)&ctx->tile_bounds, words * sizeof(int32_t)));
-    ctx->tile_srcmax = ctx->tile_bounds + nb;
-  }
+  int rc;
+  if ((rc = ecs_dev_alloc(ctx, ctx->tile_tables_dev, words * sizeof(int32_t))) ||
+      (rc = ecs_pinned_alloc(ctx, ctx->tile_bounds, words * sizeof(int32_t))))
+    return rc;
+  ctx->tile_srcmax = ctx->tile_bounds + nb;
   int32_t *d = ctx->tile_tables_dev;
   if (want_b) {
     k_tile_bounds<<<ecs_div_up(nb, 256), 256, 0, ctx->stream>>>(ntiles, ctx->sort_offset, d);
@@ -2624,16 +2632,12 @@ int ecs_part_host_pass(EcsCtx *ctx, double *pos, double *vel, int64_t np, double
   const int32_t *tb = ctx->tile_bounds;
   if (tb[ntiles] != np) return ECS_ERR_STATE;
   const int64_t nup = ecs_div_up(np, chunk);
-  if (!ctx->stage_dn[0]) {
-    ECS_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->xs_conv, cudaStreamNonBlocking));
-    ECS_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->xs_up, cudaStreamNonBlocking));
-    for (int q = 0; q < EcsCtx::kStageDn; q++) {
-      ECS_CUDA(ctx, cudaMalloc((void **)&ctx->stage_dn[q], (size_t)ecs_stage_stride(chunk) * 2 * sizeof(double)));
-      ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->xev_tiled[q], cudaEventDisableTiming));
-      ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->xev_dn_conv[q], cudaEventDisableTiming));
-      ECS_CUDA(ctx, cudaEventCreateWithFlags(&ctx->xev_dn_copy[q], cudaEventDisableTiming));
-    }
-  }
+  if ((rc = ensure_stream(ctx, ctx->xs_conv)) || (rc = ensure_stream(ctx, ctx->xs_up))) return rc;
+  for (int q = 0; q < EcsCtx::kStageDn; q++)
+    if ((rc = ecs_dev_alloc(ctx, ctx->stage_dn[q], (size_t)ecs_stage_stride(chunk) * 2 * sizeof(double))) ||
+        (rc = ensure_event(ctx, ctx->xev_tiled[q])) || (rc = ensure_event(ctx, ctx->xev_dn_conv[q])) ||
+        (rc = ensure_event(ctx, ctx->xev_dn_copy[q])))
+      return rc;
   while ((int64_t)ctx->xev_upc.size() < nup) {
     cudaEvent_t e;
     ECS_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

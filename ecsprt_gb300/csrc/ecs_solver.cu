@@ -2362,46 +2362,61 @@ void mg_bytes(const std::vector<MgDims> &lv, DeviceBytes &b) {
   if (nc <= kDirectMax) b.add(nc * nc * sizeof(T));
 }
 
+template <typename T>
+void free_mg(Multigrid<T> &mg);
+
 // An array added here goes into mg_bytes too.
+template <typename T>
+int mg_alloc_levels(EcsCtx *ctx, Multigrid<T> &mg) {
+  int rc;
+  for (const MgDims &d : mg_dims(ctx->p)) {
+    mg.lv.emplace_back();
+    MgLevel<T> &L = mg.lv.back();
+    L.nx = d.nx; L.ny = d.ny; L.nz = d.nz;
+    L.n = (size_t)d.nx * d.ny * d.nz;
+    L.hx = d.hx; L.hy = d.hy; L.hz = d.hz;
+    T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_minv, &L.zl_q};
+    for (auto a : arr)
+      if ((rc = ecs_dev_alloc(ctx, *a, L.n * sizeof(T)))) return rc;
+    if constexpr (sizeof(T) == 8) {
+      if (mg.lv.size() == 1) L.coef = ctx->coef64;
+      else if ((rc = ecs_dev_alloc(ctx, L.coef, 11 * L.n * sizeof(T)))) return rc;
+    }
+    if (zl_stored<T>(seg_len<T>(L.nz))) {
+      T **more[] = {&L.zl_a, &L.zl_cp, &L.zl_fb, &L.zl_bb};
+      for (auto a : more)
+        if ((rc = ecs_dev_alloc(ctx, *a, L.n * sizeof(T)))) return rc;
+    }
+    for (auto a : {&L.zl_a0g, &L.zl_qden})
+      if ((rc = ecs_dev_alloc(ctx, *a, (size_t)L.nx * L.ny * sizeof(T)))) return rc;
+  }
+  const size_t nc = mg.lv.back().n;
+  if (nc <= (size_t)kDirectMax) {
+    if ((rc = ecs_dev_alloc(ctx, mg.cinv, nc * nc * sizeof(T)))) return rc;
+  } else if constexpr (sizeof(T) == 4) {
+    const MgLevel<T> &C = mg.lv.back();
+    CoarseShape cs = coarse_shape(C.nx, C.ny, C.nz);
+    if (cs.ctas > 0) {
+      rc = coarse_attrs<T>(ctx, cs);
+      if (rc) return rc;
+    }
+    mg.cluster = cs;
+  }
+  return ECS_OK;
+}
+
+// The whole hierarchy or, when an allocation fails, none of it: a later call
+// starts anew.
 template <typename T>
 int mg_alloc(EcsCtx *ctx) {
   Multigrid<T> &mg = mg_of<T>(ctx);
   if (mg.built) return ECS_OK;
   // on the device of every context: a flag for the process would leave others out
   ECS_CUDA(ctx, cudaFuncSetAttribute(k_vcycle_small<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
-  for (const MgDims &d : mg_dims(ctx->p)) {
-    MgLevel<T> L;
-    L.nx = d.nx; L.ny = d.ny; L.nz = d.nz;
-    L.n = (size_t)d.nx * d.ny * d.nz;
-    L.hx = d.hx; L.hy = d.hy; L.hz = d.hz;
-    T **arr[] = {&L.dens, &L.x, &L.b, &L.r, &L.t, &L.zl_minv, &L.zl_q};
-    for (auto a : arr) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
-    if constexpr (sizeof(T) == 8) {
-      if (mg.lv.empty()) L.coef = ctx->coef64;
-      else ECS_CUDA(ctx, cudaMalloc((void **)&L.coef, 11 * L.n * sizeof(T)));
-    }
-    if (zl_stored<T>(seg_len<T>(L.nz))) {
-      T **more[] = {&L.zl_a, &L.zl_cp, &L.zl_fb, &L.zl_bb};
-      for (auto a : more) ECS_CUDA(ctx, cudaMalloc((void **)a, L.n * sizeof(T)));
-    }
-    ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_a0g, (size_t)L.nx * L.ny * sizeof(T)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&L.zl_qden, (size_t)L.nx * L.ny * sizeof(T)));
-    mg.lv.push_back(L);
-  }
-  const size_t nc = mg.lv.back().n;
-  if (nc <= (size_t)kDirectMax) {
-    ECS_CUDA(ctx, cudaMalloc((void **)&mg.cinv, nc * nc * sizeof(T)));
-  } else if constexpr (sizeof(T) == 4) {
-    const MgLevel<T> &C = mg.lv.back();
-    CoarseShape cs = coarse_shape(C.nx, C.ny, C.nz);
-    if (cs.ctas > 0) {
-      const int rc = coarse_attrs<T>(ctx, cs);
-      if (rc) return rc;
-    }
-    mg.cluster = cs;
-  }
-  mg.built = true;
-  return ECS_OK;
+  const int rc = mg_alloc_levels<T>(ctx, mg);
+  if (rc) free_mg(mg);
+  else mg.built = true;
+  return rc;
 }
 
 template <typename T>
@@ -3163,11 +3178,8 @@ int build_request_graph(EcsCtx *ctx, const double fs[3], double rtol, int max_it
     return ECS_OK;
   free_request_graph(rg);
   const size_t n = ctx->ncell, bytes = n * sizeof(double);
-  if (!rg.h_in) {
-    ECS_CUDA(ctx, cudaMallocHost((void **)&rg.h_in, bytes));
-    ECS_CUDA(ctx, cudaMallocHost((void **)&rg.h_out, bytes));
-  }
   int rc;
+  if ((rc = ecs_pinned_alloc(ctx, rg.h_in, bytes)) || (rc = ecs_pinned_alloc(ctx, rg.h_out, bytes))) return rc;
   // allocations and one-time attributes outside the capture
   if ((rc = ecs_solver_alloc(ctx))) return rc;
   if (!identity_lhs(ctx) && (rc = mg_alloc<T>(ctx))) return rc;
@@ -3247,37 +3259,45 @@ void ecs_mg_bytes(const EcsParams &p, int precision, DeviceBytes &b) {
   else mg_bytes<float>(lv, b);
 }
 
+// Each buffer that is not there yet (after a failure, the rest of them).
 int ecs_solver_alloc(EcsCtx *ctx) {
-  size_t n = ctx->ncell;
-  int m = ctx->krylov_m;
-  if (!ctx->red) {
-    ctx->nred = kSlots * 4096;
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->red, (size_t)ctx->nred * sizeof(double)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->dots, (size_t)(m + 2) * sizeof(double)));
-    ECS_CUDA(ctx, cudaMallocHost((void **)&ctx->h_dots, (size_t)(m + 2) * sizeof(double)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->r64, n * sizeof(double)));
-    ECS_CUDA(ctx, cudaMalloc(&ctx->kdev, sizeof(KrylovDev)));
-    // zeroed on the context's stream: the default stream is not ordered with
-    // it, and behind a host step's transfers its memset ran during the first solve
+  const size_t n = ctx->ncell, m = (size_t)ctx->krylov_m;
+  int rc;
+  ctx->nred = kSlots * 4096;
+  if ((rc = ecs_dev_alloc(ctx, ctx->red, (size_t)ctx->nred * sizeof(double))) ||
+      (rc = ecs_dev_alloc(ctx, ctx->dots, (m + 2) * sizeof(double))) ||
+      (rc = ecs_pinned_alloc(ctx, ctx->h_dots, (m + 2) * sizeof(double))) ||
+      (rc = ecs_dev_alloc(ctx, ctx->r64, n * sizeof(double))))
+    return rc;
+  if (!identity_lhs(ctx) && (rc = ecs_dev_alloc(ctx, ctx->coef64, 11 * n * sizeof(double)))) return rc;
+  // zeroed on the context's stream: the default stream is not ordered with
+  // it, and behind a host step's transfers its memset ran during the first solve
+  if (!ctx->kdev) {
+    if ((rc = ecs_dev_alloc(ctx, ctx->kdev, sizeof(KrylovDev)))) return rc;
     ECS_CUDA(ctx, cudaMemsetAsync(ctx->kdev, 0, sizeof(KrylovDev), ctx->stream));
-    ECS_CUDA(ctx, cudaMallocHost(&ctx->kdev_host, sizeof(KrylovDev)));
-    ECS_CUDA(ctx, cudaMallocHost(&ctx->kctl_host, sizeof(KrylovDev)));
-    memset(ctx->kdev_host, 0, sizeof(KrylovDev));
-    memset(ctx->kctl_host, 0, sizeof(KrylovDev));
-    if (!identity_lhs(ctx)) ECS_CUDA(ctx, cudaMalloc((void **)&ctx->coef64, 11 * n * sizeof(double)));
-    ECS_CUDA(ctx, cudaMalloc(&ctx->rdev, sizeof(RefineDev)));
+  }
+  if (!ctx->rdev) {
+    if ((rc = ecs_dev_alloc(ctx, ctx->rdev, sizeof(RefineDev)))) return rc;
     ECS_CUDA(ctx, cudaMemsetAsync(ctx->rdev, 0, sizeof(RefineDev), ctx->stream));
-    ECS_CUDA(ctx, cudaMallocHost(&ctx->rdev_host, sizeof(RefineDev)));
-    memset(ctx->rdev_host, 0, sizeof(RefineDev));
   }
-  if (ctx->prec == ECS_PREC_FP64 && !ctx->kv64) {
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kv64, (size_t)(m + 1) * n * sizeof(double)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kz64, (size_t)m * n * sizeof(double)));
-  }
-  if (ctx->prec == ECS_PREC_MIXED && !ctx->kv32) {
+  struct {
+    void *&p;
+    size_t bytes;
+  } host[] = {{ctx->kdev_host, sizeof(KrylovDev)}, {ctx->kctl_host, sizeof(KrylovDev)}, {ctx->rdev_host, sizeof(RefineDev)}};
+  for (auto &h : host)
+    if (!h.p) {
+      if ((rc = ecs_pinned_alloc(ctx, h.p, h.bytes))) return rc;
+      memset(h.p, 0, h.bytes);
+    }
+  if (ctx->prec == ECS_PREC_FP64) {
+    if ((rc = ecs_dev_alloc(ctx, ctx->kv64, (m + 1) * n * sizeof(double))) ||
+        (rc = ecs_dev_alloc(ctx, ctx->kz64, m * n * sizeof(double))))
+      return rc;
+  } else {
     // V, Z and the normalised residual
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kv32, (size_t)(m + 1) * n * sizeof(float)));
-    ECS_CUDA(ctx, cudaMalloc((void **)&ctx->kz32, (size_t)(m + 1) * n * sizeof(float)));
+    if ((rc = ecs_dev_alloc(ctx, ctx->kv32, (m + 1) * n * sizeof(float))) ||
+        (rc = ecs_dev_alloc(ctx, ctx->kz32, (m + 1) * n * sizeof(float))))
+      return rc;
   }
   return ECS_OK;
 }
@@ -3307,8 +3327,7 @@ int ecs_solver_run(EcsCtx *ctx, double rtol, int max_it, int warm, EcsSolveStats
     if (rc0) return rc0;
     setup = 0;
   }
-  if (setup) ctx->lhs_ready = true;  // the graph sets the operator up before it solves
-  if (!ctx->lhs_ready) return ecs_fail(ctx, ECS_ERR_STATE, "solve called before lhs");
+  if (!setup && !ctx->lhs_ready) return ecs_fail(ctx, ECS_ERR_STATE, "solve called before lhs");
   const size_t n = ctx->ncell;
   const EcsParams &p = ctx->p;
   const OpK o64 = make_op(p, p.Nx, p.Ny, p.Nz, p.dx, p.dy, p.dz);
@@ -3321,6 +3340,7 @@ int ecs_solver_run(EcsCtx *ctx, double rtol, int max_it, int warm, EcsSolveStats
   int rc;
   if (graphs) {  // the whole solve as one graph launch, one wait
     if ((rc = solve_graph_launch(ctx, rtol, max_it, warm, setup))) return rc;
+    if (setup) ctx->lhs_ready = true;  // the graph sets the operator up before it solves
     RefineDev *hr = (RefineDev *)ctx->rdev_host;
     ECS_CUDA(ctx, cudaMemcpyAsync(hr, ctx->rdev, sizeof(RefineDev), cudaMemcpyDeviceToHost, ctx->stream));
     ECS_CUDA(ctx, cudaEventRecord(ctx->ev_solve[1], ctx->stream));
